@@ -29,6 +29,7 @@
 #include <functional>
 
 #include "precond.cuh"
+#include "resident.cuh"
 #include "sell.cuh"
 #include "solver_common.cuh"
 
@@ -519,6 +520,35 @@ void drive(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, int per_chunk, 
     if (graph) cudaGraphDestroy(graph);
 }
 
+// The iterations by the resident solver (resident.cu): it stops by itself, so
+// one launch takes up to kResidentChunk iterations; with a time budget, a
+// poll interval of the caller's or a per-chunk callback the launches are as
+// long as those.  The iteration limit is rounded up to whole poll intervals.
+constexpr int kResidentChunk = 4096;
+void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const ResidentPlan &plan, bool mixed,
+                    int per_chunk, double *d_u, float wsm, double tol2, Flags &hf, long long &launches,
+                    bool &timed_out, double t_start, const std::function<void(const double *)> &on_chunk) {
+    cudaStream_t s = c->stream;
+    Flags *h = reinterpret_cast<Flags *>(c->w.hflags.p);
+    const bool polled = o.time_budget_s > 0 || o.check_every > 0 || on_chunk;
+    const long limit = ((long)o.max_iter + per_chunk - 1) / per_chunk * per_chunk;
+    for (long done = 0;;) {
+        const int iters = (int)std::min<long>(polled ? per_chunk : kResidentChunk, limit - done);
+        resident_iterations(c, plan, mixed, ws.P, ws.fl, d_u, wsm, tol2, iters, mixed && done == 0);
+        ++launches;
+        done += iters;
+        OFEA_CUDA(cudaMemcpyAsync(h, ws.fl, sizeof(Flags), cudaMemcpyDeviceToHost, s));
+        OFEA_CUDA(cudaStreamSynchronize(s));
+        if (h->done || done >= limit) break;
+        if (on_chunk) on_chunk(c->w.r.p);
+        if (o.time_budget_s > 0 && now_s() - t_start > o.time_budget_s) {
+            timed_out = true;
+            break;
+        }
+    }
+    hf = *h;
+}
+
 int solver_grid(const ofea_ctx *c) { return std::min(kMaxGrid, c->num_sms * (2048 / kBlock)); }
 
 // Clears the context's V-cycle stop flag when the solve's iterations end
@@ -545,8 +575,6 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         return;
     }
     const double t_start = now_s();
-    const int G = solver_grid(c);
-    Workspace ws = setup(c, G);
     SolverWork &w = c->w;
     cudaEvent_t e0, e1;
     OFEA_CUDA(cudaEventCreate(&e0));
@@ -595,6 +623,11 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     } else {
         w.z.ensure(n);
     }
+    ResidentPlan plan;
+    const bool resident = !learned && resident_plan(c, mixed, plan);
+    if (resident && mixed) coarse_dense_inverse(c);
+    const int G = resident ? plan.G : solver_grid(c);
+    Workspace ws = setup(c, G);
     const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;
     for (int attempt = 0; attempt < 8; ++attempt) {
         OFEA_CUDA(cudaMemsetAsync(w.p0.p, 0, sizeof(double) * n, s));
@@ -632,7 +665,9 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         const double tol2 = (0.5 * o.rtol) * (0.5 * o.rtol) * ff;
         ofea_solve_opts oo = o;
         oo.max_iter = o.max_iter - total_iters;
-        if (mixed) {
+        if (resident) {
+            drive_resident(c, oo, ws, plan, mixed, per_chunk, d_u, wsm, tol2, hf, launches, timed_out, t_start, on_chunk);
+        } else if (mixed) {
             // the V-cycle kernels of this attempt return at once once the
             // solve has stopped (the flag is cleared at every attempt)
             c->vc_stop = &ws.fl->done;
@@ -677,6 +712,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         }
         total_iters += hf.iters;
         if (hf.status == OFEA_ERR_BREAKDOWN) break;
+        if (hf.status == OFEA_ERR_TIMEOUT) fail(OFEA_ERR_TIMEOUT, "a wait of the resident solver ran out");
     }
     OFEA_CUDA(cudaEventRecord(e1, s));
     OFEA_CUDA(cudaEventSynchronize(e1));

@@ -80,7 +80,7 @@ __device__ __forceinline__ int slot_dz(int s) { return s % 3 - 1; }
 
 // ------------------------------------------------------------ level data --
 
-// Eb[I][slot][36] from the Galerkin blocks (nchunk = 1: a masked copy).
+// Eb[I][slot][36] from the Galerkin blocks' chunks (one chunk: a masked copy).
 __global__ void k_e2_blocks(int na, int nchunk, const int *__restrict__ nbr, const double *__restrict__ part,
                             double *__restrict__ Eb) {
     const long total = (long)na * 27 * 36;
@@ -754,7 +754,7 @@ void setup_learned_level(ofea_ctx *c) {
     if (C2.K_ok) return;
     cudaStream_t s = c->stream;
     const int na = C2.na;
-    const int nchunk = 1;
+    const int nchunk = galerkin_chunks(c, C2);
     OFEA_CUDA(cudaMemsetAsync(c->err_flag.p, 0, sizeof(int), s));
     setup_mark(c, "geometry");
     coarse_E_partials(c, C2, nchunk);

@@ -46,9 +46,10 @@ void coarse_correct(ofea_ctx *c, const float *t, float *x);
 void vc_resid(ofea_ctx *c, const float *b, const float *x, float *t);
 // Level-generic pieces (also used by the learned level):
 // cvec = Z^T t, x += Z g, and the Galerkin blocks of Z^T K Z into C.part
-// ([aggregate][27 neighbour slots][6 x 6]; nchunk must be 1).
+// ([aggregate][chunk][27 neighbour slots][6 x 6], chunks summed by the caller).
 void restrict_level(ofea_ctx *c, const Coarse &C, const float *t, float *cvec);
 void prolong_level(ofea_ctx *c, const Coarse &C, const float *g, float *x);
+int galerkin_chunks(const ofea_ctx *c, const Coarse &C);
 void coarse_E_partials(ofea_ctx *c, Coarse &C, int nchunk);
 
 }  // namespace ofea

@@ -10,18 +10,19 @@
 // (NP = the NR load cases padded to a power of two >= 4): the load cases of
 // one DOF are one contiguous run.  Matrices stay where their contexts keep
 // them (BSELL-32, FP64 and BF16 copies); a table of per-variant
-// descriptors points at them.
+// descriptors points at them, one of records at their slices.
 //
 // Algorithm per (variant, load case): the MIXED method of solve.cu, FP64
 // flexible CG with the FP32 two-level V(1,1) preconditioner of precond.cu, or
 // PCG64 (FP64 CG, block Jacobi).  The kernel runs every variant in lock step
 // through phases separated by grid barriers.  In the matrix phases a CTA owns
-// one slice (32 block rows) of some variant at a time: it stages the slice's
-// BSELL slots in shared memory (cp.async, double-buffered), and its
-// threads take (block row, load case) pairs, JW lanes per row, so each matrix
-// value is read from HBM once for all load cases and every gather of x is one
-// contiguous run of load cases.  The restriction takes one aggregate per
-// CTA; other phases take (coarse row) or (variant, load case) items per warp.
+// one slice (32 block rows) of some variant at a time: bulk copies bring the
+// operand's entries of the slice's distinct columns and stream its slots
+// through shared memory (matrix_phase), and its threads take (block row, load
+// cases) pairs, so each matrix value is read from HBM once for all load cases
+// and each column's entries once per slice.  The restriction takes one
+// aggregate per CTA; other phases take (coarse row) or (variant, load case)
+// items per warp.
 // The outer SpMM multiplies the preconditioned residual z, not p: q = K z +
 // beta q_old equals K p (p = z + beta p_old), and gathering z (FP32 for
 // MIXED) instead of p_old and z cuts the gathered bytes by 3x (MIXED) or 2x
@@ -65,20 +66,34 @@ struct BVar {
     int nfree, nslice, slice0, na, m, agg0, crow0, n;
     long dof0;  // first DOF of the variant in the batch (its vectors start at dof0 * NR)
     long c0;    // first coarse entry of the variant (times NR)
-    const int *sl_ptr, *scols;
+    const int *sl_ptr, *scols, *sl_g, *su_n;
+    const int2 *su_runs;
+    const uint16_t *su_idx;
     const double *sv64, *Dinv;
-    const __nv_bfloat16 *sv16;
+    const __nv_bfloat16 *sv16g;
     const float *Dinv32;
-    const int *agg_of, *agg_ptr, *agg_nodes, *node_of_free;
-    const double *xyz, *centroid;
+    const int *agg_ptr;
+    const float4 *agg_off, *row_off;  // offsets from the centroids (precond.cu)
     const float *Einv32;
-    double inv_scale;
     float wsm, pad2;
 };
 
-struct GridSync {
-    unsigned count, gen;
-    int err, pad;
+// One slice of the batch (device table, in batch order): where its slots
+// start, its distinct columns as runs of consecutive ones (first column;
+// position << 16 | length) and every slot's position among them (lidx; nu = 0:
+// read the columns directly), and what the phases need of its rows.
+struct __align__(16) BSlice {
+    const double *v64;
+    const __nv_bfloat16 *vg;  // grouped BF16 values (sell.cuh)
+    const int *cols;
+    const int2 *runs;
+    const uint16_t *lidx;
+    const double *Dinv;
+    const float *Dinv32;
+    long dof;  // the variant's first DOF in the batch
+    int W, nu, nrun, row0, nfree, v;
+    float wsm;
+    int pad;
 };
 
 struct BArgs {
@@ -86,6 +101,9 @@ struct BArgs {
     unsigned long long limit_ns;
     double rtol;
     const BVar *var;
+    const BSlice *slice;
+    unsigned *vmask;  // [V]: bit j set while load case j runs
+    int cap;          // columns the staged products' buffer holds
     const int *slice_var, *agg_var, *crow_var;
     const double *f;
     double *u, *r, *p0, *p1, *q, *z64;
@@ -93,50 +111,12 @@ struct BArgs {
     double *pa, *pb;                                    // partials [slice][NR]
     double *ff, *tol2, *rz, *alpha, *beta;              // [V * NR]
     int *live, *iters, *status, *live_cnt;              // [V * NR], live_cnt[3]
-    GridSync *gs;
+    GridBar *gs;
     unsigned long long *trace;  // NULL, or %globaltimer at the start and after each grid barrier (CTA 0)
     int trace_cap;
 };
 
 namespace {
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid barrier for a cooperative launch.  Returns false when the batch has
-// failed (a wait ran out here or elsewhere): the caller returns.
-__device__ bool grid_barrier(GridSync *gs, unsigned nblocks, unsigned long long limit_ns) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        cuda::atomic_ref<unsigned, cuda::thread_scope_device> gen(gs->gen), cnt(gs->count);
-        cuda::atomic_ref<int, cuda::thread_scope_device> err(gs->err);
-        const unsigned g = gen.load(cuda::memory_order_acquire);
-        __threadfence();
-        const unsigned arrived = cnt.fetch_add(1u, cuda::memory_order_acq_rel) + 1u;
-        if (arrived == nblocks) {
-            cnt.store(0u, cuda::memory_order_relaxed);
-            gen.fetch_add(1u, cuda::memory_order_release);
-        } else {
-            const unsigned long long t0 = global_ns();
-            while (gen.load(cuda::memory_order_acquire) == g) {
-                if (err.load(cuda::memory_order_relaxed) != 0) break;
-                if (global_ns() - t0 > limit_ns) {
-                    err.store(1, cuda::memory_order_relaxed);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        s_ok = err.load(cuda::memory_order_relaxed) == 0;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
 
 // Entry (node i, component c, load case j) of a variant in a batch vector
 // whose load-case stride is NP (NR rounded up; padding entries stay zero).
@@ -200,16 +180,67 @@ struct Lanes {
     __device__ static int j0() { return (threadIdx.x & (kLW - 1)) * RL; }
 };
 
-// Shared-memory stage of a slice's BSELL slots: two buffers of kKC slots
-// (values in FP64 or BF16, then columns), filled with cp.async while the
-// other buffer is consumed.
-constexpr int kKC = 8;
+// Shared memory of a matrix phase: three buffers of the slice's slots (kKC64
+// FP64 slots or kKC16 BF16 ones, then their column positions) and the records
+// of this slice and the next ones; partial sums and the distinct columns'
+// entries of the operand follow (dynamic).  Filled by bulk copies that complete on the
+// mbarriers (bx: the operand, bv: the slot buffers).
+constexpr int kKC64 = 4, kKC16 = 16, kStages = 3;
 struct __align__(128) Stage {
-    double v[2][kKC * 9 * kSlice];  // BF16 values use the first quarter of each buffer
-    int col[2][kKC * kSlice];
-    double red[32][32];             // [warp][load case] partial sums
+    unsigned char v[kStages][kKC64 * 9 * kSlice * 8];
+    int col[kStages][kKC16 * kSlice];
+    BSlice rec[3];
+    unsigned long long bx, bv[kStages];
 };
 static_assert(sizeof(Stage::v) >= 6 * 32 * 32 * sizeof(float), "the restriction's per-warp sums fit in the stage");
+static_assert(kKC16 / 4 * 9 * kSlice * 8 <= sizeof(Stage::v[0]), "a BF16 chunk fits a buffer");
+
+// Partial sums of a slice: [sum][warp][load case].
+__host__ __device__ constexpr int red_bytes(int np, int rl) { return 2 * (np / rl) * np * 8; }
+
+// The mbarriers' phase parities (the same in every thread).
+struct Pipe {
+    unsigned px = 0, pv = 0;
+};
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void stage_init(Stage &st, int *s_fail) {
+    if (threadIdx.x == 0) {
+        *s_fail = 0;
+        asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(&st.bx)) : "memory");
+        for (int i = 0; i < kStages; ++i)
+            asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(&st.bv[i])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, unsigned long long *b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_addr(b))
+                 : "memory");
+}
+// Waits for the phase of parity `par`; gives up after limit_ns (the failure
+// is reported at the next grid barrier).
+__device__ __forceinline__ void mbar_wait(unsigned long long *b, unsigned par, unsigned long long limit_ns, int *s_fail) {
+    unsigned long long t0 = 0;
+    for (;;) {
+        unsigned ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(smem_addr(b)), "r"(par)
+                     : "memory");
+        if (ok) return;
+        const unsigned long long t = global_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > limit_ns) {
+            *s_fail = 1;
+            return;
+        }
+    }
+}
 
 // Bulk prefetch of [p, p + bytes) from HBM into L2 (no data returned, no
 // completion to wait for).  p and bytes are multiples of 16 (the BSELL slot
@@ -222,121 +253,246 @@ __device__ __forceinline__ void l2_prefetch(const void *p, long bytes) {
     }
 }
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Start copying slots [k0, k0 + kc) of the slice at S into buffer b (16-byte
-// pieces: every chunk is a multiple of 16 bytes at a 16-byte-aligned offset).
-template <class ST>
-__device__ __forceinline__ void stage_chunk(Stage &st, int b, long S, int k0, int kc, const int *__restrict__ scols,
-                                            const ST *__restrict__ svals) {
-    const char *gv = reinterpret_cast<const char *>(svals + (S + k0) * 9L * kSlice);
-    char *sv = reinterpret_cast<char *>(st.v[b]);
-    const int nv = kc * 9 * kSlice * (int)sizeof(ST) / 16;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) cp_async16(sv + 16 * i, gv + 16 * i);
-    const char *gc = reinterpret_cast<const char *>(scols + (S + k0) * (long)kSlice);
-    char *sc = reinterpret_cast<char *>(st.col[b]);
-    const int nc = kc * kSlice * 4 / 16;
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) cp_async16(sc + 16 * i, gc + 16 * i);
-    cp_async_commit();
-}
-
-// A staged matrix value in the arithmetic type V.
-template <class V, class ST>
-__device__ __forceinline__ V staged_val(const ST &a) {
-    if constexpr (std::is_same<ST, __nv_bfloat16>::value) return (V)__bfloat162float(a);
-    else return (V)a;
-}
-
-// y[c][q] = (K x)_(row, c) for this thread's RL load cases.  The slice's
-// slots (stored as ST: FP64, or BF16 read into FP32 arithmetic) stream
-// through shared memory kKC at a time, double-buffered, shared by every load
-// case; each staged value feeds RL FMAs.  xf(col, c, out[RL]) loads the
-// operand.  Called by all threads of the CTA (rows beyond nfree read
-// padding: column 0, value 0).
-template <class V, class ST, int NP, int RL, class XF>
-__device__ __forceinline__ void spmm_slice(Stage &st, long S, int W, const int *__restrict__ scols,
-                                           const ST *__restrict__ svals, XF xf, V (&y)[3][RL]) {
-    const int r = Lanes<NP, RL>::row();
+// acc[q] += m * x[q] for RL load cases; pairs in one packed FP32 FMA.
+template <int RL>
+__device__ __forceinline__ void fma_cases(float (&acc)[RL], float m, const float (&x)[RL]) {
+    if constexpr (RL % 2 == 0) {
+        unsigned long long mm;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(mm) : "f"(m));
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int q = 0; q < RL; ++q) y[c][q] = 0;
-    const int nch = (W + kKC - 1) / kKC;
-    __syncthreads();  // both buffers are free
-    if (nch > 0) stage_chunk<ST>(st, 0, S, 0, min(kKC, W), scols, svals);
-    for (int ch = 0; ch < nch; ++ch) {
-        const int b = ch & 1, k0 = ch * kKC, kc = min(kKC, W - k0);
-        if (ch + 1 < nch) {
-            stage_chunk<ST>(st, b ^ 1, S, k0 + kKC, min(kKC, W - k0 - kKC), scols, svals);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+        for (int q = 0; q < RL; q += 2) {
+            unsigned long long av, xv;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(av) : "f"(acc[q]), "f"(acc[q + 1]));
+            asm("mov.b64 %0, {%1, %2};" : "=l"(xv) : "f"(x[q]), "f"(x[q + 1]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(av) : "l"(mm), "l"(xv));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[q]), "=f"(acc[q + 1]) : "l"(av));
         }
-        __syncthreads();
-        const ST *sv = reinterpret_cast<const ST *>(st.v[b]);
-        // A full chunk runs without per-slot guards, so the compiler can
-        // hoist its gathers (measured 13 % faster per batched solve).
-        auto run = [&](auto full_t) {
-            constexpr bool FULL = decltype(full_t)::value;
+    } else {
 #pragma unroll
-            for (int k2 = 0; k2 < kKC; k2 += 2) {
-                V x[2][3][RL];
+        for (int q = 0; q < RL; ++q) acc[q] = fmaf(m, x[q], acc[q]);
+    }
+}
+template <int RL, class X>
+__device__ __forceinline__ void fma_cases(double (&acc)[RL], double m, const X (&x)[RL]) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u)
-                    if (FULL || k2 + u < kc) {
-                        const int col = st.col[b][(k2 + u) * kSlice + r];
-                        xf(col, 0, x[u][0]);
-                        xf(col, 1, x[u][1]);
-                        xf(col, 2, x[u][2]);
-                    }
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-                    if (FULL || k2 + u < kc) {
-                        const ST *v = sv + (k2 + u) * 9 * kSlice + r;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const V a0 = staged_val<V>(v[(3 * c) * kSlice]),
-                                    a1 = staged_val<V>(v[(3 * c + 1) * kSlice]),
-                                    a2 = staged_val<V>(v[(3 * c + 2) * kSlice]);
-#pragma unroll
-                            for (int q = 0; q < RL; ++q)
-                                y[c][q] = fma(a0, x[u][0][q], fma(a1, x[u][1][q], fma(a2, x[u][2][q], y[c][q])));
-                        }
-                    }
+    for (int q = 0; q < RL; ++q) acc[q] = fma(m, (double)x[q], acc[q]);
+}
+
+// y[c][q] = (K x)_(row, c) for this thread's RL load cases, for every slice of
+// this CTA in turn, then fin(slice record, slice index, live mask, y).
+//
+// A slice's 32 rows name each of their columns about four times (200 to 400
+// distinct columns against 864 slots on a structured C3D8 block), so the
+// distinct columns' entries (3 NP values each; consecutive columns are one
+// contiguous run) are copied to shared memory once and gathered from there:
+// gathered through L2 the products were bound by latency, about 600 cycles
+// per slot and warp.  Values stream through three buffers shared by every
+// load case (FP64 planes, or the grouped BF16 copy, whose 8-byte words bring
+// four slots of a plane at once).  All copies are bulk copies issued by warp 0
+// (16-byte cp.async of every thread took 4,700 cycles a slice to issue), and
+// the next slice's start as soon as this slice's product is formed, under
+// fin; pf(next record) prefetches what fin will read then.  A slice without a
+// column list, or with one beyond the buffer (cap), gathers its columns
+// directly.  Slices whose load cases have all stopped are skipped.
+// Measured on 16 variants of 17.6k nodes on average x 16 load cases (ms per
+// phase and iteration, before -> after): FP64 product 0.359 -> 0.304,
+// residual 0.254 -> 0.170, post-smoothing 0.309 -> 0.210; iteration 1.207 ->
+// 0.940.  What bounds them now: the FP64 product's shared-memory reads (values
+// nine per slot and warp) with two CTAs per SM to cover the rest of a slice.
+//   T: arithmetic type, X: operand type, BF: values from the BF16 copy.
+template <class T, class X, bool BF, int NP, int RL, class Pf, class Fin>
+__device__ __forceinline__ void matrix_phase(const BArgs &a, Stage &st, Pipe &pipe, unsigned char *dyn, int cap, int *s_fail,
+                                             const X *x, bool all, Pf pf, Fin fin) {
+    constexpr int KC = BF ? kKC16 : kKC64;
+    constexpr int kColBytes = 3 * NP * (int)sizeof(X);
+    constexpr int kPieces = (int)sizeof(BSlice) / 16;
+    const int r = Lanes<NP, RL>::row(), j0 = Lanes<NP, RL>::j0();
+    const int lane = threadIdx.x & 31;
+    const bool warp0 = threadIdx.x < 32;
+    X *xs = reinterpret_cast<X *>(dyn + red_bytes(NP, RL));
+    int gsl = blockIdx.x;
+    if (gsl >= a.nslices) return;
+    auto is_staged = [&](const BSlice &R) { return R.nu > 0 && R.nu <= cap; };
+    // values and column positions of chunk ch (one thread)
+    auto issue_chunk = [&](const BSlice &R, int ch) {
+        const int k0 = ch * KC, kc = min(KC, R.W - k0), b = ch % kStages;
+        const unsigned nv = (BF ? (kc + 3) / 4 : kc) * (9 * kSlice * 8);
+        const bool sg = is_staged(R);
+        const unsigned nc = kc * kSlice * (sg ? 2 : 4);
+        mbar_expect(&st.bv[b], nv + nc);
+        if (BF) bulk_copy(st.v[b], R.vg + (long)k0 * 9 * kSlice, nv, &st.bv[b]);
+        else bulk_copy(st.v[b], R.v64 + (long)k0 * 9 * kSlice, nv, &st.bv[b]);
+        if (sg) bulk_copy(st.col[b], R.lidx + k0 * kSlice, nc, &st.bv[b]);
+        else bulk_copy(st.col[b], R.cols + k0 * kSlice, nc, &st.bv[b]);
+    };
+    // the start of a slice (warp 0): its first chunks and its columns' entries;
+    // r0, r1: the slice's runs lane and lane + 32
+    auto issue = [&](const BSlice &R, int2 r0, int2 r1) {
+        if (lane == 0) {
+            if (is_staged(R)) mbar_expect(&st.bx, R.nu * kColBytes);
+            for (int ch = 0; ch < kStages && ch * KC < R.W; ++ch) issue_chunk(R, ch);
+        }
+        __syncwarp();
+        if (is_staged(R)) {
+            const X *xv = x + R.dof * NP;
+            for (int i = lane; i < R.nrun; i += 32) {
+                const int2 q = i < 32 ? r0 : i < 64 ? r1 : R.runs[i];
+                bulk_copy(reinterpret_cast<char *>(xs) + (q.y >> 16) * kColBytes, xv + 3L * q.x * NP, (q.y & 0xffff) * kColBytes,
+                          &st.bx);
             }
-        };
-        if (kc == kKC) run(std::true_type{});
-        else run(std::false_type{});
-        __syncthreads();  // buffer b is consumed before it is refilled
+        }
+    };
+    auto load_runs = [&](const BSlice &R, int2 &r0, int2 &r1) {
+        r0 = r1 = make_int2(0, 0);
+        if (is_staged(R)) {
+            if (lane < R.nrun) r0 = R.runs[lane];
+            if (lane + 32 < R.nrun) r1 = R.runs[lane + 32];
+        }
+    };
+    __syncthreads();  // the phase before is done with the stage
+    int2 r0 = make_int2(0, 0), r1 = r0;
+    if (warp0) {
+        // the bulk copies read what earlier phases stored, and write where they wrote
+        asm volatile("fence.proxy.async;" ::: "memory");
+        if (lane < kPieces) reinterpret_cast<int4 *>(&st.rec[0])[lane] = reinterpret_cast<const int4 *>(a.slice + gsl)[lane];
+        __syncwarp();
+        load_runs(st.rec[0], r0, r1);
+    }
+    __syncthreads();
+    unsigned mask = all ? 0xffffffffu : a.vmask[st.rec[0].v], mask_next = 0;
+    if (warp0 && mask) issue(st.rec[0], r0, r1);
+    for (int cur = 0; gsl < a.nslices; gsl += gridDim.x, cur = cur == 2 ? 0 : cur + 1, mask = mask_next) {
+        const BSlice &R = st.rec[cur], &Rn = st.rec[cur == 2 ? 0 : cur + 1];
+        const bool more = gsl + (int)gridDim.x < a.nslices;
+        int4 piece = make_int4(0, 0, 0, 0);
+        if (more && threadIdx.x < kPieces) piece = reinterpret_cast<const int4 *>(a.slice + gsl + gridDim.x)[threadIdx.x];
+        const int W = R.W, nch = mask ? (W + KC - 1) / KC : 0;
+        const bool staged = is_staged(R);
+        const X *xv = x + R.dof * NP;
+        T y[3][RL];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int q = 0; q < RL; ++q) y[c][q] = 0;
+        if (mask && staged) {
+            mbar_wait(&st.bx, pipe.px, a.limit_ns, s_fail);
+            pipe.px ^= 1;
+        }
+        if (more && warp0) {  // the next slice's record and runs
+            if (lane < kPieces) reinterpret_cast<int4 *>(const_cast<BSlice *>(&Rn))[lane] = piece;
+            __syncwarp();
+            load_runs(Rn, r0, r1);
+        }
+        for (int ch = 0; ch < nch; ++ch) {
+            const int b = ch % kStages, kc = min(KC, W - ch * KC);
+            mbar_wait(&st.bv[b], (pipe.pv >> b) & 1u, a.limit_ns, s_fail);
+            pipe.pv ^= 1u << b;
+            const double *v64 = reinterpret_cast<const double *>(st.v[b]) + r;
+            const uint2 *v16 = reinterpret_cast<const uint2 *>(st.v[b]) + r;
+            auto run = [&](auto staged_t) {
+                constexpr bool ST = decltype(staged_t)::value;
+                auto operand = [&](int k, X (&o)[3][RL]) {
+                    const X *p;
+                    if constexpr (ST) p = xs + (reinterpret_cast<const uint16_t *>(st.col[b])[k * kSlice + r] * 3) * NP + j0;
+                    else p = xv + 3L * st.col[b][k * kSlice + r] * NP + j0;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) ldv<X, RL>(p + c * NP, o[c]);
+                };
+                // four slots from k on (full: without per-slot guards, so their
+                // loads are all issued before the first FMA)
+                auto four = [&](int k, auto full_t) {
+                    constexpr bool FULL = decltype(full_t)::value;
+                    constexpr int H = RL == 4 && !BF ? 1 : 2;  // slots in flight
+                    [[maybe_unused]] uint2 raw[BF ? 9 : 1];
+                    if constexpr (BF) {
+#pragma unroll
+                        for (int e = 0; e < 9; ++e) raw[e] = v16[((k >> 2) * 9 + e) * kSlice];
+                    }
+#pragma unroll
+                    for (int h = 0; h < 4; h += H) {
+                        X o[H][3][RL];
+#pragma unroll
+                        for (int u = 0; u < H; ++u)
+                            if (FULL || k + h + u < kc) operand(k + h + u, o[u]);
+#pragma unroll
+                        for (int u = 0; u < H; ++u)
+                            if (FULL || k + h + u < kc)
+#pragma unroll
+                                for (int i = 2; i >= 0; --i)
+#pragma unroll
+                                    for (int c = 0; c < 3; ++c) {
+                                        if constexpr (BF) {
+                                            const unsigned w = (h + u) < 2 ? raw[3 * c + i].x : raw[3 * c + i].y;
+                                            fma_cases<RL>(y[c], __uint_as_float(((h + u) & 1) ? (w & 0xFFFF0000u) : (w << 16)),
+                                                          o[u][i]);
+                                        } else {
+                                            fma_cases<RL>(y[c], v64[((k + h + u) * 9 + 3 * c + i) * kSlice], o[u][i]);
+                                        }
+                                    }
+                    }
+                };
+                int k = 0;
+                if constexpr (ST) {
+#pragma unroll 1
+                    for (; k + 4 <= kc; k += 4) four(k, std::true_type{});
+                }
+#pragma unroll 1
+                for (; k < kc; k += 4) four(k, std::false_type{});
+            };
+            if (staged) run(std::true_type{});
+            else run(std::false_type{});
+            if (ch + kStages < nch) {  // this buffer takes a later chunk
+                __syncthreads();
+                if (threadIdx.x == 0) issue_chunk(R, ch + kStages);
+            }
+        }
+        __syncthreads();  // the product is formed: the stage is free, the next record is in place
+        if (more) {
+            mask_next = all ? 0xffffffffu : a.vmask[Rn.v];
+            if (mask_next) {
+                if (warp0) issue(Rn, r0, r1);
+                else if (threadIdx.x == 32) pf(Rn);
+            }
+        }
+        if (mask) fin(R, gsl, mask, y);
     }
 }
 
-// Sums of p[q] over the CTA's 32 rows for each of this thread's load cases,
-// stored as P[gsl * NR + j] for j < NR (fixed order: lanes, then warps).
+// Sums of p[q] (and p2[q] unless P2 is null) over the CTA's 32 rows for each
+// of this thread's load cases, stored as P[gsl * NR + j] for j < NR (fixed
+// order: lanes, then warps).
 template <int NP, int RL>
-__device__ __forceinline__ void slice_partial(Stage &st, double (&p)[RL], double *P, int gsl, int NR) {
+__device__ __forceinline__ void slice_partial(unsigned char *dyn, double (&p)[RL], double *P, double (&p2)[RL], double *P2, int gsl,
+                                              int NR) {
     constexpr int LW = Lanes<NP, RL>::kLW;
 #pragma unroll
     for (int q = 0; q < RL; ++q)
 #pragma unroll
-        for (int off = LW; off < 32; off <<= 1) p[q] += __shfl_xor_sync(0xffffffffu, p[q], off);
+        for (int off = LW; off < 32; off <<= 1) {
+            p[q] += __shfl_xor_sync(0xffffffffu, p[q], off);
+            if (P2) p2[q] += __shfl_xor_sync(0xffffffffu, p2[q], off);
+        }
+    constexpr int kW = Lanes<NP, RL>::kWarps;
+    double *red = reinterpret_cast<double *>(dyn);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     __syncthreads();
     if (lane < LW)
 #pragma unroll
-        for (int q = 0; q < RL; ++q) st.red[w][lane * RL + q] = p[q];
+        for (int q = 0; q < RL; ++q) {
+            red[w * NP + lane * RL + q] = p[q];
+            if (P2) red[(kW + w) * NP + lane * RL + q] = p2[q];
+        }
     __syncthreads();
-    if ((int)threadIdx.x < NR) {
+    const int h = threadIdx.x / NP, j = threadIdx.x % NP;
+    if (h < (P2 ? 2 : 1) && j < NR) {
         double s = 0;
-        for (int ww = 0; ww < Lanes<NP, RL>::kWarps; ++ww) s += st.red[ww][threadIdx.x];
-        P[(long)gsl * NR + threadIdx.x] = s;
+        for (int ww = 0; ww < kW; ++ww) s += red[(h * kW + ww) * NP + j];
+        (h ? P2 : P)[(long)gsl * NR + j] = s;
     }
+}
+template <int NP, int RL>
+__device__ __forceinline__ void slice_partial(unsigned char *dyn, double (&p)[RL], double *P, int gsl, int NR) {
+    slice_partial<NP, RL>(dyn, p, P, p, nullptr, gsl, NR);
 }
 
 // Reduce phase: one warp per (variant, load case); f(v, j, sum_pa, sum_pb).
@@ -361,25 +517,28 @@ __device__ __forceinline__ void for_pairs(const BArgs &a, bool two, F f) {
 
 // The persistent batched solver.  MIXED: FP64 FCG + FP32 V-cycle; else PCG64.
 // One CTA per slice item (grid-stride); NP / RL lanes per block row, RL load
-// cases per lane.  The PCG64 instances are held to 3 (RL <= 2) or 2 CTAs per
-// SM worth of registers and MIXED with RL = 2 to 2 (measured faster than the
-// compiler's choice); the other MIXED ones keep theirs (bounds spill and
-// measured slower).
-constexpr int batch_min_ctas(int threads, int rl, bool mixed) {
-    return mixed ? (rl == 2 ? 2 : 1) : ((rl <= 2 ? 3 : 2) * threads <= 2048 ? (rl <= 2 ? 3 : 2) : 2048 / threads);
-}
+// cases per lane.  Shared memory lets two CTAs share an SM, so the instances
+// of up to 256 threads are compiled for two (128 registers).
+constexpr int batch_min_ctas(int threads) { return threads <= 256 ? 2 : 1; }
 template <int NP, int RL, bool MIXED>
-__global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL), RL, MIXED)) k_batch_solve(BArgs a) {
+__global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))) k_batch_solve(BArgs a) {
     __shared__ Stage st;
+    __shared__ int s_fail;
+    extern __shared__ __align__(16) unsigned char dyn[];
     using LN = Lanes<NP, RL>;
+    using ZT = typename std::conditional<MIXED, float, double>::type;  // the outer product's operand
     const unsigned nb = gridDim.x + a.extra_arrivals;
+    unsigned target = 0;
+    Pipe pipe;
+    stage_init(st, &s_fail);
     const int NR = a.NR;
     const int r = LN::row(), j0 = LN::j0();
     const bool tracer = a.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     int tn = 0;
     if (tracer && tn < a.trace_cap) a.trace[tn++] = global_ns();
     auto sync = [&]() {
-        const bool ok = grid_barrier(a.gs, nb, a.limit_ns);
+        target += nb;
+        const bool ok = grid_barrier(a.gs, target, a.limit_ns, &s_fail);
         if (tracer && tn < a.trace_cap) a.trace[tn++] = global_ns();
         return ok;
     };
@@ -409,6 +568,10 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
             f(B, v, gsl, ls, row, live, any);
         }
     };
+    auto stop = [&](int v, int jj) {  // load case jj of variant v stops
+        a.live[v * NR + jj] = 0;
+        atomicAnd(&a.vmask[v], ~(1u << jj));
+    };
     auto for_slices = [&](auto f) { for_slices_pf([](const BVar &, int) {}, f); };
     // Prefetch pieces for a slice lsn of variant Bn: the rows' runs of a batch
     // vector (esize bytes per entry), the rows' inverse diagonal blocks (FP32
@@ -432,24 +595,29 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
     };
 
     // ---- init: r = f - K u, partials ||r||^2 (pa), ||f||^2 (pb); start of M(r)
-    for_slices([&](const BVar &B, int v, int gsl, int ls, int row, const bool (&)[RL], bool) {
-        const int S = B.sl_ptr[ls], W = B.sl_ptr[ls + 1] - S;
-        double y[3][RL];
-        spmm_slice<double, double, NP, RL>(st, S, W, B.scols, B.sv64,
-                                   [&](int k, int c, double (&o)[RL]) { ldv<double, RL>(a.u + vidx<NP>(B, k, c, j0), o); }, y);
+    // prefetch into L2 of the next slice's rows of a vector (esize bytes per entry)
+    auto pf_vec = [&](const BSlice &R, const void *base, int esize) {
+        l2_prefetch(static_cast<const char *>(base) + (R.dof + 3L * R.row0) * NP * esize,
+                    3L * min(kSlice, R.nfree - R.row0) * NP * esize);
+    };
+    auto XR = [&](const BSlice &R, int row, int c) { return (R.dof + 3L * row + c) * NP + j0; };
+    // MIXED gathers the FP64 u directly: the stage is sized for the iteration's operand
+    matrix_phase<double, double, false, NP, RL>(a, st, pipe, dyn, MIXED ? 0 : a.cap, &s_fail, a.u, true, [](const BSlice &) {},
+                                                [&](const BSlice &B, int gsl, unsigned, double (&y)[3][RL]) {
+        const int row = B.row0 + r;
         double prr[RL] = {}, pff[RL] = {};
         if (row < B.nfree) {
             double rv[3][RL];
             for (int c = 0; c < 3; ++c) {
                 double fv[RL];
-                ldv<double, RL>(a.f + X(B, row, c), fv);
+                ldv<double, RL>(a.f + XR(B, row, c), fv);
 #pragma unroll
                 for (int q = 0; q < RL; ++q) {
                     rv[c][q] = fv[q] - y[c][q];
                     prr[q] += rv[c][q] * rv[c][q];
                     pff[q] += fv[q] * fv[q];
                 }
-                stv<double, RL>(a.r + X(B, row, c), rv[c]);
+                stv<double, RL>(a.r + XR(B, row, c), rv[c]);
             }
             if (MIXED) {
                 float b[3][RL], x[3][RL];
@@ -464,8 +632,8 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                     }
                 }
                 for (int c = 0; c < 3; ++c) {
-                    stv<float, RL>(a.b32 + X(B, row, c), b[c]);
-                    stv<float, RL>(a.x32 + X(B, row, c), x[c]);
+                    stv<float, RL>(a.b32 + XR(B, row, c), b[c]);
+                    stv<float, RL>(a.x32 + XR(B, row, c), x[c]);
                 }
             } else {
                 double z[3][RL];
@@ -476,11 +644,10 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                     block3_apply(B.Dinv + 9L * row, rr, zz);
                     for (int c = 0; c < 3; ++c) z[c][q] = zz[c];
                 }
-                for (int c = 0; c < 3; ++c) stv<double, RL>(a.z64 + X(B, row, c), z[c]);
+                for (int c = 0; c < 3; ++c) stv<double, RL>(a.z64 + XR(B, row, c), z[c]);
             }
         }
-        slice_partial<NP, RL>(st, prr, a.pa, gsl, NR);
-        slice_partial<NP, RL>(st, pff, a.pb, gsl, NR);
+        slice_partial<NP, RL>(dyn, prr, a.pa, pff, a.pb, gsl, NR);
     });
     if (!sync()) return;
     for_pairs(a, true, [&](int v, int jj, double rr, double ff) {
@@ -489,6 +656,7 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
         const double t = 0.5 * a.rtol;
         a.tol2[vj] = t * t * ff;
         a.live[vj] = (ff > 0.0 && rr > a.tol2[vj] && isfinite(rr)) ? 1 : 0;
+        if (a.live[vj]) atomicOr(&a.vmask[v], 1u << jj);
         a.iters[vj] = 0;
         a.status[vj] = isfinite(rr) ? OFEA_OK : OFEA_ERR_BREAKDOWN;
         a.beta[vj] = 0.0;
@@ -500,18 +668,17 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
     // call sites: a call would put every captured local on the stack.
     auto precondition = [&](float *znew, const float *zold) __attribute__((always_inline)) -> bool {
         // t = b - K32 x
-        for_slices([&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
-            const int S = B.sl_ptr[ls], W = B.sl_ptr[ls + 1] - S;
-            float y[3][RL];
-            spmm_slice<float, __nv_bfloat16, NP, RL>(st, S, W, B.scols, B.sv16,
-                                      [&](int k, int c, float (&o)[RL]) { ldv<float, RL>(a.x32 + vidx<NP>(B, k, c, j0), o); }, y);
-            if (any && row < B.nfree)
+        matrix_phase<float, float, true, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, a.x32, false,
+                                                 [&](const BSlice &Rn) { pf_vec(Rn, a.b32, 4); },
+                                                 [&](const BSlice &B, int, unsigned mask, float (&y)[3][RL]) {
+            const int row = B.row0 + r;
+            if (((mask >> j0) & ((1u << RL) - 1)) && row < B.nfree)
                 for (int c = 0; c < 3; ++c) {
                     float bv[RL], t[RL];
-                    ldv<float, RL>(a.b32 + X(B, row, c), bv);
+                    ldv<float, RL>(a.b32 + XR(B, row, c), bv);
 #pragma unroll
                     for (int q = 0; q < RL; ++q) t[q] = bv[q] - y[c][q];
-                    stv<float, RL>(a.t32 + X(B, row, c), t);
+                    stv<float, RL>(a.t32 + XR(B, row, c), t);
                 }
         });
         if (!sync()) return false;
@@ -530,13 +697,8 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                 const bool live = jj < NR && a.live[v * NR + jj] != 0;
                 float acc[6] = {0, 0, 0, 0, 0, 0};
                 if (live) {
-                    const float cx = (float)B.centroid[3L * I], cy = (float)B.centroid[3L * I + 1],
-                                cz = (float)B.centroid[3L * I + 2];
-                    const float sc = (float)B.inv_scale;
-                    auto add = [&](int node, float tx, float ty, float tz) {
-                        const float dx = ((float)B.xyz[3L * node] - cx) * sc;
-                        const float dy = ((float)B.xyz[3L * node + 1] - cy) * sc;
-                        const float dz = ((float)B.xyz[3L * node + 2] - cz) * sc;
+                    auto add = [&](const float4 &o, float tx, float ty, float tz) {
+                        const float dx = o.x, dy = o.y, dz = o.z;
                         acc[0] += tx;
                         acc[1] += ty;
                         acc[2] += tz;
@@ -547,23 +709,21 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                     const int e = B.agg_ptr[I + 1];
                     int idx = B.agg_ptr[I] + sub;
                     for (; idx + (kU - 1) * G < e; idx += kU * G) {
-                        int rr[kU], node[kU];
+                        float4 o[kU];
                         float t[kU][3];
 #pragma unroll
-                        for (int u = 0; u < kU; ++u) rr[u] = B.agg_nodes[idx + u * G];
+                        for (int u = 0; u < kU; ++u) o[u] = __ldg(B.agg_off + idx + u * G);
 #pragma unroll
-                        for (int u = 0; u < kU; ++u) {
-                            node[u] = B.node_of_free[rr[u]];
+                        for (int u = 0; u < kU; ++u)
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) t[u][c] = a.t32[vidx<NP>(B, rr[u], c, jj)];
-                        }
+                            for (int c = 0; c < 3; ++c) t[u][c] = a.t32[vidx<NP>(B, __float_as_int(o[u].w), c, jj)];
 #pragma unroll
-                        for (int u = 0; u < kU; ++u) add(node[u], t[u][0], t[u][1], t[u][2]);
+                        for (int u = 0; u < kU; ++u) add(o[u], t[u][0], t[u][1], t[u][2]);
                     }
                     for (; idx < e; idx += G) {
-                        const int rr = B.agg_nodes[idx];
-                        add(B.node_of_free[rr], a.t32[vidx<NP>(B, rr, 0, jj)], a.t32[vidx<NP>(B, rr, 1, jj)],
-                            a.t32[vidx<NP>(B, rr, 2, jj)]);
+                        const float4 o = __ldg(B.agg_off + idx);
+                        const int rr = __float_as_int(o.w);
+                        add(o, a.t32[vidx<NP>(B, rr, 0, jj)], a.t32[vidx<NP>(B, rr, 1, jj)], a.t32[vidx<NP>(B, rr, 2, jj)]);
                     }
                 }
 #pragma unroll
@@ -612,10 +772,9 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
             },
             [&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
             if (!any || row >= B.nfree) return;
-            const int I = B.agg_of[row], node = B.node_of_free[row];
-            const float dx = (float)((B.xyz[3L * node] - B.centroid[3L * I]) * B.inv_scale);
-            const float dy = (float)((B.xyz[3L * node + 1] - B.centroid[3L * I + 1]) * B.inv_scale);
-            const float dz = (float)((B.xyz[3L * node + 2] - B.centroid[3L * I + 2]) * B.inv_scale);
+            const float4 o = __ldg(B.row_off + row);
+            const int I = __float_as_int(o.w);
+            const float dx = o.x, dy = o.y, dz = o.z;
             float e[6][RL], x[3][RL];
             for (int k = 0; k < 6; ++k) ldv<float, RL>(a.evec + (B.c0 + 6L * I + k) * NP + j0, e[k]);
             for (int c = 0; c < 3; ++c) ldv<float, RL>(a.x32 + X(B, row, c), x[c]);
@@ -629,21 +788,27 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
         });
         if (!sync()) return false;
         // post-smoothing: z_new = x + w Dinv32 (b - K32 x); partials r.z_new, r.z_old
-        for_slices([&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
-            const int S = B.sl_ptr[ls], W = B.sl_ptr[ls + 1] - S;
-            float y[3][RL];
-            spmm_slice<float, __nv_bfloat16, NP, RL>(st, S, W, B.scols, B.sv16,
-                                      [&](int k, int c, float (&o)[RL]) { ldv<float, RL>(a.x32 + vidx<NP>(B, k, c, j0), o); }, y);
+        matrix_phase<float, float, true, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, a.x32, false,
+                                                 [&](const BSlice &Rn) {
+                                                     pf_vec(Rn, a.b32, 4);
+                                                     pf_vec(Rn, a.r, 8);
+                                                     if (zold) pf_vec(Rn, zold, 4);
+                                                 },
+                                                 [&](const BSlice &B, int gsl, unsigned mask, float (&y)[3][RL]) {
+            const int row = B.row0 + r;
+            bool live[RL], any = false;
+#pragma unroll
+            for (int q = 0; q < RL; ++q) any |= live[q] = (mask >> (j0 + q)) & 1u;
             double pn[RL] = {}, po[RL] = {};
             if (any && row < B.nfree) {
                 float res[3][RL], xv[3][RL], zn[3][RL], zo[3][RL];
                 double rv[3][RL];
                 for (int c = 0; c < 3; ++c) {
                     float bv[RL];
-                    ldv<float, RL>(a.b32 + X(B, row, c), bv);
-                    ldv<float, RL>(a.x32 + X(B, row, c), xv[c]);
-                    ldv<double, RL>(a.r + X(B, row, c), rv[c]);
-                    if (zold) ldv<float, RL>(zold + X(B, row, c), zo[c]);
+                    ldv<float, RL>(a.b32 + XR(B, row, c), bv);
+                    ldv<float, RL>(a.x32 + XR(B, row, c), xv[c]);
+                    ldv<double, RL>(a.r + XR(B, row, c), rv[c]);
+                    if (zold) ldv<float, RL>(zold + XR(B, row, c), zo[c]);
 #pragma unroll
                     for (int q = 0; q < RL; ++q) res[c][q] = bv[q] - y[c][q];
                 }
@@ -660,10 +825,9 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                         }
                     }
                 }
-                for (int c = 0; c < 3; ++c) stv<float, RL>(znew + X(B, row, c), zn[c]);
+                for (int c = 0; c < 3; ++c) stv<float, RL>(znew + XR(B, row, c), zn[c]);
             }
-            slice_partial<NP, RL>(st, pn, a.pa, gsl, NR);
-            slice_partial<NP, RL>(st, po, a.pb, gsl, NR);
+            slice_partial<NP, RL>(dyn, pn, a.pa, po, a.pb, gsl, NR);
         });
         return sync();
     };
@@ -683,7 +847,7 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
 #pragma unroll
                     for (int q = 0; q < RL; ++q) p[q] += rv[q] * zv[q];
                 }
-            slice_partial<NP, RL>(st, p, a.pa, gsl, NR);
+            slice_partial<NP, RL>(dyn, p, a.pa, gsl, NR);
         });
         if (!sync()) return;
     }
@@ -697,28 +861,36 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
         // slot (k + 1) % 3 was last read two barriers ago at least
         if (blockIdx.x == 0 && threadIdx.x == 0) a.live_cnt[(k + 1) % 3] = 0;
         // A: p = z + beta p_old, q = K64 z + beta q_old (= K64 p), partial p.q
-        for_slices([&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
-            const int S = B.sl_ptr[ls], W = B.sl_ptr[ls + 1] - S;
+        auto zval = [&](long d, double (&o)[RL]) {
+            if (MIXED) {
+                float zf[RL];
+                ldv<float, RL>(zcur + d, zf);
+#pragma unroll
+                for (int q = 0; q < RL; ++q) o[q] = (double)zf[q];
+            } else {
+                ldv<double, RL>(a.z64 + d, o);
+            }
+        };
+        const ZT *zop;
+        if constexpr (MIXED) zop = zcur;
+        else zop = a.z64;
+        matrix_phase<double, ZT, false, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, zop, false,
+                                                [&](const BSlice &Rn) {
+                                                    pf_vec(Rn, pold, 8);
+                                                    pf_vec(Rn, a.q, 8);
+                                                },
+                                                [&](const BSlice &B, int gsl, unsigned mask, double (&y)[3][RL]) {
+            const int v = B.v, row = B.row0 + r;
+            bool live[RL], any = false;
+#pragma unroll
+            for (int q = 0; q < RL; ++q) any |= live[q] = (mask >> (j0 + q)) & 1u;
             double bt[RL];
 #pragma unroll
             for (int q = 0; q < RL; ++q) bt[q] = live[q] ? a.beta[v * NR + j0 + q] : 0.0;
-            auto zval = [&](long d, double (&o)[RL]) {
-                if (MIXED) {
-                    float zf[RL];
-                    ldv<float, RL>(zcur + d, zf);
-#pragma unroll
-                    for (int q = 0; q < RL; ++q) o[q] = (double)zf[q];
-                } else {
-                    ldv<double, RL>(a.z64 + d, o);
-                }
-            };
-            double y[3][RL];
-            spmm_slice<double, double, NP, RL>(st, S, W, B.scols, B.sv64,
-                                       [&](int kk, int c, double (&o)[RL]) { zval(vidx<NP>(B, kk, c, j0), o); }, y);
             double ppq[RL] = {};
             if (any && row < B.nfree)
                 for (int c = 0; c < 3; ++c) {
-                    const long d = X(B, row, c);
+                    const long d = XR(B, row, c);
                     double zn[RL], po[RL], qo[RL], pn[RL], qn[RL];
                     zval(d, zn);
                     ldv<double, RL>(pold + d, po);
@@ -732,14 +904,14 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                     stv<double, RL>(pnew + d, pn);
                     stv<double, RL>(a.q + d, qn);
                 }
-            slice_partial<NP, RL>(st, ppq, a.pa, gsl, NR);
+            slice_partial<NP, RL>(dyn, ppq, a.pa, gsl, NR);
         });
         if (!sync()) return;
         for_pairs(a, false, [&](int v, int jj, double pq, double) {
             const int vj = v * NR + jj;
             if (!a.live[vj]) return;
             if (!(pq > 0.0) || !isfinite(pq)) {
-                a.live[vj] = 0;
+                stop(v, jj);
                 a.status[vj] = OFEA_ERR_BREAKDOWN;
                 a.iters[vj] = k;
                 return;
@@ -811,8 +983,7 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
                     for (int c = 0; c < 3; ++c) stv<double, RL>(a.z64 + X(B, row, c), z[c]);
                 }
             }
-            slice_partial<NP, RL>(st, prr, a.pa, gsl, NR);
-            if (!MIXED) slice_partial<NP, RL>(st, prz, a.pb, gsl, NR);
+            slice_partial<NP, RL>(dyn, prr, a.pa, prz, MIXED ? nullptr : a.pb, gsl, NR);
         });
         if (!sync()) return;
         for_pairs(a, !MIXED, [&](int v, int jj, double rr, double rz) {
@@ -820,16 +991,16 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL),
             if (!a.live[vj]) return;
             a.iters[vj] = k + 1;
             if (!isfinite(rr)) {
-                a.live[vj] = 0;
+                stop(v, jj);
                 a.status[vj] = OFEA_ERR_BREAKDOWN;
                 return;
             }
             if (rr <= a.tol2[vj]) {
-                a.live[vj] = 0;
+                stop(v, jj);
                 return;
             }
             if (k + 1 >= a.max_iter) {
-                a.live[vj] = 0;
+                stop(v, jj);
                 a.status[vj] = OFEA_ERR_NOT_CONVERGED;
                 return;
             }
@@ -877,19 +1048,20 @@ template <int NP, int RL>
 __global__ void __launch_bounds__(32 * (NP / RL)) k_batch_residual(BArgs a) {
     __shared__ Stage st;
     using LN = Lanes<NP, RL>;
+    __shared__ int s_fail;
+    extern __shared__ __align__(16) unsigned char dyn[];
     const int NR = a.NR, j0 = LN::j0(), r = LN::row();
-    for (int gsl = blockIdx.x; gsl < a.nslices; gsl += gridDim.x) {
-        const BVar B = a.var[a.slice_var[gsl]];
-        const int ls = gsl - B.slice0, row = ls * kSlice + r;
-        const int S = B.sl_ptr[ls], W = B.sl_ptr[ls + 1] - S;
-        double y[3][RL];
-        spmm_slice<double, double, NP, RL>(st, S, W, B.scols, B.sv64,
-                                   [&](int k, int c, double (&o)[RL]) { ldv<double, RL>(a.u + vidx<NP>(B, k, c, j0), o); }, y);
+    Pipe pipe;
+    stage_init(st, &s_fail);
+    // u gathered directly: once per solve
+    matrix_phase<double, double, false, NP, RL>(a, st, pipe, dyn, 0, &s_fail, a.u, true, [](const BSlice &) {},
+                                                [&](const BSlice &B, int gsl, unsigned, double (&y)[3][RL]) {
+        const int row = B.row0 + r;
         double prr[RL] = {}, pff[RL] = {};
         if (row < B.nfree)
             for (int c = 0; c < 3; ++c) {
                 double fv[RL];
-                ldv<double, RL>(a.f + vidx<NP>(B, row, c, j0), fv);
+                ldv<double, RL>(a.f + (B.dof + 3L * row + c) * NP + j0, fv);
 #pragma unroll
                 for (int q = 0; q < RL; ++q) {
                     const double rv = fv[q] - y[c][q];
@@ -897,8 +1069,38 @@ __global__ void __launch_bounds__(32 * (NP / RL)) k_batch_residual(BArgs a) {
                     pff[q] += fv[q] * fv[q];
                 }
             }
-        slice_partial<NP, RL>(st, prr, a.pa, gsl, NR);
-        slice_partial<NP, RL>(st, pff, a.pb, gsl, NR);
+        slice_partial<NP, RL>(dyn, prr, a.pa, pff, a.pb, gsl, NR);
+    });
+    __syncthreads();
+    if (threadIdx.x == 0 && s_fail) a.gs->err = 1;
+}
+
+// The slices' records from the variants' descriptors.
+__global__ void k_batch_slices(int nslices, const BVar *__restrict__ var, const int *__restrict__ slice_var,
+                               BSlice *__restrict__ out) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nslices; g += gridDim.x * blockDim.x) {
+        const int v = slice_var[g];
+        const BVar &B = var[v];
+        const int ls = g - B.slice0;
+        const long S = B.sl_ptr[ls];
+        BSlice R;
+        R.v64 = B.sv64 + S * 9 * kSlice;
+        R.vg = B.sv16g + (long)B.sl_g[ls] * 9 * kSlice * 4;
+        R.cols = B.scols + S * kSlice;
+        R.runs = B.su_runs + S * kSlice;
+        R.lidx = B.su_idx + S * kSlice;
+        R.Dinv = B.Dinv;
+        R.Dinv32 = B.Dinv32;
+        R.dof = B.dof0;
+        R.W = B.sl_ptr[ls + 1] - (int)S;
+        R.nu = B.su_n[2 * ls];
+        R.nrun = B.su_n[2 * ls + 1];
+        R.row0 = ls * kSlice;
+        R.nfree = B.nfree;
+        R.v = v;
+        R.wsm = B.wsm;
+        R.pad = 0;
+        out[g] = R;
     }
 }
 
@@ -912,8 +1114,10 @@ __global__ void k_batch_rel(BArgs a, double *rel) {
 // A bounded wait that nothing releases: one extra arrival is expected at
 // the first barrier, so every CTA's wait runs out after limit_ns and the
 // kernel reports the failure (used to test the failure path).
-__global__ void k_barrier_probe(GridSync *gs, unsigned extra, unsigned long long limit_ns, int *out) {
-    const bool ok = grid_barrier(gs, gridDim.x + extra, limit_ns);
+__global__ void k_barrier_probe(GridBar *gs, unsigned extra, unsigned long long limit_ns, int *out) {
+    __shared__ int s_fail;
+    if (threadIdx.x == 0) s_fail = 0;
+    const bool ok = grid_barrier(gs, gridDim.x + extra, limit_ns, &s_fail);
     if (blockIdx.x == 0 && threadIdx.x == 0) *out = ok ? 1 : 0;
 }
 
@@ -952,12 +1156,24 @@ const void *solve_kernel_raw(int np, int rl, bool mixed) {
     }
     fail(OFEA_ERR_INVALID_ARG, "unsupported load-case stride");
 }
+// Dynamic shared memory of the staged products: the distinct columns' entries
+// of the operand (FP32 for MIXED, FP64 for PCG64).
+// At most what lets two CTAs share an SM (228 KB, 1 KB reserved per CTA).
+constexpr int kStageLimit = 112 * 1024 - (int)sizeof(Stage) - 256;  // partial sums included
+int col_bytes(int np, bool mixed) { return 3 * np * (mixed ? 4 : 8); }
+int stage_cap(int su_max, int np, int rl, bool mixed) {
+    return std::min(su_max, (kStageLimit - red_bytes(np, rl)) / col_bytes(np, mixed));
+}
+int stage_bytes(int su_max, int np, int rl, bool mixed) {
+    return red_bytes(np, rl) + stage_cap(su_max, np, rl, mixed) * col_bytes(np, mixed);
+}
 // Kernel instance for (NP, RL, mixed), with the shared-memory carveout at its
 // maximum so that several CTAs' slot stages fit on an SM.
 const void *solve_kernel(int np, int rl, bool mixed) {
     const void *fn = solve_kernel_raw(np, rl, mixed);
     OFEA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    (int)cudaSharedmemCarveoutMaxShared));
+    OFEA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageLimit));
     return fn;
 }
 template <int NP>
@@ -1044,14 +1260,16 @@ struct ofea_batch {
     std::vector<ofea_ctx *> ctx;
     std::vector<long> dof0, c0;
     long ndof = 0, ncoarse = 0;
-    int nslices = 0, naggs = 0, ncrows = 0;
+    int nslices = 0, naggs = 0, ncrows = 0, su_max = 0;
     bool mixed_ready = false, have_rhs = false;
     ofea::DevBuf<ofea::BVar> var;
+    ofea::DevBuf<ofea::BSlice> slice;
+    ofea::DevBuf<unsigned> vmask;
     ofea::DevBuf<int> slice_var, agg_var, crow_var;
     ofea::DevBuf<double> f, u, r, p0, p1, q, z64, pa, pb, ff, tol2, rz, alpha, beta, rel, stage;
     ofea::DevBuf<float> b32, x32, t32, zA, zB, cvec, evec;
     ofea::DevBuf<int> live, iters, status, live_cnt;
-    ofea::DevBuf<ofea::GridSync> gs;
+    ofea::DevBuf<ofea::GridBar> gs;
     ofea::DevBuf<unsigned long long> trace;  // per-phase timestamps when tracing (trace_cap > 0)
     ofea::HostBuf<double> bounce[2];          // page-locked blocks between the callers' arrays and the device
     int trace_cap = 0;
@@ -1094,7 +1312,12 @@ void build_desc(ofea_batch *b, bool mixed) {
         B.scols = c->scols.p;
         B.sv64 = c->sv64.p;
         B.Dinv = c->Dinv.p;
-        B.sv16 = c->sv16.p;
+        B.sl_g = c->sl_g.p;
+        B.su_runs = reinterpret_cast<const int2 *>(c->su_runs.p);
+        B.su_n = c->su_n.p;
+        B.su_idx = c->su_idx.p;
+        B.sv16g = c->sv16g.p;
+        b->su_max = std::max(b->su_max, c->su_max);
         B.Dinv32 = c->Dinv32.p;
         for (int s = 0; s < B.nslice; ++s) sv.push_back(v);
         slice0 += B.nslice;
@@ -1106,14 +1329,10 @@ void build_desc(ofea_batch *b, bool mixed) {
             B.crow0 = crow0;
             B.c0 = c0;
             b->c0[v] = c0;
-            B.agg_of = C.agg_of.p;
             B.agg_ptr = C.agg_ptr.p;
-            B.agg_nodes = C.agg_nodes.p;
-            B.node_of_free = c->node_of_free.p;
-            B.xyz = c->xyz.p;
-            B.centroid = C.centroid.p;
+            B.agg_off = reinterpret_cast<const float4 *>(C.agg_off.p);
+            B.row_off = reinterpret_cast<const float4 *>(C.row_off.p);
             B.Einv32 = C.Einv32.p;
-            B.inv_scale = C.inv_scale;
             B.wsm = smoother_weight(c, kBatchSmootherDamping);
             for (int a = 0; a < C.na; ++a) av.push_back(v);
             for (int i = 0; i < C.m; ++i) cv.push_back(v);
@@ -1129,6 +1348,11 @@ void build_desc(ofea_batch *b, bool mixed) {
     cudaStream_t s = b->stream;
     b->var.upload(d.data(), d.size(), s);
     b->slice_var.upload(sv.data(), sv.size(), s);
+    b->slice.ensure(std::max<size_t>(1, sv.size()));
+    b->vmask.ensure(b->V);
+    k_batch_slices<<<std::max(1, std::min(kMaxGrid, (slice0 + 255) / 256)), 256, 0, s>>>(slice0, b->var.p, b->slice_var.p,
+                                                                                       b->slice.p);
+    OFEA_CHECK_LAUNCH();
     if (mixed) {
         b->agg_var.upload(av.data(), av.size(), s);
         b->crow_var.upload(cv.data(), cv.size(), s);
@@ -1179,6 +1403,9 @@ BArgs make_args(ofea_batch *b, bool mixed, const TuneCfg &t, int max_iter, doubl
     a.limit_ns = 5000000000ull;  // 5 s: far above any phase
     a.rtol = rtol;
     a.var = b->var.p;
+    a.slice = b->slice.p;
+    a.vmask = b->vmask.p;
+    a.cap = stage_cap(b->su_max, b->NP, t.rl, mixed);
     a.slice_var = b->slice_var.p;
     a.agg_var = b->agg_var.p;
     a.crow_var = b->crow_var.p;
@@ -1213,9 +1440,9 @@ BArgs make_args(ofea_batch *b, bool mixed, const TuneCfg &t, int max_iter, doubl
     return a;
 }
 
-int grid_of(ofea_batch *b, const void *fn, const TuneCfg &t) {
+int grid_of(ofea_batch *b, const void *fn, const TuneCfg &t, int smem) {
     int occ = 0;
-    OFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads_for(b->NP, t.rl), 0));
+    OFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads_for(b->NP, t.rl), smem));
     if (occ < 1) fail(OFEA_ERR_CAPACITY, "batched solver kernel does not fit on an SM");
     return b->num_sms * std::min(occ, t.ctas_per_sm);
 }
@@ -1226,14 +1453,16 @@ void enqueue(ofea_batch *b, const BArgs &a, const TuneCfg &t, bool mixed) {
     const size_t n = (size_t)b->ndof * b->NP;
     OFEA_CUDA(cudaMemsetAsync(b->p0.p, 0, sizeof(double) * n, s));
     OFEA_CUDA(cudaMemsetAsync(b->p1.p, 0, sizeof(double) * n, s));
-    OFEA_CUDA(cudaMemsetAsync(b->gs.p, 0, sizeof(GridSync), s));
+    OFEA_CUDA(cudaMemsetAsync(b->gs.p, 0, sizeof(GridBar), s));
     OFEA_CUDA(cudaMemsetAsync(b->live_cnt.p, 0, sizeof(int) * 3, s));
+    OFEA_CUDA(cudaMemsetAsync(b->vmask.p, 0, sizeof(unsigned) * b->V, s));
     if (a.trace) OFEA_CUDA(cudaMemsetAsync(a.trace, 0, sizeof(unsigned long long) * a.trace_cap, s));
     const void *fn = solve_kernel(b->NP, t.rl, mixed);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid_of(b, fn, t));
+    const int smem = stage_bytes(b->su_max, b->NP, t.rl, mixed);
+    cfg.gridDim = dim3(grid_of(b, fn, t, smem));
     cfg.blockDim = dim3(threads_for(b->NP, t.rl));
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1251,7 +1480,8 @@ void residuals(ofea_batch *b, const TuneCfg &t) {
     const void *fn = residual_kernel(b->NP, t.rl);
     const int G = std::min(kMaxGrid, b->num_sms * 4);
     void *args[] = {(void *)&a};
-    OFEA_CUDA(cudaLaunchKernel(fn, dim3(G), dim3(threads_for(b->NP, t.rl)), args, 0, s));
+    OFEA_CUDA(cudaLaunchKernel(fn, dim3(G), dim3(threads_for(b->NP, t.rl)), args,
+                               (size_t)red_bytes(b->NP, t.rl), s));
     k_batch_rel<<<std::max(1, std::min(kMaxGrid, (b->V * b->NR + 7) / 8)), 256, 0, s>>>(a, b->rel.p);
     OFEA_CHECK_LAUNCH();
 }
@@ -1287,7 +1517,8 @@ TuneCfg autotune(ofea_batch *b, bool mixed, double rtol) {
     for (int rl : {1, 2, 4}) {
         int occ = 0;
         OFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve_kernel(b->NP, rl, mixed),
-                                                                threads_for(b->NP, rl), 0));
+                                                                threads_for(b->NP, rl),
+                                                                stage_bytes(b->su_max, b->NP, rl, mixed)));
         std::vector<int> cps{1, 2, 4, occ};
         std::sort(cps.begin(), cps.end());
         cps.erase(std::unique(cps.begin(), cps.end()), cps.end());
@@ -1314,7 +1545,7 @@ TuneCfg autotune(ofea_batch *b, bool mixed, double rtol) {
             OFEA_CUDA(cudaEventSynchronize(e1));
             float ms = 0;
             OFEA_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            GridSync g{};
+            GridBar g{};
             OFEA_CUDA(cudaMemcpy(&g, b->gs.p, sizeof(g), cudaMemcpyDeviceToHost));
             if (g.err) fail(OFEA_ERR_TIMEOUT, "batched solver: a grid-barrier wait ran out while tuning");
             ms_min = std::min(ms_min, (double)ms);
@@ -1353,7 +1584,7 @@ ofea_batch *batch_create(ofea_ctx *const *ctxs, int nv, int nrhs) {
         if (!c) fail(OFEA_ERR_INVALID_ARG, "batch: NULL context");
         if (!c->K_ok || !c->sell_ok) fail(OFEA_ERR_STATE, "batch: variant " + std::to_string(v) + " not assembled");
         OFEA_CUDA(cudaSetDevice(c->device));
-        ensure_sv16(c);  // BF16 planes of the V-cycle SpMMs (a fused assembly leaves them to be derived)
+        ensure_slice_columns(c);  // once per pattern
         OFEA_CUDA(cudaStreamSynchronize(c->stream));
         if (c->device != ctxs[0]->device) fail(OFEA_ERR_INVALID_ARG, "batch: variants on different GPUs");
         b->ctx.push_back(c);
@@ -1552,7 +1783,7 @@ void batch_solve(ofea_batch *b, const ofea_solve_opts &o, ofea_solve_stats *stat
         ++launches;
         residuals(b, t);
         launches += 2;
-        GridSync g{};
+        GridBar g{};
         OFEA_CUDA(cudaMemcpyAsync(&g, b->gs.p, sizeof(g), cudaMemcpyDeviceToHost, s));
         OFEA_CUDA(cudaMemcpyAsync(hit.data(), b->iters.p, sizeof(int) * VJ, cudaMemcpyDeviceToHost, s));
         OFEA_CUDA(cudaMemcpyAsync(hst.data(), b->status.p, sizeof(int) * VJ, cudaMemcpyDeviceToHost, s));
@@ -1646,12 +1877,12 @@ void batch_phase_times(ofea_batch *b, double *ms, int cap, int *count) {
 }
 
 void barrier_probe(ofea_ctx *c, int limit_ms, int *released) {
-    DevBuf<GridSync> gs;
+    DevBuf<GridBar> gs;
     DevBuf<int> out;
     gs.ensure(1);
     out.ensure(1);
     cudaStream_t s = c->stream;
-    OFEA_CUDA(cudaMemsetAsync(gs.p, 0, sizeof(GridSync), s));
+    OFEA_CUDA(cudaMemsetAsync(gs.p, 0, sizeof(GridBar), s));
     OFEA_CUDA(cudaMemsetAsync(out.p, 0xff, sizeof(int), s));
     unsigned extra = 1;
     unsigned long long lim = (unsigned long long)limit_ms * 1000000ull;

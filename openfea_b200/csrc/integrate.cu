@@ -820,7 +820,7 @@ constexpr int kIncBatch = 8;   // incidences whose loads are in flight together
 struct SellOut {
     const int *sl_ptr, *sl_g;
     double *sv64;
-    __nv_bfloat16 *sv16, *svg;
+    __nv_bfloat16 *svg;
 };
 
 // One warp per free node (block row).  Rows wider than kRowCap accumulate in
@@ -896,7 +896,6 @@ __global__ void __launch_bounds__(kBlock) k_gather_assemble(
                 const int k = v / 9, e = v - 9 * k;
                 const double x = k < deg ? acc[v] : 0.0;
                 so.sv64[((S + k) * 9 + e) * kSlice + t] = x;
-                so.sv16[((S + k) * 9 + e) * kSlice + t] = __double2bfloat16(x);
             }
             const long G = so.sl_g[sl];
             uint2 *svg2 = reinterpret_cast<uint2 *>(so.svg);
@@ -951,12 +950,6 @@ __global__ void k_sell_to_kb(int nfree, const int *__restrict__ rowptr, const in
     }
 }
 
-// BF16 plane copy from the FP64 planes (the batched engine's operand).
-__global__ void k_sv64_to_sv16(long len, const double *__restrict__ sv64, __nv_bfloat16 *__restrict__ sv16) {
-    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < len; v += (long)gridDim.x * blockDim.x)
-        sv16[v] = __double2bfloat16(sv64[v]);
-}
-
 static void integrate(ofea_ctx *c, bool nl, const double *d_u) {
     upload_hex_table();
     cudaStream_t s = c->stream;
@@ -994,7 +987,7 @@ static void integrate(ofea_ctx *c, bool nl, const double *d_u) {
 static void gather(ofea_ctx *c, bool with_f, double *d_fint) {
     c->Kb.ensure((size_t)std::max<long long>(9 * c->nnzb, 1));
     if (!c->sell_layout_ok) build_sell_layout(c);
-    const SellOut so{c->sl_ptr.p, c->sl_g.p, c->sv64.p, c->sv16.p, c->sv16g.p};
+    const SellOut so{c->sl_ptr.p, c->sl_g.p, c->sv64.p, c->sv16g.p};
     int gw = grid_for(c, c->nfree, kWarpsPerBlock);
     if (with_f)
         k_gather_assemble<true><<<gw, kBlock, 0, c->stream>>>(
@@ -1008,8 +1001,7 @@ static void gather(ofea_ctx *c, bool with_f, double *d_fint) {
     c->K_ok = true;
     c->kb_ok = true;
     c->asm_path = 1;
-    c->sell_ok = true;  // written by the gather, BF16 planes included
-    c->sv16_ok = true;
+    c->sell_ok = true;  // written by the gather
     c->jacobi_fresh = false;
     c->coarse.K_ok = false;
     c->coarse2.K_ok = false;
@@ -1067,7 +1059,6 @@ static bool assemble_linear_fused(ofea_ctx *c) {
     c->asm_path = 0;
     c->sell_ok = true;
     c->kb_ok = false;        // block CSR on demand (ensure_kb)
-    c->sv16_ok = false;      // BF16 planes on demand (ensure_sv16)
     c->ke_ok = false;        // element matrices on demand (ensure_element_matrices)
     c->jacobi_fresh = true;  // Dinv written by the kernel
     c->coarse.K_ok = false;
@@ -1102,14 +1093,6 @@ void ensure_kb(ofea_ctx *c) {
                                                                               c->sv64.p, c->Kb.p);
     OFEA_CHECK_LAUNCH();
     c->kb_ok = true;
-}
-
-void ensure_sv16(ofea_ctx *c) {
-    if (c->sv16_ok) return;
-    const long len = 9L * std::max<long long>(c->sell_len, 1) * kSlice;
-    k_sv64_to_sv16<<<grid_for(c, len, kBlock), kBlock, 0, c->stream>>>(len, c->sv64.p, c->sv16.p);
-    OFEA_CHECK_LAUNCH();
-    c->sv16_ok = true;
 }
 
 void ensure_element_matrices(ofea_ctx *c) {

@@ -14,7 +14,7 @@
 //                                      position within the row, 0xFFFF if b is fixed
 //   Kb         double[9*nnzb]          K values, block-row-major, 3x3 blocks row-major
 //                                      (derived from sv64 on demand after a fused assembly)
-//   sl_ptr, scols, sv64, sv16          the solver's copy of K in BSELL-32 (sell.cuh),
+//   sl_ptr, scols, sv64, sv16g         the solver's copy of K in BSELL-32 (sell.cuh),
 //                                      FP64 values and a BF16 rounding
 //   se_ptr, se_list, inc_loc           per BSELL slice the sorted elements of its rows, and
 //                                      each incidence's position in them (fused assembly)
@@ -228,9 +228,9 @@ struct ofea_ctx {
     ofea::DevBuf<float> Dinv32;
     bool K_ok = false, jacobi_ok = false;
     // what the last assembly left current besides the solver copy: the fused
-    // linear assembly writes only sv64, sv16g and Dinv; Kb, sv16 and Ke are
-    // derived on demand (ensure_kb, ensure_sv16, ensure_element_matrices)
-    bool kb_ok = false, sv16_ok = false, ke_ok = false, jacobi_fresh = false;
+    // linear assembly writes only sv64, sv16g and Dinv; Kb and Ke are derived
+    // on demand (ensure_kb, ensure_element_matrices)
+    bool kb_ok = false, ke_ok = false, jacobi_fresh = false;
     int asm_path = 1;  // 0: the fused assembly made K, 1: the two-pass assembly or a CSC upload
     // per-slice element lists of the fused assembly (integrate.cu), per pattern:
     // se_state 0 not built, 1 built, -1 the mesh takes the two-pass assembly
@@ -241,9 +241,16 @@ struct ofea_ctx {
     // solver layout of K (sell.cuh): BSELL-32, FP64 and BF16 values
     ofea::DevBuf<int> sl_ptr, scols;
     ofea::DevBuf<double> sv64;
-    ofea::DevBuf<__nv_bfloat16> sv16;  // BF16 copy (plane layout) for the batched solver's V-cycle
     ofea::DevBuf<int> sl_g;            // slot-group offsets of the grouped BF16 copy (sell.cuh)
-    ofea::DevBuf<__nv_bfloat16> sv16g; // grouped BF16 copy for the single-matrix V-cycle SpMVs
+    ofea::DevBuf<__nv_bfloat16> sv16g; // grouped BF16 copy for the V-cycle's products
+    // the slices' distinct columns for the batched solver's staged products
+    // (sell.cu), in runs of consecutive ones: slice s at su_runs[32 sl_ptr[s]]
+    // (first column; position << 16 | length), su_n[2 s] columns (0: not
+    // listed) in su_n[2 s + 1] runs, and every slot's position among them
+    ofea::DevBuf<int> su_runs, su_n;
+    ofea::DevBuf<uint16_t> su_idx;
+    int su_max = 0;
+    bool su_ok = false;
     long long sell_len = 0;
     bool sell_ok = false;         // values of the solver copy current
     bool sell_layout_ok = false;  // slice pointers, columns and buffers for the current pattern
@@ -272,12 +279,12 @@ void assemble_linear(ofea_ctx *c);
 void assemble_nl(ofea_ctx *c, const double *d_u, double *d_fint);
 void build_block_jacobi(ofea_ctx *c);
 void ensure_kb(ofea_ctx *c);
-void ensure_sv16(ofea_ctx *c);
 void ensure_element_matrices(ofea_ctx *c);
 void stress_recovery(ofea_ctx *c, const double *d_u, int mode, double *d_elem, double *d_node);
 // sell.cu
 void build_sell_layout(ofea_ctx *c);
 void build_sell(ofea_ctx *c);
+void ensure_slice_columns(ofea_ctx *c);
 // solve.cu
 void spmv64(ofea_ctx *c, const double *d_x, double *d_y);
 void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_opts &o,

@@ -55,42 +55,9 @@ struct RArgs {
     double tol2;
     Parts P;
     Flags *fl;
-    unsigned *bar;  // [0] arrivals, [1] error
+    GridBar *bar;
     unsigned long long limit_ns;
 };
-
-__device__ __forceinline__ unsigned long long res_global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Grid barrier of a cooperative launch; arrivals count up over the launch
-// (target = barriers so far x CTAs).  False: the wait ran out, here or
-// elsewhere, and the caller returns.
-__device__ __forceinline__ bool res_barrier(unsigned *bar, unsigned target, unsigned long long limit_ns, int *s_fail) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-        unsigned long long t0 = 0;
-        for (unsigned spin = 1;; ++spin) {
-            unsigned c;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
-            if (c >= target) break;
-            if ((spin & 255u) == 0) {
-                const unsigned long long t = res_global_ns();
-                if (t0 == 0) t0 = t;
-                if (*(volatile unsigned *)(bar + 1) != 0 || t - t0 > limit_ns) {
-                    *(volatile unsigned *)(bar + 1) = 1;
-                    *s_fail = 1;
-                    break;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    return *s_fail == 0;
-}
 
 // Part `part` of S of a row's product: FP64 slots part, part + S, ..., two in
 // flight.
@@ -195,7 +162,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     }
     auto sync = [&]() {
         target += G;
-        return res_barrier(a.bar, target, a.limit_ns, &s_fail);
+        return grid_barrier(a.bar, target, a.limit_ns, &s_fail);
     };
     // this CTA's partial of one or two sums (threads' values x, y)
     auto put = [&](double x, double *Px, double y, double *Py) {
@@ -568,9 +535,9 @@ void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, const P
     a.P = P;
     a.fl = fl;
     w.bar.ensure(2);
-    a.bar = w.bar.p;
+    a.bar = reinterpret_cast<GridBar *>(w.bar.p);
     a.limit_ns = 5000000000ull;  // 5 s: far above any phase
-    OFEA_CUDA(cudaMemsetAsync(w.bar.p, 0, 2 * sizeof(unsigned), c->stream));
+    OFEA_CUDA(cudaMemsetAsync(w.bar.p, 0, sizeof(GridBar), c->stream));
     void *args[] = {(void *)&a};
     const void *fn = mixed ? (const void *)k_resident<true> : (const void *)k_resident<false>;
     OFEA_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.G), dim3(kResThreads), args, 0, c->stream));

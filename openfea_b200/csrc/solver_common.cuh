@@ -53,6 +53,45 @@ __device__ __forceinline__ bool cta_done(const Flags *fl) {
     return s_done != 0;
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Grid barrier of a cooperative launch (zeroed before it): arrivals count up
+// over the launch, target = arrivals expected so far.  One release-add and an
+// acquire spin per CTA; what the CTAs wrote before is visible after.  Returns
+// false (in every thread of the CTA) when the wait ran out here or elsewhere:
+// the caller returns.  s_fail: shared, zero before the first barrier.
+struct GridBar {
+    unsigned count;
+    int err;
+};
+__device__ __forceinline__ bool grid_barrier(GridBar *bar, unsigned target, unsigned long long limit_ns, int *s_fail) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->count) : "memory");
+        unsigned long long t0 = 0;
+        for (unsigned spin = 1;; ++spin) {
+            unsigned c;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&bar->count) : "memory");
+            if ((int)(c - target) >= 0) break;
+            if ((spin & 255u) == 0) {
+                const unsigned long long t = global_ns();
+                if (t0 == 0) t0 = t;
+                if (*(volatile int *)&bar->err != 0 || t - t0 > limit_ns) {
+                    *(volatile int *)&bar->err = 1;
+                    *s_fail = 1;
+                    break;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    return *s_fail == 0;
+}
+
 // Per-CTA partial sums, all arrays of kMaxGrid doubles.
 struct Parts {
     double *pq, *rz0, *rz1, *rzo, *rr, *ff;

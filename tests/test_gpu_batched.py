@@ -174,3 +174,29 @@ def test_batched_phase_trace(gpu_ctx_factory, tmp_path, monkeypatch, method, ini
     with pytest.raises(ob.OfeaError):
         b.phase_times()
     b.close()
+
+
+@pytest.mark.parametrize("method", ["GPU_MIXED", "GPU_PCG"])
+@pytest.mark.parametrize("nrhs", [2, 5, 9, 17, 32])
+def test_staged_and_direct_columns(gpu_ctx_factory, method, nrhs):
+    # slices whose distinct columns fit the products' buffer and slices (many
+    # load cases in FP64; a cross-section of 30 x 30 nodes) beyond it, every
+    # load-case stride, C3D4 columns that are not in runs: the residual of
+    # each load case on the host
+    meshes = [mg.structured_hex(5, 2, 3, 0.025, 0.01, 0.015, 210e9, 0.3),
+              mg.structured_hex(4, 29, 29, 0.02, 0.145, 0.145, 210e9, 0.3), mg.tet_block(5, 4, 3)[0]]
+    ctxs, loads = [], []
+    for i, m in enumerate(meshes):
+        c = gpu_ctx_factory()
+        c.upload_mesh(m)
+        c.assemble_pattern()
+        c.assemble_linear()
+        ctxs.append(c)
+        loads.append(np.random.default_rng(i).normal(size=(nrhs, c.n)))
+    U, _ = ob.Batch(ctxs, nrhs).solve(loads, method=method, rtol=1e-9)
+    for c, F, u in zip(ctxs, loads, U):
+        rp, col, val = c.get_csr()
+        K = sp.csr_matrix((val, col, rp), shape=(c.n, c.n))
+        floor = np.diff(rp).max() * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u.T), axis=0)
+        norms = np.linalg.norm(F, axis=1)
+        assert np.all(np.linalg.norm(F.T - K @ u.T, axis=0) <= 1e-9 * norms + floor)

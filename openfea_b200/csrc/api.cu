@@ -327,6 +327,7 @@ int ofea_mesh_set_modulus(ofea_ctx *c, const double *E_elem, double E0) {
         need(c->mesh_ok, OFEA_ERR_STATE, "no mesh uploaded");
         use_device(c);
         HVec<double> E8, E4;
+        c->K_linear = false;  // the moduli on the device leave K behind until the next assembly
         split_modulus(c, E_elem, E0, E8, E4);
         c->E0 = E0;
         c->E8.upload(E8.data(), E8.size(), c->stream);
@@ -436,6 +437,7 @@ int ofea_matrix_upload_csc(ofea_ctx *c, int nd, const double *xyz, const int *fr
         c->mesh_ok = true;
         c->pattern_ok = true;
         c->K_ok = true;
+        c->K_linear = false;
         c->kb_ok = true;
         c->asm_path = 1;
         c->jacobi_fresh = false;

@@ -1067,12 +1067,16 @@ static bool assemble_linear_fused(ofea_ctx *c) {
 }
 
 void assemble_linear(ofea_ctx *c) {
-    if (assemble_linear_fused(c)) return;
-    integrate(c, false, nullptr);
-    gather(c, false, nullptr);
+    c->K_linear = false;
+    if (!assemble_linear_fused(c)) {
+        integrate(c, false, nullptr);
+        gather(c, false, nullptr);
+    }
+    c->K_linear = true;
 }
 
 void assemble_nl(ofea_ctx *c, const double *d_u, double *d_fint) {
+    c->K_linear = false;
     integrate(c, true, d_u);
     gather(c, true, d_fint);
 }

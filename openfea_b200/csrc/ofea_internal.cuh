@@ -237,6 +237,14 @@ struct ofea_ctx {
     ofea::DevBuf<int> se_ptr, se_list;
     ofea::DevBuf<uint16_t> inc_loc;
     int se_state = 0;
+    // products with K from the elements (matfree.cu): K_linear: K is the linear
+    // stiffness of the mesh as it is on the device; the tables are per
+    // pattern; mf_fe: the element forces
+    bool K_linear = false;
+    ofea::DevBuf<int> mf_list, mf_rows;
+    ofea::DevBuf<unsigned char> mf_link;
+    ofea::DevBuf<double> mf_fe;
+    int mf_state = 0, mf_width = 0;
     bool fused_off = false;  // ofea_set_assembly_path(ctx, 1): always the two-pass assembly
     // solver layout of K (sell.cuh): BSELL-32, FP64 and BF16 values
     ofea::DevBuf<int> sl_ptr, scols;

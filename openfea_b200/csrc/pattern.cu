@@ -334,6 +334,8 @@ void build_pattern(ofea_ctx *c) {
     c->sell_ok = false;
     c->sell_layout_ok = false;
     c->se_state = 0;
+    c->mf_state = 0;
+    c->K_linear = false;
     c->coarse.K_ok = false;  // the coarse geometry depends on the mesh alone: it stays
     c->coarse2.K_ok = false;
     c->learned.links_ok = false;

@@ -119,6 +119,23 @@ __device__ __forceinline__ void for_each_sell_row(int nfree, const int *__restri
     }
 }
 
+// The product's rows for the solvers' row kernels: f(r, y, pre(r)) for each of
+// this thread's block rows r, y = (K x)_r from the stored K (x(k): entry k of
+// x).
+struct SellRows {
+    static constexpr int kCtas = 8;  // 256-thread CTAs per SM the row kernels are compiled for (32 registers)
+    const int *sl_ptr, *scols;
+    const double *sv64;
+    template <class XF, class Pre, class F>
+    __device__ __forceinline__ void rows(int nfree, XF x, Pre pre, F f) const {
+        for_each_sell_row(nfree, sl_ptr, [&](int r, long S, int t, int W) {
+            double y[3];
+            sell_row<double, 2>(S, t, W, scols, sv64, x, y[0], y[1], y[2]);
+            f(r, y, pre(r));
+        });
+    }
+};
+
 // Read access to block (r, k) of K: block CSR when it is current, else the
 // FP64 BSELL copy (all a fused assembly writes).
 struct KBlocks {
@@ -130,6 +147,8 @@ struct KBlocks {
         return sv64[((long)(sl_ptr[r / kSlice] + k) * 9 + e) * kSlice + (r % kSlice)];
     }
 };
+
+inline SellRows sell_rows(const ofea_ctx *c) { return SellRows{c->sl_ptr.p, c->scols.p, c->sv64.p}; }
 
 inline KBlocks kblocks(const ofea_ctx *c) {
     return KBlocks{c->kb_ok ? c->Kb.p : nullptr, c->rowptr.p, c->sl_ptr.p, c->sv64.p};

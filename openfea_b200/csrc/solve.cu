@@ -16,6 +16,11 @@
 // Kernels per iteration: A, B (+ pre-smoothing), residual, restriction, GEMV,
 // prolongation, post-smoothing (+ the r.z dots).
 //
+// Three ways to run the iterations: in one resident kernel (resident.cu; PCG64
+// and MIXED up to some 10^5 rows), launch per phase with the stored K, and
+// launch per phase with the outer products formed from the elements
+// (matfree.cu; large models of C3D8 elements).
+//
 // Scalars (alpha, beta, convergence) are formed redundantly and identically
 // by every CTA from the previous kernel's partials, in a fixed order: results
 // are bitwise reproducible and no host round trip is needed per iteration.
@@ -28,6 +33,7 @@
 #include <cmath>
 #include <functional>
 
+#include "matfree.cuh"
 #include "precond.cuh"
 #include "resident.cuh"
 #include "sell.cuh"
@@ -99,11 +105,16 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_residual64(
     }
 }
 
+// A row's own entries of p_old, z and q.
+struct OwnRow {
+    double p[3], z[3], q[3];
+};
+
 // Iteration kernel A: p = z + beta p_old, q = K p as K z + beta q_old, partial
 // p.q.  tol2 = (target ||r||)^2.
-__global__ void __launch_bounds__(kBlock, kSpmvCtas) k_pcg64_A(
-    int nfree, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
-    const double *__restrict__ sv64, const double *__restrict__ z, double *__restrict__ pA,
+template <class Rows>
+__global__ void __launch_bounds__(kBlock, Rows::kCtas) k_pcg64_A(
+    int nfree, const Rows K, const double *__restrict__ z, double *__restrict__ pA,
     double *__restrict__ pB, double *__restrict__ q, Parts P, Flags *fl, double tol2) {
     __shared__ double sh[kWarpsPerBlock];
     if (cta_done(fl)) return;
@@ -124,13 +135,14 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_pcg64_A(
     const double *pold = (k & 1) ? pB : pA;
     double *pnew = (k & 1) ? pA : pB;
     double ppq = 0;
-    for_each_sell_row(nfree, sl_ptr, [&](int rw, long S, int t, int W) {
-        double y[3];
-        sell_row<double, 2>(S, t, W, scols, sv64, [&](int kk) { return z[kk]; }, y[0], y[1], y[2]);
+    auto own = [&](int rw) { return OwnRow{{pold[3L * rw], pold[3L * rw + 1], pold[3L * rw + 2]},
+                                          {z[3L * rw], z[3L * rw + 1], z[3L * rw + 2]},
+                                          {q[3L * rw], q[3L * rw + 1], q[3L * rw + 2]}}; };
+    K.rows(nfree, [&](int kk) { return z[kk]; }, own, [&](int rw, const double (&y)[3], const OwnRow &o) {
         for (int i = 0; i < 3; ++i) {
             const long d = 3L * rw + i;
-            const double pn = fma(beta, pold[d], z[d]);
-            const double qn = fma(beta, q[d], y[i]);  // K p = K z + beta K p_old
+            const double pn = fma(beta, o.p[i], o.z[i]);
+            const double qn = fma(beta, o.q[i], y[i]);  // K p = K z + beta K p_old
             pnew[d] = pn;
             q[d] = qn;
             ppq += pn * qn;
@@ -198,9 +210,9 @@ __global__ void __launch_bounds__(kBlock) k_pcg64_B(
 // p <- double(z_k) + beta p, q = K64 p as K64 z + beta q (the SpMV gathers z
 // alone; drift of q from K p is caught by the FP64 true-residual check),
 // partial p.q.
-__global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_A(
-    int nfree, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
-    const double *__restrict__ sv64, const float *__restrict__ zA, const float *__restrict__ zB,
+template <class Rows>
+__global__ void __launch_bounds__(kBlock, Rows::kCtas) k_fcg_A(
+    int nfree, const Rows K, const float *__restrict__ zA, const float *__restrict__ zB,
     double *__restrict__ pA, double *__restrict__ pB, double *__restrict__ q, Parts P, Flags *fl,
     double tol2) {
     __shared__ double sh[kWarpsPerBlock];
@@ -225,13 +237,14 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_A(
     const double *pold = (k & 1) ? pB : pA;
     double *pnew = (k & 1) ? pA : pB;
     double ppq = 0;
-    for_each_sell_row(nfree, sl_ptr, [&](int rw, long S, int t, int W) {
-        double y[3];
-        sell_row<double, 2>(S, t, W, scols, sv64, [&](int kk) { return (double)z[kk]; }, y[0], y[1], y[2]);
+    auto own = [&](int rw) { return OwnRow{{pold[3L * rw], pold[3L * rw + 1], pold[3L * rw + 2]},
+                                          {(double)z[3L * rw], (double)z[3L * rw + 1], (double)z[3L * rw + 2]},
+                                          {q[3L * rw], q[3L * rw + 1], q[3L * rw + 2]}}; };
+    K.rows(nfree, [&](int kk) { return (double)z[kk]; }, own, [&](int rw, const double (&y)[3], const OwnRow &o) {
         for (int i = 0; i < 3; ++i) {
             const long d = 3L * rw + i;
-            const double pn = fma(beta, pold[d], (double)z[d]);
-            const double qn = fma(beta, q[d], y[i]);  // K p = K z + beta K p_old
+            const double pn = fma(beta, o.p[i], o.z[i]);
+            const double qn = fma(beta, o.q[i], y[i]);  // K p = K z + beta K p_old
             pnew[d] = pn;
             q[d] = qn;
             ppq += pn * qn;
@@ -560,6 +573,15 @@ struct StopFlagScope {
 
 }  // namespace
 
+// Block rows from which the outer products of a linear C3D8 model are formed
+// from its elements (matfree.cu).  Below, K stays in L2 and the resident
+// solver's PCG64 iteration is the faster one (139k DOF: 20.7 us there, 27.9
+// from the elements; 288k: 48 and 37; 706k: 105 and 68; 1.56M: 221 and 130;
+// MIXED, launch per phase, stored K and elements: 706k 215 and 170, 1.56M 398
+// and 311).  The smoother's products keep the stored BF16 K: formed from the
+// elements in FP32 they took as long (44 + 14 us against 61 at 1.56M DOF).
+constexpr int kMatfreeRows = 70000;
+
 // Damping of the block-Jacobi smoother: omega = damping / lmax, lmax the power
 // iteration's estimate of lambda_max(D^-1 K).  The V(1,1) cycle stays
 // positive definite while omega lmax < 2 (with margin for the estimate,
@@ -624,7 +646,8 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         w.z.ensure(n);
     }
     ResidentPlan plan;
-    const bool resident = !learned && resident_plan(c, mixed, plan);
+    const bool matfree = nf >= kMatfreeRows && matfree_ready(c);
+    const bool resident = !learned && !(matfree && !mixed) && resident_plan(c, mixed, plan);
     if (resident && mixed) coarse_dense_inverse(c);
     const int G = resident ? plan.G : solver_grid(c);
     Workspace ws = setup(c, G);
@@ -674,33 +697,39 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
             const StopFlagScope stop_scope{c};
             // initial preconditioner application z_0 = M(r_0)
             k_set_itB<<<1, 1, 0, s>>>(ws.fl, -1);
-            vc_resid(c, w.b32.p, w.x32.p, w.t32.p);
-            if (learned) learned_coarse_correct(c, w.t32.p, w.x32.p);
-            else coarse_correct(c, w.t32.p, w.x32.p);
-            k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm, w.b32.p,
-                                            w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl);
-            OFEA_CHECK_LAUNCH();
+            auto precondition = [&] {
+                vc_resid(c, w.b32.p, w.x32.p, w.t32.p);
+                if (learned) learned_coarse_correct(c, w.t32.p, w.x32.p);
+                else coarse_correct(c, w.t32.p, w.x32.p);
+                k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm, w.b32.p,
+                                                w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl);
+                OFEA_CHECK_LAUNCH();
+            };
+            precondition();
             launches += learned ? 12 : 6;
             auto chunk = [&](int iters) {
                 for (int it = 0; it < iters; ++it) {
-                    k_fcg_A<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, w.z32a.p, w.z32b.p,
-                                                 w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+                    auto A = [&](auto K) {
+                        k_fcg_A<<<G, kBlock, 0, s>>>(nf, K, w.z32a.p, w.z32b.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+                    };
+                    if (matfree) {
+                        matfree_forces(c, w.z32a.p, w.z32b.p, ws.fl);
+                        A(matfree_rows(c));
+                    } else {
+                        A(sell_rows(c));
+                    }
                     k_fcg_B<<<G, kBlock, 0, s>>>(nf, c->Dinv32.p, wsm, w.p0.p, w.p1.p, w.q.p, d_u, w.r.p,
                                                  w.b32.p, w.x32.p, ws.P, ws.fl);
-                    vc_resid(c, w.b32.p, w.x32.p, w.t32.p);
-                    if (learned) learned_coarse_correct(c, w.t32.p, w.x32.p);
-                    else coarse_correct(c, w.t32.p, w.x32.p);
-                    k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm,
-                                                    w.b32.p, w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl);
+                    precondition();
                 }
                 OFEA_CHECK_LAUNCH();
             };
-            drive(c, oo, ws, per_chunk, chunk, hf, launches, learned ? 13 : 7, timed_out, t_start, {});
+            drive(c, oo, ws, per_chunk, chunk, hf, launches, (learned ? 13 : 7) + (matfree ? 1 : 0), timed_out, t_start, {});
         } else {
             auto chunk = [&](int iters) {
                 for (int it = 0; it < iters; ++it) {
-                    k_pcg64_A<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, w.z.p, w.p0.p,
-                                                   w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+                    matfree_forces(c, w.z.p, ws.fl);
+                    k_pcg64_A<<<G, kBlock, 0, s>>>(nf, matfree_rows(c), w.z.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
                     k_pcg64_B<<<G, kBlock, 0, s>>>(nf, c->Dinv.p, w.p0.p, w.p1.p, w.q.p, d_u, w.r.p, w.z.p,
                                                    ws.P, ws.fl);
                 }
@@ -708,7 +737,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
             };
             std::function<void()> after;
             if (on_chunk) after = [&] { on_chunk(w.r.p); };
-            drive(c, oo, ws, per_chunk, chunk, hf, launches, 2, timed_out, t_start, after);
+            drive(c, oo, ws, per_chunk, chunk, hf, launches, 3, timed_out, t_start, after);
         }
         total_iters += hf.iters;
         if (hf.status == OFEA_ERR_BREAKDOWN) break;
@@ -776,8 +805,7 @@ void profile_kernels(ofea_ctx *c, int method, int reps, double *ms, double *byte
         double *u = w.t.p;
         OFEA_CUDA(cudaEventRecord(e0, s));
         for (int i = 0; i < reps; ++i)
-            k_pcg64_A<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, w.z.p, w.p0.p, w.p1.p,
-                                           w.q.p, ws.P, ws.fl, tol2);
+            k_pcg64_A<<<G, kBlock, 0, s>>>(nf, sell_rows(c), w.z.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
         OFEA_CUDA(cudaEventRecord(e1, s));
         for (int i = 0; i < reps; ++i)
             k_pcg64_B<<<G, kBlock, 0, s>>>(nf, c->Dinv.p, w.p0.p, w.p1.p, w.q.p, u, w.r.p, w.z.p, ws.P, ws.fl);
@@ -790,8 +818,7 @@ void profile_kernels(ofea_ctx *c, int method, int reps, double *ms, double *byte
         const float wsm = smoother_weight(c, kSmootherDamping);
         OFEA_CUDA(cudaEventRecord(e0, s));
         for (int i = 0; i < reps; ++i)
-            k_fcg_A<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, w.z32a.p, w.z32b.p, w.p0.p,
-                                         w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+            k_fcg_A<<<G, kBlock, 0, s>>>(nf, sell_rows(c), w.z32a.p, w.z32b.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
         OFEA_CUDA(cudaEventRecord(e1, s));
         for (int i = 0; i < reps; ++i)
             k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm, w.b32.p,

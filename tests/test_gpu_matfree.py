@@ -1,0 +1,78 @@
+"""Solves of large linear C3D8 models, whose outer products are formed from the
+elements (matfree.cu) and not from the stored K.
+
+The checks are on the assembled K (the arrays the oracle tests pin to the
+reference): the residual of the returned u in FP64 on the host, for elements
+in the usual order (each standing on the one before), in a random order (no
+two of them linked), with numbered-about nodes and distorted elements.
+"""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from openfea_b200 import meshgen as mg
+
+pytestmark = pytest.mark.gpu
+
+
+def model(shape, order, seed=5):
+    m = mg.structured_hex(*shape, *(0.005 * s for s in shape), 210e9, 0.3)
+    rng = np.random.default_rng(seed)
+    ext = 0.005 * np.array(shape)
+    inside = np.all((m.xyz > 1e-9) & (m.xyz < ext - 1e-9), axis=1)
+    m.xyz[inside] += rng.uniform(-0.0005, 0.0005, (int(inside.sum()), 3))
+    m.E = 210e9 * mg.simp_density(shape, 3) ** 3
+    if order != "lines":
+        p = rng.permutation(m.ne)
+        m.topo, m.E = m.topo[p], m.E[p]
+    if order == "nodes":
+        new = rng.permutation(m.nd)  # node i becomes new[i]
+        xyz = np.empty_like(m.xyz)
+        xyz[new] = m.xyz
+        m.xyz, m.topo, m.fix = xyz, (new[m.topo - 1] + 1).astype(np.int32), np.sort(new[m.fix - 1] + 1).astype(np.int32)
+    return m
+
+
+def residual(ctx, f, u):
+    rp, col, val = ctx.get_csr()
+    K = sp.csr_matrix((val, col, rp), shape=(f.size, f.size))
+    floor = int(np.diff(rp).max()) * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u))
+    return np.linalg.norm(f - K @ u) / np.linalg.norm(f), floor / np.linalg.norm(f)
+
+
+# 70,000 block rows and more take the elements; MIXED beyond the resident solver
+@pytest.mark.parametrize("method,shape,order", [
+    ("GPU_PCG", (62, 35, 32), "lines"), ("GPU_PCG", (62, 35, 32), "elements"), ("GPU_PCG", (61, 34, 33), "nodes"),
+    ("GPU_MIXED", (95, 36, 33), "lines"), ("GPU_MIXED", (95, 36, 33), "elements")])
+def test_solves_from_the_elements(gpu_ctx_factory, method, shape, order):
+    m = model(shape, order)
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    assert ctx.n >= 3 * 70000
+    f = np.random.default_rng(7).normal(size=ctx.n)
+    u, st = ctx.solve(f, method=method, rtol=1e-9)
+    rel, floor = residual(ctx, f, u)
+    assert rel <= 1e-9 + floor
+    u2, _ = ctx.solve(f, method=method, rtol=1e-9)
+    assert np.array_equal(u, u2)
+
+
+def test_the_current_k_is_solved(gpu_ctx_factory):
+    # new moduli, and a tangent that the linear elements do not give
+    m = model((62, 35, 32), "lines")
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    f = np.random.default_rng(8).normal(size=ctx.n)
+    for step in ("linear", "moduli", "tangent"):
+        if step == "moduli":
+            ctx.set_modulus(np.linspace(50e9, 90e9, m.ne), 70e9)
+        if step == "tangent":
+            ctx.assemble_nl(np.random.default_rng(9).uniform(-5e-5, 5e-5, ctx.n))
+        else:
+            ctx.assemble_linear()
+        u, _ = ctx.solve(f, method="GPU_PCG", rtol=1e-9)
+        rel, floor = residual(ctx, f, u)
+        assert rel <= 1e-9 + floor, step

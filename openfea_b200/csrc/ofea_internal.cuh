@@ -133,7 +133,7 @@ struct SolverWork {
     DevBuf<float> b32, x32, t32, z32a, z32b;    // FP32 preconditioner vectors
     DevBuf<double> partials;   // reduction partials (several arrays of kMaxGrid)
     DevBuf<int> flags;         // [0]=done [1]=iters [2]=status
-    DevBuf<unsigned> bar;      // the resident solver's grid barrier: arrivals, error
+    DevBuf<unsigned> bar;      // the resident solver's barrier slots and error flag
     HostBuf<int> hflags;
     HostBuf<double> hscal;
 };

@@ -25,9 +25,15 @@
 // visible, so no mutable vector may be read through the non-coherent path.
 //
 // Per iteration, launch-per-phase kernels before, this after (B200): PCG64
-// 27.9 -> 9.0 us at 1.5k DOF, 28.7 -> 11.2 at 46k, 58.0 -> 20.7 at 139k;
-// MIXED 62 -> 22.7, 66 -> 28.4 and 111 -> 56 us.  What is left at the small
-// end is the barriers and the reductions beside them (about 4 us a phase).
+// 27.9 -> 7.6 us at 1.5k DOF, 28.7 -> 9.3 at 46k, 58.0 -> 18.4 at 139k; MIXED
+// 62 -> 19.5, 66 -> 24.9, 111 -> 54 and 132 -> 98 us (288k).  What is left at
+// the small end is the barriers: 2,600 to 2,900 cycles each, 2,000 more to
+// drain a phase's stores, and 800 for the first load after.  Sums of a phase are
+// taken under the next product where nothing needs them earlier, a CTA's own
+// rows are loaded under the wait.  Measured and not used: every CTA reading
+// every other's tagged partial instead of a counter (30 us against 21 at 139k
+// DOF), the next step's columns or the own rows in registers across the
+// product (spills: 25 against 18).
 //
 // Every wait is bounded (%globaltimer): on expiry the kernel sets the error
 // status and every CTA returns.
@@ -59,18 +65,36 @@ struct RArgs {
     unsigned long long limit_ns;
 };
 
+// A warp's slice of the first round, kept in registers for the launch: where
+// it starts, and the columns of its part's first step.
+struct Home {
+    int S, W, c0, c1;
+};
+__device__ __forceinline__ Home home(const int *__restrict__ sl_ptr, const int *__restrict__ scols, int slice, int lane, int k0, int k1) {
+    Home h;
+    h.S = __ldg(sl_ptr + slice);
+    h.W = __ldg(sl_ptr + slice + 1) - h.S;
+    h.c0 = k0 < h.W ? __ldg(scols + ((long)h.S + k0) * kSlice + lane) : 0;
+    h.c1 = k1 < h.W ? __ldg(scols + ((long)h.S + k1) * kSlice + lane) : h.c0;
+    return h;
+}
+
 // Part `part` of S of a row's product: FP64 slots part, part + S, ..., two in
 // flight.
 template <class XF>
-__device__ __forceinline__ void part64(long Sb, int t, int W, int part, int S, const int *__restrict__ scols,
+__device__ __forceinline__ void part64(const Home &h, int t, int part, int S, const int *__restrict__ scols,
                                        const double *__restrict__ sv, XF x, double (&y)[3]) {
-    const int *cp = scols + Sb * kSlice + t;
-    const double *vp = sv + Sb * 9 * kSlice + t;
+    const int *cp = scols + (long)h.S * kSlice + t;
+    const double *vp = sv + (long)h.S * 9 * kSlice + t;
     y[0] = y[1] = y[2] = 0.0;
-    for (int k = part; k < W; k += 2 * S) {
-        const bool two = k + S < W;
+    int c0 = h.c0, c1 = h.c1;
+    for (int k = part; k < h.W; k += 2 * S) {
+        const bool two = k + S < h.W;
         const int k1 = two ? k + S : k;
-        const int c0 = __ldg(cp + (long)k * kSlice), c1 = __ldg(cp + (long)k1 * kSlice);
+        if (k != part) {
+            c0 = __ldg(cp + (long)k * kSlice);
+            c1 = __ldg(cp + (long)k1 * kSlice);
+        }
         double v[2][9];
 #pragma unroll
         for (int e = 0; e < 9; ++e) {
@@ -92,15 +116,19 @@ __device__ __forceinline__ void part64(long Sb, int t, int W, int part, int S, c
 }
 
 // The same from the grouped BF16 copy (sell.cuh): pairs of slots part,
-// part + S, ...
-__device__ __forceinline__ void part16(long Sb, long Gb, int t, int W, int part, int S, const int *__restrict__ scols,
+// part + S, ... (the slot beyond W holds zeros)
+__device__ __forceinline__ void part16(const Home &h, long Gb, int t, int part, int S, const int *__restrict__ scols,
                                        const __nv_bfloat16 *__restrict__ svg, const float *x, float (&y)[3]) {
-    const int *cp = scols + Sb * kSlice + t;
+    const int *cp = scols + (long)h.S * kSlice + t;
     const unsigned *vp = reinterpret_cast<const unsigned *>(svg) + (Gb * 9 * kSlice + t) * 2;
     y[0] = y[1] = y[2] = 0.f;
-    for (int k = 2 * part; k < W; k += 2 * S) {
-        const bool two = k + 1 < W;  // the slot beyond W holds zeros; its column is read from slot k
-        const int c0 = __ldg(cp + (long)k * kSlice), c1 = __ldg(cp + (long)(two ? k + 1 : k) * kSlice);
+    int c0 = h.c0, c1 = h.c1;
+    for (int k = 2 * part; k < h.W; k += 2 * S) {
+        const bool two = k + 1 < h.W;
+        if (k != 2 * part) {
+            c0 = __ldg(cp + (long)k * kSlice);
+            c1 = __ldg(cp + (long)(two ? k + 1 : k) * kSlice);
+        }
         unsigned raw[9];
 #pragma unroll
         for (int e = 0; e < 9; ++e) raw[e] = __ldg(vp + ((long)(k >> 2) * 9 + e) * kSlice * 2 + ((k >> 1) & 1));
@@ -140,7 +168,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     __shared__ unsigned s_touch[MIXED ? kResMaxM / 6 / 32 : 1];
     __shared__ int s_fail, s_k, s_done;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const unsigned G = gridDim.x;
+    const int G = gridDim.x;
     const int sl0 = blockIdx.x * a.spc, sl1 = min(a.nslice, sl0 + a.spc);
     const int row0 = sl0 * kSlice, row1 = min(a.nfree, sl1 * kSlice);
     unsigned target = 0;
@@ -160,9 +188,26 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
             atomicOr(&s_touch[I >> 5], 1u << (I & 31));
         }
     }
-    auto sync = [&]() {
+    // this warp's slices of the first round
+    const int ng64 = kResWarps / a.S64, g64 = w / a.S64, p64 = w - g64 * a.S64;
+    Home h64{0, 0, 0, 0}, h16{0, 0, 0, 0};
+    long G16 = 0;
+    if (g64 < ng64 && sl0 + g64 < sl1) h64 = home(a.sl_ptr, a.scols, sl0 + g64, lane, p64, p64 + a.S64);
+    const int ng16 = kResWarps / a.S16, g16 = w / a.S16, p16 = w - g16 * a.S16;
+    if (MIXED && g16 < ng16 && sl0 + g16 < sl1) {
+        h16 = home(a.sl_ptr, a.scols, sl0 + g16, lane, 2 * p16, 2 * p16 + 1);
+        G16 = __ldg(a.sl_g + sl0 + g16);
+    }
+    // a barrier in two steps: what a CTA needs of its own rows next is loaded
+    // between them
+    auto arrive = [&]() {
         target += G;
-        return grid_barrier(a.bar, target, a.limit_ns, &s_fail);
+        grid_arrive(a.bar);
+    };
+    auto wait = [&]() { return grid_wait(a.bar, target, a.limit_ns, &s_fail); };
+    auto sync = [&]() {
+        arrive();
+        return wait();
     };
     // this CTA's partial of one or two sums (threads' values x, y)
     auto put = [&](double x, double *Px, double y, double *Py) {
@@ -182,6 +227,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
             }
         }
     };
+    // s_sum[slot] = the sum of the CTAs' partials, by one warp; read after the
+    // next block barrier (the products' own: the sums are under them)
+    auto sum = [&](int slot, const double *P) {
+        const double v = warp_partials(P, G);
+        if (lane == 0) s_sum[slot] = v;
+    };
     auto stop = [&](int status, int iters) {
         if (blockIdx.x == 0 && tid == 0) {
             a.fl->done = 1;
@@ -195,73 +246,82 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
             a.fl->status = OFEA_ERR_TIMEOUT;
         }
     };
-    // y = (this CTA's rows of) K x in rounds of kResWarps / S slices; fin(row, y)
-    // by the first warps, one row per lane
-    auto spmm64 = [&](auto x, auto fin) {
-        const int S = a.S64, ng = kResWarps / S, g = w / S, part = w - g * S;
+    // y = (this CTA's rows of) K x in rounds of kResWarps / S slices; the first
+    // warps, one row per lane, load pre(row) and pass it to fin(row, y, own)
+    // (nothing when done() after the first block barrier: returns true)
+    auto spmm64 = [&](auto x, auto pre, auto done, auto fin) {
+        const int S = a.S64, ng = ng64, g = g64;
         for (int b = sl0; b < sl1; b += ng) {
             double y[3] = {0.0, 0.0, 0.0};
             if (g < ng && b + g < sl1) {
-                const int Sb = __ldg(a.sl_ptr + b + g), W = __ldg(a.sl_ptr + b + g + 1) - Sb;
-                part64(Sb, lane, W, part, S, a.scols, a.sv64, x, y);
+                const Home h = b == sl0 ? h64 : home(a.sl_ptr, a.scols, b + g, lane, p64, p64 + S);
+                part64(h, lane, p64, S, a.scols, a.sv64, x, y);
 #pragma unroll
                 for (int i = 0; i < 3; ++i) s_red[(w * 3 + i) * 32 + lane] = y[i];
             }
-            __syncthreads();
             const int row = (b + w) * kSlice + lane;
-            if (w < ng && b + w < sl1 && row < a.nfree) {
+            const bool mine = w < ng && b + w < sl1 && row < a.nfree;
+            __syncthreads();
+            if (b == sl0 && done()) return true;
+            if (mine) {
+                const auto own = pre(row);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    y[i] = 0.0;
-                    for (int p = 0; p < S; ++p) y[i] += s_red[((w * S + p) * 3 + i) * 32 + lane];
-                }
-                fin(row, y);
+                for (int i = 0; i < 3; ++i) y[i] = 0.0;
+                for (int p = 0; p < S; ++p)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) y[i] += s_red[((w * S + p) * 3 + i) * 32 + lane];
+                fin(row, y, own);
             }
             if (b + ng < sl1) __syncthreads();
         }
+        return false;
     };
-    auto spmm16 = [&](const float *x, auto fin) {
+    auto spmm16 = [&](const float *x, auto pre, auto done, auto fin) {
         float *red = reinterpret_cast<float *>(s_red);
-        const int S = a.S16, ng = kResWarps / S, g = w / S, part = w - g * S;
+        const int S = a.S16, ng = ng16, g = g16;
         for (int b = sl0; b < sl1; b += ng) {
             float y[3] = {0.f, 0.f, 0.f};
             if (g < ng && b + g < sl1) {
-                const int Sb = __ldg(a.sl_ptr + b + g), W = __ldg(a.sl_ptr + b + g + 1) - Sb;
-                part16(Sb, __ldg(a.sl_g + b + g), lane, W, part, S, a.scols, a.svg, x, y);
+                const Home h = b == sl0 ? h16 : home(a.sl_ptr, a.scols, b + g, lane, 2 * p16, 2 * p16 + 1);
+                part16(h, b == sl0 ? G16 : (long)__ldg(a.sl_g + b + g), lane, p16, S, a.scols, a.svg, x, y);
 #pragma unroll
                 for (int i = 0; i < 3; ++i) red[(w * 3 + i) * 32 + lane] = y[i];
             }
-            __syncthreads();
             const int row = (b + w) * kSlice + lane;
-            if (w < ng && b + w < sl1 && row < a.nfree) {
+            const bool mine = w < ng && b + w < sl1 && row < a.nfree;
+            __syncthreads();
+            if (b == sl0 && done()) return true;
+            if (mine) {
+                const auto own = pre(row);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    y[i] = 0.f;
-                    for (int p = 0; p < S; ++p) y[i] += red[((w * S + p) * 3 + i) * 32 + lane];
-                }
-                fin(row, y);
+                for (int i = 0; i < 3; ++i) y[i] = 0.f;
+                for (int p = 0; p < S; ++p)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) y[i] += red[((w * S + p) * 3 + i) * 32 + lane];
+                fin(row, y, own);
             }
             if (b + ng < sl1) __syncthreads();
         }
+        return false;
     };
-    // z_{kk+1} = M(b32), x32 = the pre-smoothed start; partials r.z_{kk+1}, r.z_kk.
-    // rr: stop when ||r||^2 is below the target (not before the first).
+    struct F3 {
+        float v[3];
+    };
+    auto f3 = [](const float *p, int row) { return F3{{p[3L * row], p[3L * row + 1], p[3L * row + 2]}}; };
+    auto never = [] { return false; };
+    // z_{kk+1} = M(b32), x32 = the pre-smoothed start; partials r.z_{kk+1} and
+    // r.z_kk.  With check the solve stops when ||r||^2 has reached the target.
+    // 0, 1: stopped, 2: a wait ran out.
     auto vcycle = [&](int kk, bool check) -> int {
-        if (check) {
-            if (w == 0) {
-                const double rr = warp_partials(a.P.rr, G);
-                if (lane == 0) s_sum[0] = rr;
-            }
-            __syncthreads();
-            if (s_sum[0] <= a.tol2) {
-                stop(OFEA_OK, kk + 1);
-                return 1;
-            }
-        }
-        spmm16(a.x32, [&](int row, float (&y)[3]) {
+        if (check && w == kResWarps - 1) sum(0, a.P.rr);
+        if (spmm16(a.x32, [&](int row) { return f3(a.b32, row); }, [&] { return check && s_sum[0] <= a.tol2; },
+                   [&](int row, float (&y)[3], const F3 &b) {
 #pragma unroll
-            for (int i = 0; i < 3; ++i) a.t32[3L * row + i] = a.b32[3L * row + i] - y[i];
-        });
+                       for (int i = 0; i < 3; ++i) a.t32[3L * row + i] = b.v[i] - y[i];
+                   })) {
+            stop(OFEA_OK, kk + 1);
+            return 1;
+        }
         if (!sync()) return 2;
         {  // c = Z^T t, one CTA per aggregate
             float *sh = reinterpret_cast<float *>(s_red);  // [6][warps]
@@ -324,21 +384,28 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
         float *znew = ((kk + 1) & 1) ? a.zB : a.zA;
         const float *zold = ((kk + 1) & 1) ? a.zA : a.zB;
         double prz = 0.0, przo = 0.0;
-        spmm16(a.x32, [&](int row, float (&y)[3]) {
-            float d[3], o[3];
+        struct Own {
+            F3 b, x, z;
+            double r[3];
+        };
+        spmm16(a.x32,
+               [&](int row) {
+                   return Own{f3(a.b32, row), f3(a.x32, row), f3(zold, row), {a.r[3L * row], a.r[3L * row + 1], a.r[3L * row + 2]}};
+               },
+               never,
+               [&](int row, float (&y)[3], const Own &n) {
+                   float d[3], o[3];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) d[i] = a.b32[3L * row + i] - y[i];
-            block3_apply(a.Dinv32 + 9L * row, d, o);
+                   for (int i = 0; i < 3; ++i) d[i] = n.b.v[i] - y[i];
+                   block3_apply(a.Dinv32 + 9L * row, d, o);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const long dd = 3L * row + i;
-                const float zn = fmaf(a.wsm, o[i], a.x32[dd]);
-                const double rv = a.r[dd];
-                prz += rv * (double)zn;
-                przo += rv * (double)zold[dd];
-                znew[dd] = zn;
-            }
-        });
+                   for (int i = 0; i < 3; ++i) {
+                       const float zn = fmaf(a.wsm, o[i], n.x.v[i]);
+                       prz += n.r[i] * (double)zn;
+                       przo += n.r[i] * (double)n.z.v[i];
+                       znew[3L * row + i] = zn;
+                   }
+               });
         put(prz, ((kk + 1) & 1) ? a.P.rz1 : a.P.rz0, przo, a.P.rzo);
         return sync() ? 0 : 2;
     };
@@ -351,57 +418,72 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     }
     for (int it = 0; it < a.iters; ++it, ++k) {
         double *Pcur = (k & 1) ? a.P.rz1 : a.P.rz0, *Pother = (k & 1) ? a.P.rz0 : a.P.rz1;
-        // the sums of the phase before: warps 1 .. 4, one each, while the
-        // other warps are already in the product
-        if (w == 1) {
-            const double v = warp_partials(Pcur, G);
-            if (lane == 0) s_sum[0] = v;
-        } else if (w == 2 && k > 0) {
-            const double v = warp_partials(Pother, G);
-            if (lane == 0) s_sum[1] = v;
-        } else if (w == 3 && MIXED && k > 0) {
-            const double v = warp_partials(a.P.rzo, G);
-            if (lane == 0) s_sum[2] = v;
-        } else if (w == 4 && !MIXED) {
-            const double v = warp_partials(a.P.rr, G);
-            if (lane == 0) s_sum[2] = v;
-        }
-        if (!MIXED) {
-            __syncthreads();
-            if (s_sum[2] <= a.tol2) {
-                stop(OFEA_OK, k);
-                return;
-            }
-        }
+        // the sums of the phases before, by the last warps
+        if (w == kResWarps - 1) sum(0, Pcur);
+        else if (w == kResWarps - 2 && k > 0) sum(1, Pother);
+        else if (w == kResWarps - 3) sum(2, MIXED ? a.P.rzo : a.P.rr);
         const double *pold = (k & 1) ? a.p1 : a.p0;
         double *pnew = (k & 1) ? a.p0 : a.p1;
         const float *zf = (k & 1) ? a.zB : a.zA;
         const double *zd = a.z;
-        double ppq = 0.0;
+        double ppq = 0.0, beta = 0.0;
         auto zat = [&](long d) { return MIXED ? (double)zf[d] : zd[d]; };
-        spmm64(zat, [&](int row, double (&y)[3]) {
-            double beta = 0.0;  // the partial sums are complete: the product's block barrier is behind
-            if (k > 0) beta = MIXED ? (s_sum[0] - s_sum[2]) / s_sum[1] : s_sum[0] / s_sum[1];
+        struct Own {
+            double p[3], z[3], q[3];
+        };
+        if (spmm64(zat,
+                   [&](int row) {
+                       Own o;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const long d = 3L * row + i;
-                const double pn = fma(beta, pold[d], zat(d));
-                const double qn = fma(beta, a.q[d], y[i]);  // K p = K z + beta K p_old
-                pnew[d] = pn;
-                a.q[d] = qn;
-                ppq += pn * qn;
-            }
-        });
+                       for (int i = 0; i < 3; ++i) {
+                           o.p[i] = pold[3L * row + i];
+                           o.z[i] = zat(3L * row + i);
+                           o.q[i] = a.q[3L * row + i];
+                       }
+                       return o;
+                   },
+                   [&] {
+                       if (k > 0) beta = (MIXED ? s_sum[0] - s_sum[2] : s_sum[0]) / s_sum[1];
+                       return !MIXED && s_sum[2] <= a.tol2;
+                   },
+                   [&](int row, double (&y)[3], const Own &o) {
+#pragma unroll
+                       for (int i = 0; i < 3; ++i) {
+                           const double pn = fma(beta, o.p[i], o.z[i]);
+                           const double qn = fma(beta, o.q[i], y[i]);  // K p = K z + beta K p_old
+                           pnew[3L * row + i] = pn;
+                           a.q[3L * row + i] = qn;
+                           ppq += pn * qn;
+                       }
+                   })) {
+            stop(OFEA_OK, k);
+            return;
+        }
         put(ppq, a.P.pq, 0.0, nullptr);
-        if (!sync()) {
+        arrive();
+        // B: alpha, u, r, and the block-Jacobi step.  The rows are this CTA's
+        // own: the first one's entries are loaded under the wait.
+        struct Row {
+            double u[3], r[3], p[3], q[3];
+        };
+        auto load = [&](int i) {
+            Row t;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                t.u[c] = a.u[3L * i + c];
+                t.r[c] = a.r[3L * i + c];
+                t.p[c] = pnew[3L * i + c];
+                t.q[c] = a.q[3L * i + c];
+            }
+            return t;
+        };
+        int i = row0 + tid;
+        Row cur = load(i < row1 ? i : row0);
+        if (!wait()) {
             timed_out();
             return;
         }
-        // B: alpha, u, r, and the block-Jacobi step
-        if (w == 0) {
-            const double v = warp_partials(a.P.pq, G);
-            if (lane == 0) s_sum[3] = v;
-        }
+        if (w == 0) sum(3, a.P.pq);
         __syncthreads();
         const double pq = s_sum[3], rz = s_sum[0];
         if (!(pq > 0.0) || !isfinite(pq)) {
@@ -410,14 +492,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
         }
         const double alpha = rz / pq;
         double prr = 0.0, prz = 0.0;
-        for (int i = row0 + tid; i < row1; i += kResThreads) {
+        while (i < row1) {
             double rv[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const long d = 3L * i + c;
-                a.u[d] = fma(alpha, pnew[d], a.u[d]);
-                rv[c] = fma(-alpha, a.q[d], a.r[d]);
-                a.r[d] = rv[c];
+                a.u[3L * i + c] = fma(alpha, cur.p[c], cur.u[c]);
+                rv[c] = fma(-alpha, cur.q[c], cur.r[c]);
+                a.r[3L * i + c] = rv[c];
                 prr += rv[c] * rv[c];
             }
             if (MIXED) {
@@ -437,6 +518,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
                     prz += rv[c] * zz[c];
                 }
             }
+            i += kResThreads;
+            if (i < row1) cur = load(i);
         }
         if (MIXED) put(prr, a.P.rr, 0.0, nullptr);
         else put(prr, a.P.rr, prz, Pother);
@@ -461,11 +544,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
 bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
     const int nslice = (c->nfree + kSlice - 1) / kSlice;
     // MIXED: up to 3,500 slices (336k DOF), beyond which the launch-per-phase
-    // kernels' wider grids win (288k DOF: 102 us per iteration here, 132
+    // kernels' wider grids win (288k DOF: 98 us per iteration here, 132
     // there; 467k DOF: 191 here, 164 there, the coarse solve of 930 unknowns
-    // repeated by every CTA); PCG64 is the faster one at every size measured
-    // (1.5k DOF 9.0 against 27.9 us, 77k 11.0 / 24.5, 139k 20.7 / 58.0, 706k
-    // 105 / 122).
+    // repeated by every CTA); PCG64 with the stored K is the faster one at
+    // every size measured (706k DOF 105 against 122 us).
     if (nslice < 1) return false;
     if (mixed && (nslice > 3500 || c->coarse.m > kResMaxM)) return false;
     p.spc = (nslice + c->num_sms - 1) / c->num_sms;

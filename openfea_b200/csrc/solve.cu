@@ -575,7 +575,7 @@ struct StopFlagScope {
 
 // Block rows from which the outer products of a linear C3D8 model are formed
 // from its elements (matfree.cu).  Below, K stays in L2 and the resident
-// solver's PCG64 iteration is the faster one (139k DOF: 20.7 us there, 27.9
+// solver's PCG64 iteration is the faster one (139k DOF: 18.4 us there, 27.9
 // from the elements; 288k: 48 and 37; 706k: 105 and 68; 1.56M: 221 and 130;
 // MIXED, launch per phase, stored K and elements: 706k 215 and 170, 1.56M 398
 // and 311).  The smoother's products keep the stored BF16 K: formed from the

@@ -68,10 +68,12 @@ struct GridBar {
     unsigned count;
     int err;
 };
-__device__ __forceinline__ bool grid_barrier(GridBar *bar, unsigned target, unsigned long long limit_ns, int *s_fail) {
+__device__ __forceinline__ void grid_arrive(GridBar *bar) {
     __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->count) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(GridBar *bar, unsigned target, unsigned long long limit_ns, int *s_fail) {
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->count) : "memory");
         unsigned long long t0 = 0;
         for (unsigned spin = 1;; ++spin) {
             unsigned c;
@@ -90,6 +92,10 @@ __device__ __forceinline__ bool grid_barrier(GridBar *bar, unsigned target, unsi
     }
     __syncthreads();
     return *s_fail == 0;
+}
+__device__ __forceinline__ bool grid_barrier(GridBar *bar, unsigned target, unsigned long long limit_ns, int *s_fail) {
+    grid_arrive(bar);
+    return grid_wait(bar, target, limit_ns, s_fail);
 }
 
 // Per-CTA partial sums, all arrays of kMaxGrid doubles.

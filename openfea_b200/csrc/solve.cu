@@ -74,14 +74,14 @@ void spmv64(ofea_ctx *c, const double *d_x, double *d_y) {
 
 // r = f - K u, z = Dinv r; partials r.z -> rz0, r.r -> rr, f.f -> ff.
 __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_residual64(
-    int nfree, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
+    int nfree, bool zero_u, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
     const double *__restrict__ sv64, const double *__restrict__ Dinv, const double *__restrict__ f,
     const double *__restrict__ u, double *__restrict__ r, double *__restrict__ z, Parts P) {
     __shared__ double sh[kWarpsPerBlock];
     double prz = 0, prr = 0, pff = 0;
     for_each_sell_row(nfree, sl_ptr, [&](int rw, long S, int t, int W) {
-        double y[3], rv[3], zz[3];
-        sell_row<double, 2>(S, t, W, scols, sv64, [&](int k) { return u[k]; }, y[0], y[1], y[2]);
+        double y[3] = {0.0, 0.0, 0.0}, rv[3], zz[3];
+        if (!zero_u) sell_row<double, 2>(S, t, W, scols, sv64, [&](int k) { return u[k]; }, y[0], y[1], y[2]);
         for (int i = 0; i < 3; ++i) {
             const double fi = f[3L * rw + i];
             rv[i] = fi - y[i];
@@ -305,16 +305,16 @@ __global__ void __launch_bounds__(kBlock) k_fcg_B(
 
 // Init for MIXED: r = f - K64 u (FP64), ||r||^2, ||f||^2, b32, x32 pre-smoothing.
 __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_init(
-    int nfree, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
+    int nfree, bool zero_u, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
     const double *__restrict__ sv64, const float *__restrict__ Dinv32, float w,
     const double *__restrict__ f, const double *__restrict__ u, double *__restrict__ r,
     float *__restrict__ b32, float *__restrict__ x32, Parts P) {
     __shared__ double sh[kWarpsPerBlock];
     double prr = 0, pff = 0;
     for_each_sell_row(nfree, sl_ptr, [&](int rw, long S, int t, int W) {
-        double y[3];
+        double y[3] = {0.0, 0.0, 0.0};
         float b[3], x[3];
-        sell_row<double, 2>(S, t, W, scols, sv64, [&](int k) { return u[k]; }, y[0], y[1], y[2]);
+        if (!zero_u) sell_row<double, 2>(S, t, W, scols, sv64, [&](int k) { return u[k]; }, y[0], y[1], y[2]);
         for (int i = 0; i < 3; ++i) {
             const double fi = f[3L * rw + i];
             const double rv = fi - y[i];
@@ -374,11 +374,17 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_post(
     }
 }
 
-// Single CTA: final reductions of rr and ff into out[0..1].
-__global__ void k_final_norms(Parts P, double *out) {
+// Single CTA: final reductions of rr and ff into out[0..1]; the partials of rr
+// and rz0 become G entries of the same sum.
+__global__ void k_final_norms(Parts P, int G, double *out) {
     __shared__ double sh[kWarpsPerBlock];
     const double rr = sum_partials(P.rr, P.G, sh);
     const double ff = sum_partials(P.ff, P.G, sh);
+    const double rz = sum_partials(P.rz0, P.G, sh);
+    for (int i = threadIdx.x; i < G; i += blockDim.x) {
+        P.rr[i] = i ? 0.0 : rr;
+        P.rz0[i] = i ? 0.0 : rz;
+    }
     if (threadIdx.x == 0) {
         out[0] = rr;
         out[1] = ff;
@@ -534,16 +540,15 @@ void drive(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, int per_chunk, 
 }
 
 // The iterations by the resident solver (resident.cu): it stops by itself, so
-// one launch takes up to kResidentChunk iterations; with a time budget, a
-// poll interval of the caller's or a per-chunk callback the launches are as
-// long as those.  The iteration limit is rounded up to whole poll intervals.
+// one launch takes up to kResidentChunk iterations; with a time budget or a
+// poll interval of the caller's the launches are as long as those.  The iteration limit is rounded up to whole poll intervals.
 constexpr int kResidentChunk = 4096;
 void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const ResidentPlan &plan, bool mixed,
                     int per_chunk, double *d_u, float wsm, double tol2, Flags &hf, long long &launches,
-                    bool &timed_out, double t_start, const std::function<void(const double *)> &on_chunk) {
+                    bool &timed_out, double t_start) {
     cudaStream_t s = c->stream;
     Flags *h = reinterpret_cast<Flags *>(c->w.hflags.p);
-    const bool polled = o.time_budget_s > 0 || o.check_every > 0 || on_chunk;
+    const bool polled = o.time_budget_s > 0 || o.check_every > 0;
     const long limit = ((long)o.max_iter + per_chunk - 1) / per_chunk * per_chunk;
     for (long done = 0;;) {
         const int iters = (int)std::min<long>(polled ? per_chunk : kResidentChunk, limit - done);
@@ -553,7 +558,6 @@ void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const 
         OFEA_CUDA(cudaMemcpyAsync(h, ws.fl, sizeof(Flags), cudaMemcpyDeviceToHost, s));
         OFEA_CUDA(cudaStreamSynchronize(s));
         if (h->done || done >= limit) break;
-        if (on_chunk) on_chunk(c->w.r.p);
         if (o.time_budget_s > 0 && now_s() - t_start > o.time_budget_s) {
             timed_out = true;
             break;
@@ -646,28 +650,32 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         w.z.ensure(n);
     }
     ResidentPlan plan;
-    const bool matfree = nf >= kMatfreeRows && matfree_ready(c);
-    const bool resident = !learned && !(matfree && !mixed) && resident_plan(c, mixed, plan);
+    // A solve that hands its residuals to a callback (the learned stage's
+    // training samples) keeps the launch-per-phase kernels on the stored K and
+    // their order of sums: training amplifies rounding (samples 1e-13 apart on
+    // an unsmoothed density field gave weights 3 % apart), so a model trained
+    // before is still the one that training gives.
+    const bool sampling = (bool)on_chunk;
+    const bool matfree = !sampling && nf >= kMatfreeRows && matfree_ready(c);
+    const bool resident = !sampling && !learned && !(matfree && !mixed) && resident_plan(c, mixed, plan);
     if (resident && mixed) coarse_dense_inverse(c);
     const int G = resident ? plan.G : solver_grid(c);
     Workspace ws = setup(c, G);
     const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;
     for (int attempt = 0; attempt < 8; ++attempt) {
-        OFEA_CUDA(cudaMemsetAsync(w.p0.p, 0, sizeof(double) * n, s));
-        OFEA_CUDA(cudaMemsetAsync(w.p1.p, 0, sizeof(double) * n, s));
-        OFEA_CUDA(cudaMemsetAsync(w.q.p, 0, sizeof(double) * n, s));  // q = K p is kept by recurrence
-        OFEA_CUDA(cudaMemsetAsync(ws.fl, 0, sizeof(Flags), s));
-        if (mixed) {
-            OFEA_CUDA(cudaMemsetAsync(w.z32a.p, 0, sizeof(float) * n, s));
-            OFEA_CUDA(cudaMemsetAsync(w.z32b.p, 0, sizeof(float) * n, s));
-            k_fcg_init<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, c->Dinv32.p, wsm, d_f,
-                                            d_u, w.r.p, w.b32.p, w.x32.p, ws.P);
-        } else {
-            k_residual64<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sv64.p, c->Dinv.p, d_f, d_u,
-                                               w.r.p, w.z.p, ws.P);
-        }
+        // the whole GPU forms the residual, whatever the iterations run on; its
+        // partials are then folded into the G the iterations read.  Every solve
+        // starts from u = 0: the first residual is f, without the product.
+        Parts PI = ws.P;
+        PI.G = solver_grid(c);
+        if (mixed)
+            k_fcg_init<<<PI.G, kBlock, 0, s>>>(nf, attempt == 0, c->sl_ptr.p, c->scols.p, c->sv64.p, c->Dinv32.p, wsm, d_f,
+                                               d_u, w.r.p, w.b32.p, w.x32.p, PI);
+        else
+            k_residual64<<<PI.G, kBlock, 0, s>>>(nf, attempt == 0, c->sl_ptr.p, c->scols.p, c->sv64.p, c->Dinv.p, d_f, d_u,
+                                                 w.r.p, w.z.p, PI);
         OFEA_CHECK_LAUNCH();
-        k_final_norms<<<1, kBlock, 0, s>>>(ws.P, ws.scal);
+        k_final_norms<<<1, kBlock, 0, s>>>(PI, G, ws.scal);
         OFEA_CUDA(cudaMemcpyAsync(w.hscal.p, ws.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
         OFEA_CUDA(cudaStreamSynchronize(s));
         launches += 2;
@@ -684,12 +692,20 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         }
         if (rel <= o.rtol || total_iters >= o.max_iter || timed_out) break;
         if (attempt > 0) ++restarts;
+        OFEA_CUDA(cudaMemsetAsync(w.p0.p, 0, sizeof(double) * n, s));
+        OFEA_CUDA(cudaMemsetAsync(w.p1.p, 0, sizeof(double) * n, s));
+        OFEA_CUDA(cudaMemsetAsync(w.q.p, 0, sizeof(double) * n, s));  // q = K p is kept by recurrence
+        OFEA_CUDA(cudaMemsetAsync(ws.fl, 0, sizeof(Flags), s));
+        if (mixed) {
+            OFEA_CUDA(cudaMemsetAsync(w.z32a.p, 0, sizeof(float) * n, s));
+            OFEA_CUDA(cudaMemsetAsync(w.z32b.p, 0, sizeof(float) * n, s));
+        }
         // recursive residual target a little below rtol; the true residual is re-checked
         const double tol2 = (0.5 * o.rtol) * (0.5 * o.rtol) * ff;
         ofea_solve_opts oo = o;
         oo.max_iter = o.max_iter - total_iters;
         if (resident) {
-            drive_resident(c, oo, ws, plan, mixed, per_chunk, d_u, wsm, tol2, hf, launches, timed_out, t_start, on_chunk);
+            drive_resident(c, oo, ws, plan, mixed, per_chunk, d_u, wsm, tol2, hf, launches, timed_out, t_start);
         } else if (mixed) {
             // the V-cycle kernels of this attempt return at once once the
             // solve has stopped (the flag is cleared at every attempt)
@@ -728,8 +744,15 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         } else {
             auto chunk = [&](int iters) {
                 for (int it = 0; it < iters; ++it) {
-                    matfree_forces(c, w.z.p, ws.fl);
-                    k_pcg64_A<<<G, kBlock, 0, s>>>(nf, matfree_rows(c), w.z.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+                    auto A = [&](auto K) {
+                        k_pcg64_A<<<G, kBlock, 0, s>>>(nf, K, w.z.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
+                    };
+                    if (matfree) {
+                        matfree_forces(c, w.z.p, ws.fl);
+                        A(matfree_rows(c));
+                    } else {
+                        A(sell_rows(c));
+                    }
                     k_pcg64_B<<<G, kBlock, 0, s>>>(nf, c->Dinv.p, w.p0.p, w.p1.p, w.q.p, d_u, w.r.p, w.z.p,
                                                    ws.P, ws.fl);
                 }
@@ -737,7 +760,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
             };
             std::function<void()> after;
             if (on_chunk) after = [&] { on_chunk(w.r.p); };
-            drive(c, oo, ws, per_chunk, chunk, hf, launches, 3, timed_out, t_start, after);
+            drive(c, oo, ws, per_chunk, chunk, hf, launches, matfree ? 3 : 2, timed_out, t_start, after);
         }
         total_iters += hf.iters;
         if (hf.status == OFEA_ERR_BREAKDOWN) break;

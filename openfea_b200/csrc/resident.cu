@@ -37,6 +37,10 @@
 //
 // Every wait is bounded (%globaltimer): on expiry the kernel sets the error
 // status and every CTA returns.
+#include <map>
+#include <mutex>
+#include <type_traits>
+
 #include "precond.cuh"
 #include "resident.cuh"
 #include "sell.cuh"
@@ -539,7 +543,441 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     }
 }
 
+// --------------------------------------------------- one cluster, small K --
+//
+// The same iterations for matrices of a few thousand rows in one thread-block
+// cluster.  A grid barrier costs 2,000 to 5,000 cycles (arrival after the
+// phase's stores have drained to L2, the spin, the first load after it); here
+// the gathered vectors (z; the V-cycle's x) are kept whole in every CTA's shared
+// memory, the owners of rows write them into all CTAs, partial sums go the
+// same way, and a phase ends at the cluster's hardware barrier.  The other
+// vectors live in the owner's shared memory.  K and the inverse diagonal blocks
+// are read through L1.  The coarse level: every CTA restricts its own rows, the
+// partial c of all CTAs are summed by each, and e = E^-1 c and x += Z e are
+// formed by every CTA for its whole copy of x, so the coarse correction costs
+// one barrier.  Barriers per iteration: PCG64 2, MIXED 4.
+//
+// The sums of a phase go to an inbox of their own; an inbox, and a whole
+// vector, is written again only after a barrier that follows its last reading.
+//
+// Per iteration, grid of CTAs before, cluster after: PCG64 7.6 -> 5.3 us at 1.5k
+// DOF, 7.9 -> 6.5 at 3.3k; MIXED 19.5 -> 12.5 and 20.4 -> 15.0.  With 32 warps
+// per CTA instead of 16 the idle ones' instructions cost more than their help
+// (6.3 and 14.2 us).  Bound by the instruction chains of its phases (the
+// reductions' shuffles, the product's combine) and 700 cycles per barrier.
+
+namespace {
+
+constexpr int kClMax = 16;       // CTAs of the largest cluster (beyond 8 if the device allows it)
+constexpr int kClSpc = 4;        // slices per CTA at most
+constexpr int kClRows = kClSpc * kSlice;
+constexpr int kClM = 192;        // coarse unknowns at most
+constexpr int kClThreads = 512, kClWarps = kClThreads / 32;
+
+struct ClShared {
+    double red[kClWarps * 3 * 32];
+    double u[3 * kClRows], r[3 * kClRows], p[3 * kClRows], q[3 * kClRows];
+    double in[4][2][kClMax];     // inboxes: p.q; ||r||^2 (and r.z); r.z and r.z_old
+    float b[3 * kClRows], t[3 * kClRows];
+    float cin[kClMax][kClM], c[kClM], e[kClM];
+    double w[2][kClWarps];
+};
+
+// The cluster's barrier.  Writes into other CTAs are ordered by their writers
+// (peer_done after the stores), this CTA's own by the block barrier: a
+// releasing arrival of every warp cost a fence in each.
+__device__ __forceinline__ void peer_done() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The same shared-memory address in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned peer(const void *p, unsigned rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), o;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(rank));
+    return o;
+}
+__device__ __forceinline__ void peer_st(unsigned a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+__device__ __forceinline__ void peer_st(unsigned a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void peer_st(unsigned a, float4 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+}  // namespace
+
+template <bool MIXED>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    ClShared &sh = *reinterpret_cast<ClShared *>(dyn);
+    using ZT = typename std::conditional<MIXED, float, double>::type;
+    const int npad = 3 * kSlice * a.nslice;  // whole vectors, padded to slices
+    ZT *zr = reinterpret_cast<ZT *>(dyn + sizeof(ClShared));
+    float *xr = reinterpret_cast<float *>(zr + npad);  // MIXED
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int C = gridDim.x;
+    const int rank = (int)cluster_rank();
+    const int sl0 = min(a.nslice, rank * a.spc), sl1 = min(a.nslice, sl0 + a.spc);
+    const int row0 = sl0 * kSlice, row1 = min(a.nfree, sl1 * kSlice), own3 = 3 * (row1 - row0);
+    if (*(volatile int *)&a.fl->done) return;  // written by an earlier launch: the same in every CTA
+    int k = *(volatile int *)&a.fl->itA;
+    // state of the launch before
+    {
+        const double *pold = (k & 1) ? a.p1 : a.p0;
+        for (int i = tid; i < own3; i += kClThreads) {
+            const long d = 3L * row0 + i;
+            sh.u[i] = a.u[d];
+            sh.r[i] = a.r[d];
+            sh.p[i] = pold[d];
+            sh.q[i] = a.q[d];
+            if (MIXED) sh.b[i] = a.b32[d];
+        }
+        const float *zf = (k & 1) ? a.zB : a.zA;
+        for (int i = tid; i < npad; i += kClThreads) {
+            if constexpr (MIXED) {
+                zr[i] = i < 3 * a.nfree ? zf[i] : 0.f;
+                xr[i] = i < 3 * a.nfree ? a.x32[i] : 0.f;
+            } else {
+                zr[i] = i < 3 * a.nfree ? a.z[i] : 0.0;
+            }
+        }
+    }
+    double rz = warp_partials((k & 1) ? a.P.rz1 : a.P.rz0, a.P.G), rzp = warp_partials((k & 1) ? a.P.rz0 : a.P.rz1, a.P.G);
+    double rzo = MIXED ? warp_partials(a.P.rzo, a.P.G) : 0.0, rr = warp_partials(a.P.rr, a.P.G);
+    const int ng64 = kClWarps / a.S64, g64 = w / a.S64, p64 = w - g64 * a.S64;
+    const int ng16 = kClWarps / a.S16, g16 = w / a.S16, p16 = w - g16 * a.S16;
+    Home h64{0, 0, 0, 0}, h16{0, 0, 0, 0};
+    long G16 = 0;
+    if (g64 < ng64 && sl0 + g64 < sl1) h64 = home(a.sl_ptr, a.scols, sl0 + g64, lane, p64, p64 + a.S64);
+    if (MIXED && g16 < ng16 && sl0 + g16 < sl1) {
+        h16 = home(a.sl_ptr, a.scols, sl0 + g16, lane, 2 * p16, 2 * p16 + 1);
+        G16 = __ldg(a.sl_g + sl0 + g16);
+    }
+    for (int i = tid; i < 4 * 2 * kClMax; i += kClThreads) (&sh.in[0][0][0])[i] = 0.0;
+    // every CTA is here before the first write into another's shared memory
+    cluster_sync();
+
+    // y = K x for the own rows, fin(own row, y)
+    auto spmm = [&](auto half, auto x, auto fin) {
+        constexpr bool BF = decltype(half)::value;
+        using T = typename std::conditional<BF, float, double>::type;
+        T *red = reinterpret_cast<T *>(sh.red);
+        const int S = BF ? a.S16 : a.S64, ng = BF ? ng16 : ng64, g = BF ? g16 : g64, part = BF ? p16 : p64;
+        for (int b = sl0; b < sl1; b += ng) {
+            T y[3] = {0, 0, 0};
+            if (g < ng && b + g < sl1) {
+                const bool first = b == sl0;
+                if constexpr (BF) {
+                    const Home h = first ? h16 : home(a.sl_ptr, a.scols, b + g, lane, 2 * part, 2 * part + 1);
+                    part16(h, first ? G16 : (long)__ldg(a.sl_g + b + g), lane, part, S, a.scols, a.svg, x, y);
+                } else {
+                    const Home h = first ? h64 : home(a.sl_ptr, a.scols, b + g, lane, part, part + S);
+                    part64(h, lane, part, S, a.scols, a.sv64, x, y);
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) red[(w * 3 + i) * 32 + lane] = y[i];
+            }
+            __syncthreads();
+            const int row = (b + w) * kSlice + lane;
+            if (w < ng && b + w < sl1 && row < a.nfree) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) y[i] = 0;
+                for (int p = 0; p < S; ++p)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) y[i] += red[((w * S + p) * 3 + i) * 32 + lane];
+                fin(row - row0, y);
+            }
+            __syncthreads();
+        }
+    };
+    // this CTA's partial sums (of its first nw warps' values) into every CTA's
+    // inbox
+    auto send = [&](int box, int nw, double x, double y) {
+        if (w < nw) {
+            x = warp_sum(x);
+            y = warp_sum(y);
+            if (lane == 0) {
+                sh.w[0][w] = x;
+                sh.w[1][w] = y;
+            }
+        }
+        __syncthreads();
+        if (w < 2) {
+            const double s = warp_sum(lane < nw ? sh.w[w][lane] : 0.0);
+            if (lane < C) peer_st(peer(&sh.in[box][w][rank], lane), s);
+            peer_done();
+        }
+    };
+    auto inbox = [&](int box, int which) {  // unused entries are zero
+        const double *v = sh.in[box][which];
+        double s[kClMax];
+#pragma unroll
+        for (int i = 0; i < kClMax; ++i) s[i] = v[i];
+#pragma unroll
+        for (int d = kClMax / 2; d > 0; d >>= 1)
+#pragma unroll
+            for (int i = 0; i < d; ++i) s[i] += s[i + d];
+        return s[0];
+    };
+    // the own rows of a whole vector, written here, into the other CTAs
+    auto spread = [&](auto *v) {
+        using T = typename std::remove_reference<decltype(*v)>::type;
+        constexpr int E = 16 / (int)sizeof(T);
+        __syncthreads();
+        const int n4 = (own3 + E - 1) / E;
+        for (int i = tid; i < n4 * (C - 1); i += kClThreads) {
+            const int j = i / n4, o = i - j * n4;
+            int to = rank + 1 + j;
+            if (to >= C) to -= C;
+            T *src = v + 3 * row0 + o * E;
+            peer_st(peer(src, to), *reinterpret_cast<const float4 *>(src));
+        }
+        peer_done();
+    };
+    // everything the next launch, or the caller, reads
+    auto leave = [&](int status, int done) {
+        double *pk = (k & 1) ? a.p1 : a.p0;
+        float *zf = (k & 1) ? a.zB : a.zA;
+        for (int i = tid; i < own3; i += kClThreads) {
+            const long d = 3L * row0 + i;
+            a.u[d] = sh.u[i];
+            a.r[d] = sh.r[i];
+            pk[d] = sh.p[i];
+            a.q[d] = sh.q[i];
+            if constexpr (MIXED) {
+                a.b32[d] = sh.b[i];
+                a.x32[d] = xr[d];
+                zf[d] = zr[d];
+            } else {
+                a.z[d] = zr[d];
+            }
+        }
+        if (rank == 0) {
+            double *Pc = (k & 1) ? a.P.rz1 : a.P.rz0, *Po = (k & 1) ? a.P.rz0 : a.P.rz1;
+            for (int j = tid; j < a.P.G; j += kClThreads) {
+                Pc[j] = j ? 0.0 : rz;
+                Po[j] = j ? 0.0 : rzp;
+                a.P.rzo[j] = j ? 0.0 : rzo;
+                a.P.rr[j] = j ? 0.0 : rr;
+            }
+            if (tid == 0) {
+                a.fl->done = done;
+                a.fl->status = status;
+                a.fl->itA = k;
+                a.fl->iters = k;
+            }
+        }
+        cluster_sync();  // no CTA leaves while another may write into it
+    };
+    // z = M(b), from the pre-smoothed x in every CTA; sums r.z, r.z_old
+    auto vcycle = [&]() {
+        if constexpr (MIXED) {
+            spmm(std::true_type{}, (const float *)xr, [&](int i, float (&y)[3]) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sh.t[3 * i + c] = sh.b[3 * i + c] - y[c];
+            });
+            // own rows' part of c = Z^T t, a warp per aggregate
+            for (int I = w; I < a.na; I += kClWarps) {
+                float acc[6] = {0, 0, 0, 0, 0, 0};
+                for (int i = lane; i < row1 - row0; i += 32) {
+                    const float4 o = __ldg(a.row_off + row0 + i);
+                    if (__float_as_int(o.w) != I) continue;
+                    const float tx = sh.t[3 * i], ty = sh.t[3 * i + 1], tz = sh.t[3 * i + 2];
+                    acc[0] += tx;
+                    acc[1] += ty;
+                    acc[2] += tz;
+                    acc[3] += -o.z * ty + o.y * tz;
+                    acc[4] += o.z * tx - o.x * tz;
+                    acc[5] += -o.y * tx + o.x * ty;
+                }
+#pragma unroll
+                for (int q = 0; q < 6; ++q) acc[q] = warp_sum(acc[q]);
+                if (lane < C)
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) peer_st(peer(&sh.cin[rank][6 * I + q], lane), acc[q]);
+            }
+            peer_done();
+            cluster_sync();
+            for (int i = tid; i < a.m; i += kClThreads) {
+                float s = 0.f;
+                for (int j = 0; j < C; ++j) s += sh.cin[j][i];
+                sh.c[i] = s;
+            }
+            __syncthreads();
+            for (int i = w; i < a.m; i += kClWarps) {
+                const float *row = a.Einv + (long)i * a.m;
+                float s = 0.f;
+                for (int j = lane; j < a.m; j += 32) s = fmaf(__ldg(row + j), sh.c[j], s);
+                s = warp_sum(s);
+                if (lane == 0) sh.e[i] = s;
+            }
+            __syncthreads();
+            for (int r = tid; r < a.nfree; r += kClThreads) {
+                const float4 o = __ldg(a.row_off + r);
+                const float *e = sh.e + 6 * __float_as_int(o.w);
+                xr[3 * r] += e[0] + o.z * e[4] - o.y * e[5];
+                xr[3 * r + 1] += e[1] - o.z * e[3] + o.x * e[5];
+                xr[3 * r + 2] += e[2] + o.y * e[3] - o.x * e[4];
+            }
+            __syncthreads();
+            double prz = 0.0, przo = 0.0;
+            spmm(std::true_type{}, (const float *)xr, [&](int i, float (&y)[3]) {
+                float d[3], o[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) d[c] = sh.b[3 * i + c] - y[c];
+                block3_apply(a.Dinv32 + 9L * (row0 + i), d, o);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const int g = 3 * (row0 + i) + c;
+                    const float zn = fmaf(a.wsm, o[c], xr[g]);
+                    const double rv = sh.r[3 * i + c];
+                    prz += rv * (double)zn;
+                    przo += rv * (double)zr[g];
+                    zr[g] = zn;
+                }
+            });
+            spread(zr);
+            send(2, ng16, prz, przo);
+            cluster_sync();
+            rz = inbox(2, 0);
+            rzo = inbox(2, 1);
+        }
+    };
+    if (MIXED && a.first) vcycle();
+    for (int it = 0; it < a.iters; ++it) {
+        if (!MIXED && rr <= a.tol2) {
+            leave(OFEA_OK, 1);
+            return;
+        }
+        const double beta = k > 0 ? (MIXED ? rz - rzo : rz) / rzp : 0.0;
+        double ppq = 0.0;
+        spmm(std::false_type{}, [&](int i) { return (double)zr[i]; }, [&](int i, double (&y)[3]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int d = 3 * i + c;
+                const double pn = fma(beta, sh.p[d], (double)zr[3 * row0 + d]);
+                const double qn = fma(beta, sh.q[d], y[c]);  // K p = K z + beta K p_old
+                sh.p[d] = pn;
+                sh.q[d] = qn;
+                ppq += pn * qn;
+            }
+        });
+        send(0, ng64, ppq, 0.0);
+        cluster_sync();
+        const double pq = inbox(0, 0);
+        if (!(pq > 0.0) || !isfinite(pq)) {
+            leave(OFEA_ERR_BREAKDOWN, 1);
+            return;
+        }
+        const double alpha = rz / pq;
+        double prr = 0.0, prz = 0.0;
+        for (int i = tid; i < row1 - row0; i += kClThreads) {
+            double rv[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int d = 3 * i + c;
+                sh.u[d] = fma(alpha, sh.p[d], sh.u[d]);
+                rv[c] = fma(-alpha, sh.q[d], sh.r[d]);
+                sh.r[d] = rv[c];
+                prr += rv[c] * rv[c];
+            }
+            if constexpr (MIXED) {
+                float b[3] = {(float)rv[0], (float)rv[1], (float)rv[2]}, x[3];
+                block3_apply(a.Dinv32 + 9L * (row0 + i), b, x);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    sh.b[3 * i + c] = b[c];
+                    xr[3 * (row0 + i) + c] = a.wsm * x[c];
+                }
+            } else {
+                double zz[3];
+                block3_apply(a.Dinv + 9L * (row0 + i), rv, zz);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    zr[3 * (row0 + i) + c] = zz[c];
+                    prz += rv[c] * zz[c];
+                }
+            }
+        }
+        if constexpr (MIXED) spread(xr);
+        else spread(zr);
+        send(1, a.spc, prr, prz);
+        cluster_sync();
+        rr = inbox(1, 0);
+        rzp = rz;
+        ++k;
+        if constexpr (MIXED) {
+            if (rr <= a.tol2) {
+                leave(OFEA_OK, 1);
+                return;
+            }
+            vcycle();
+        } else {
+            rz = inbox(1, 1);
+        }
+    }
+    leave(OFEA_OK, 0);
+}
+
 // ------------------------------------------------------------------- host --
+
+namespace {
+
+int cluster_smem(int nslice, bool mixed) {
+    const size_t whole = 3 * (size_t)kSlice * nslice;
+    return (int)(sizeof(ClShared) + whole * 8);  // z in FP64, or z and x in FP32
+}
+
+// The largest cluster of k_cluster_solve the device runs (16, 8 or none), asked
+// for once per device.
+int cluster_limit(int device) {
+    static std::mutex mu;
+    static std::map<int, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(device);
+    if (it != known.end()) return it->second;
+    int limit = 0;
+    for (int C : {16, 8}) {
+        bool ok = true;
+        for (const void *fn : {(const void *)k_cluster_solve<true>, (const void *)k_cluster_solve<false>}) {
+            const int smem = cluster_smem(C * kClSpc, true);
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cluster_smem(kClMax * kClSpc, true)) != cudaSuccess ||
+                (C > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+                ok = false;
+                break;
+            }
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = C;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(C);
+            cfg.blockDim = dim3(kClThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess || n < 1) {
+                ok = false;
+                break;
+            }
+        }
+        if (ok) {
+            limit = C;
+            break;
+        }
+        cudaGetLastError();
+    }
+    known[device] = limit;
+    return limit;
+}
+
+}  // namespace
 
 bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
     const int nslice = (c->nfree + kSlice - 1) / kSlice;
@@ -549,17 +987,14 @@ bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
     // repeated by every CTA); PCG64 with the stored K is the faster one at
     // every size measured (706k DOF 105 against 122 us).
     if (nslice < 1) return false;
-    if (mixed && (nslice > 3500 || c->coarse.m > kResMaxM)) return false;
-    p.spc = (nslice + c->num_sms - 1) / c->num_sms;
-    p.G = (nslice + p.spc - 1) / p.spc;
+    const int W = (int)std::max<long long>(1, c->sell_len / nslice);
     // warps per slice: the fewest serial steps over all rounds, a round's own
     // latency counted as two steps
-    const int W = (int)std::max<long long>(1, c->sell_len / nslice);
-    auto pick = [&](int units) {
+    auto pick = [&](int units, int warps) {
         int best = 1;
         long cost = -1;
-        for (int S = 1; S <= 32; ++S) {
-            const int ng = kResWarps / S, rounds = (p.spc + ng - 1) / ng;
+        for (int S = 1; S <= warps; ++S) {
+            const int ng = warps / S, rounds = (p.spc + ng - 1) / ng;
             const long t = (long)rounds * ((units + S - 1) / S + 2);
             if (cost < 0 || t < cost) {
                 cost = t;
@@ -568,8 +1003,22 @@ bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
         }
         return best;
     };
-    p.S64 = pick((W + 1) / 2);  // two slots in flight per step
-    p.S16 = pick((W + 1) / 2);
+    p.cluster = 0;
+    // one cluster up to 64 slices (6.1k DOF), where the two meet (6.1k DOF:
+    // PCG64 7.5 us, 7.9 on the grid; 7.9k DOF: 7.7 us on the grid)
+    const int limit = cluster_limit(c->device);
+    if (limit > 0 && nslice <= limit * kClSpc && (!mixed || c->coarse.m <= kClM)) {
+        int C = 1;
+        while (C < limit && C < nslice) C *= 2;
+        p.cluster = p.G = C;
+        p.spc = (nslice + C - 1) / C;
+        p.S64 = p.S16 = pick((W + 1) / 2, kClWarps);
+        return true;
+    }
+    if (mixed && (nslice > 3500 || c->coarse.m > kResMaxM)) return false;
+    p.spc = (nslice + c->num_sms - 1) / c->num_sms;
+    p.G = (nslice + p.spc - 1) / p.spc;
+    p.S64 = p.S16 = pick((W + 1) / 2, kResWarps);  // two slots in flight per step
     return true;
 }
 
@@ -616,6 +1065,22 @@ void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, const P
     a.tol2 = tol2;
     a.P = P;
     a.fl = fl;
+    if (p.cluster) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = p.cluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(p.cluster);
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = cluster_smem(a.nslice, mixed);
+        cfg.stream = c->stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        void *args[] = {(void *)&a};
+        OFEA_CUDA(cudaLaunchKernelExC(&cfg, mixed ? (const void *)k_cluster_solve<true> : (const void *)k_cluster_solve<false>, args));
+        return;
+    }
     w.bar.ensure(2);
     a.bar = reinterpret_cast<GridBar *>(w.bar.p);
     a.limit_ns = 5000000000ull;  // 5 s: far above any phase

@@ -8,8 +8,10 @@ namespace ofea {
 // Launch shape of the resident solver for one matrix: G CTAs of kResThreads
 // threads, CTA b owning the slices [b * spc, (b + 1) * spc); in a matrix
 // phase S warps share a slice (S64: FP64 slots, S16: pairs of BF16 slots).
+// cluster: the CTAs are one thread-block cluster of that size (small
+// matrices); 0: a cooperative grid.
 struct ResidentPlan {
-    int G = 0, spc = 0, S64 = 1, S16 = 1;
+    int G = 0, spc = 0, S64 = 1, S16 = 1, cluster = 0;
 };
 
 constexpr int kResThreads = 1024;

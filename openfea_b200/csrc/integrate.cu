@@ -1073,6 +1073,7 @@ void assemble_linear(ofea_ctx *c) {
         gather(c, false, nullptr);
     }
     c->K_linear = true;
+    ++c->K_gen;
 }
 
 void assemble_nl(ofea_ctx *c, const double *d_u, double *d_fint) {

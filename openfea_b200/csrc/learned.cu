@@ -1174,13 +1174,20 @@ void learned_gradient(ofea_ctx *c, const float *h_x, int B, double *loss, float 
 // pass over the fine vector serve both levels (Z1 = Z2 P): c1 = P^T c2, and
 // the level-1 correction joins the stage's output in level-2 modes.
 void learned_coarse_correct(ofea_ctx *c, const float *t, float *x) {
+    restrict_level(c, c->coarse2, t, c->coarse2.cvec.p);
+    learned_coarse_solve(c);
+    prolong_level(c, c->coarse2, c->coarse2.cvec.p, x);
+}
+
+// coarse2.cvec: the restricted residual -> the correction in the nested
+// level's modes.
+void learned_coarse_solve(ofea_ctx *c) {
     Coarse &C1 = c->coarse;
     Coarse &C2 = c->coarse2;
     Learned &N = c->learned;
     const Learned::Layout L = Learned::layout();
     cudaStream_t s = c->stream;
     const int na = C2.na;
-    restrict_level(c, C2, t, C2.cvec.p);
     k_restrict_parent<<<grid_for(c, 6L * C1.na, 128), 128, 0, s>>>(C1.na, N.children.p, N.pdel.p, C2.cvec.p,
                                                                  C1.cvec.p, c->vc_stop);
     coarse_gemv(c, C1.cvec.p, C1.evec.p);
@@ -1194,7 +1201,6 @@ void learned_coarse_correct(ofea_ctx *c, const float *t, float *x) {
     apply_M_rest(c, na, coef, wv);
     k_poly_out_e1<<<grid_for(c, 6L * na, kBlock), kBlock, 0, s>>>(na, N.scale.p, wv, N.dsq.p, N.parent.p,
                                                                    N.pdel.p, C1.evec.p, C2.cvec.p, c->vc_stop);
-    prolong_level(c, C2, C2.cvec.p, x);
     OFEA_CHECK_LAUNCH();
 }
 

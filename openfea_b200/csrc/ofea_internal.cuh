@@ -161,6 +161,15 @@ struct Coarse {
     int nbw = 0, ldf = 0;  // block half-bandwidth; row stride of F (m rounded up to 4)
     DevBuf<double> Sb, Lb;
     DevBuf<float> F32, zvec;
+    // K Z of the level (precond.cu): entries (row, aggregate) grouped by
+    // aggregate, aggregate J's at md_ptr[J], 18 planes of md_n values; and the
+    // same in row order, row r's at md_rptr[r] (entry e at md_rpos[e]).
+    // md_state 0: not built, 1: built for the pattern, -1: no memory for it;
+    // md_gen: the assembly whose values md_val holds.
+    DevBuf<int> md_ptr, md_row, md_agg, md_rptr, md_rpos, md_ragg;
+    DevBuf<float> md_val, md_rval;
+    int md_state = 0, md_n = 0;
+    long md_gen = -1;
     std::vector<int> agg_cell_h, cell_agg_h;  // host copies (nesting of the learned level)
     std::vector<double> centroid_h;
 };
@@ -241,6 +250,7 @@ struct ofea_ctx {
     // stiffness of the mesh as it is on the device; the tables are per
     // pattern; mf_fe: the element forces
     bool K_linear = false;
+    long K_gen = 0;  // counts the assemblies
     ofea::DevBuf<int> mf_list, mf_rows;
     ofea::DevBuf<unsigned char> mf_link;
     ofea::DevBuf<double> mf_fe;
@@ -309,6 +319,7 @@ void geometry_start(ofea_ctx *c);
 void geometry_join(ofea_ctx *c);
 void setup_learned_solver(ofea_ctx *c);
 void learned_coarse_correct(ofea_ctx *c, const float *t, float *x);
+void learned_coarse_solve(ofea_ctx *c);
 // Batched persistent solver (batched.cu).
 ofea_batch *batch_create(ofea_ctx *const *ctxs, int nv, int nrhs);
 void batch_destroy(ofea_batch *b);

@@ -335,6 +335,7 @@ void build_pattern(ofea_ctx *c) {
     c->sell_layout_ok = false;
     c->se_state = 0;
     c->mf_state = 0;
+    c->coarse.md_state = c->coarse2.md_state = 0;
     c->K_linear = false;
     c->coarse.K_ok = false;  // the coarse geometry depends on the mesh alone: it stays
     c->coarse2.K_ok = false;

@@ -255,6 +255,7 @@ static void bin_nodes(ofea_ctx *c, Coarse &C, const int nc[3], const double lo[3
     C.agg_cell_h = std::move(agg_cell3);
     C.cell_agg_h = std::move(cell_agg);
     C.centroid_h = std::move(cen);
+    C.md_state = 0;
     C.geom_ok = true;  // K_ok is false already: every change of the geometry resets it first
 }
 
@@ -1293,6 +1294,7 @@ static void release_geometry(Coarse &C) {
     C.agg_off.release();
     C.row_off.release();
     C.row_cell.release();
+    C.md_state = 0;
     C.geom_ok = C.K_ok = false;
 }
 
@@ -1392,6 +1394,210 @@ void setup_coarse(ofea_ctx *c, int target_nodes) {
     coarse_finish(c);
 }
 
+// ----------------------------------------------------- K times the modes --
+//
+// With S the smoother, x0 = S b, the V-cycle is
+//     c = Z^T (b - K x0),  e = E^-1 c,  z = x0 + Z e + S (b - K x0 - K Z e).
+// K is symmetric, so Z^T K x0 = (K Z)^T x0, and K Z is sparse: K annihilates the
+// rigid motions of everything a row couples to, so a row whose columns all lie
+// in its own aggregate, away from fixed nodes, has K Z = 0.  Only the other rows
+// have entries, a 3 x 6 block per (row, aggregate among its columns), 0.3 to
+// 1.8 per row on the average.  With K Z at hand (rounded to FP32 from the FP64
+// K once) a cycle takes one product with the smoother's BF16 K, K x0, instead
+// of two: M = 2 S - S K S + (Z - S K Z) E^-1 (Z - S K Z)^T stays symmetric
+// whatever K x0 is rounded to, and no pass writes x0 + Z e: at 1.56M DOF
+// restriction 17 us and post-smoothing 79 against 61 + 7 + 5 + 62 us.  (Taking K Z in the
+// restriction alone leaves the two halves apart by that rounding: 129
+// iterations instead of 113 at 1.5k DOF.)
+//
+// Which rows have entries is known from the mesh for the linear stiffness
+// only; other matrices (a tangent annihilates rotations of the deformed shape
+// alone; a matrix without elements) restrict the residual.
+
+// Per row the slots of its columns' aggregates (bit of the 27 neighbour cells);
+// 0 for a row without entries.
+__global__ void k_row_slots(int nfree, const int *__restrict__ rowptr, const int *__restrict__ cols,
+                            const unsigned long long *__restrict__ row_cell, const int *__restrict__ node_of_free,
+                            const int *__restrict__ inc_ptr, const int *__restrict__ inc, int ne8,
+                            const int *__restrict__ topo8, const int *__restrict__ topo4, const int *__restrict__ free_map,
+                            unsigned *__restrict__ slots) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nfree; r += gridDim.x * blockDim.x) {
+        const unsigned long long p0 = row_cell[r];
+        const int x0 = (int)(p0 & kCellMask), y0 = (int)((p0 >> kCellBits) & kCellMask), z0 = (int)(p0 >> (2 * kCellBits));
+        unsigned m = 0;
+        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
+            const unsigned long long p = row_cell[cols[k]];
+            const int dx = (int)(p & kCellMask) - x0, dy = (int)((p >> kCellBits) & kCellMask) - y0,
+                      dz = (int)(p >> (2 * kCellBits)) - z0;
+            m |= 1u << ((dx + 1) * 9 + (dy + 1) * 3 + (dz + 1));  // within 1 of each other: the set-up has checked
+        }
+        if (__popc(m) == 1) {
+            bool fixed = false;
+            const int node = node_of_free[r];
+            for (int t = inc_ptr[node]; t < inc_ptr[node + 1] && !fixed; ++t) {
+                const int g = inc[t] >> 3;
+                const int *n = g < ne8 ? topo8 + 8L * g : topo4 + 4L * (g - ne8);
+                for (int a = 0; a < (g < ne8 ? 8 : 4); ++a) fixed |= free_map[n[a]] < 0;
+            }
+            if (!fixed) m = 0;
+        }
+        slots[r] = m;
+    }
+}
+
+// Entries of aggregate J, one CTA: the rows of J and its 27 neighbours (in
+// slot, then aggregate order) that have J among their slots.  count (row null)
+// or write.
+__global__ void __launch_bounds__(kBlock) k_mode_entries(int na, const int *__restrict__ agg_ptr, const int *__restrict__ agg_nodes,
+                                                         const int *__restrict__ nbr, const unsigned *__restrict__ slots,
+                                                         int *__restrict__ cnt, const int *__restrict__ ptr,
+                                                         int *__restrict__ row, int *__restrict__ agg) {
+    __shared__ int wsum[kWarpsPerBlock];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int J = blockIdx.x; J < na; J += gridDim.x) {
+        int at = row ? ptr[J] : 0;
+        for (int sl = 0; sl < 27; ++sl) {
+            const int I = nbr[27L * J + sl];
+            if (I < 0) continue;
+            for (int b = agg_ptr[I]; b < agg_ptr[I + 1]; b += kBlock) {
+                const int idx = b + threadIdx.x;
+                const int r = idx < agg_ptr[I + 1] ? agg_nodes[idx] : -1;
+                const bool has = r >= 0 && (slots[r] >> (26 - sl) & 1u);  // J as seen from I
+                const unsigned m = __ballot_sync(0xffffffffu, has);
+                if (lane == 0) wsum[w] = __popc(m);
+                __syncthreads();
+                int off = at, tot = 0;
+                for (int q = 0; q < kWarpsPerBlock; ++q) {
+                    if (q < w) off += wsum[q];
+                    tot += wsum[q];
+                }
+                if (has && row) {
+                    const int e = off + __popc(m & ((1u << lane) - 1));
+                    row[e] = r;
+                    agg[e] = J;
+                }
+                at += tot;
+                __syncthreads();
+            }
+        }
+        if (!row && threadIdx.x == 0) cnt[J] = at;
+    }
+}
+
+// Values of the entries: (K Z_J)_r, a thread per entry over the row's blocks
+// in J.
+__global__ void __launch_bounds__(kBlock) k_mode_values(int n, const int *__restrict__ row, const int *__restrict__ agg,
+                                                        const int *__restrict__ rowptr, const int *__restrict__ cols,
+                                                        const float4 *__restrict__ row_off, KBlocks KB,
+                                                        const int *__restrict__ rpos, float *__restrict__ val,
+                                                        float *__restrict__ rval) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int r = row[e], J = agg[e], rb = rowptr[r], deg = rowptr[r + 1] - rb;
+        double W[18];
+#pragma unroll
+        for (int q = 0; q < 18; ++q) W[q] = 0.0;
+        for (int k = 0; k < deg; ++k) {
+            const float4 oj = row_off[cols[rb + k]];
+            if (__float_as_int(oj.w) != J) continue;
+            const double d[3] = {oj.x, oj.y, oj.z};
+            double K[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) K[q] = KB.at(r, k, q);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                for (int l = 0; l < 3; ++l) W[6 * i + l] += K[3 * i + l];
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    double z[3];
+                    cross_e(t, d, z);
+                    W[6 * i + 3 + t] += K[3 * i] * z[0] + K[3 * i + 1] * z[1] + K[3 * i + 2] * z[2];
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 18; ++q) {
+            val[(long)q * n + e] = (float)W[q];
+            rval[(long)q * n + rpos[e]] = (float)W[q];
+        }
+    }
+}
+
+// The entries in row order, a row's in slot order: entry e goes where its
+// aggregate's slot ranks among the row's.
+__global__ void k_row_counts(int nfree, const unsigned *__restrict__ slots, int *__restrict__ cnt) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nfree; r += gridDim.x * blockDim.x) cnt[r] = __popc(slots[r]);
+}
+__global__ void k_row_entries(int n, const int *__restrict__ row, const int *__restrict__ agg,
+                              const unsigned long long *__restrict__ row_cell, const int *__restrict__ agg_cell,
+                              const unsigned *__restrict__ slots, const int *__restrict__ rptr, int *__restrict__ rpos,
+                              int *__restrict__ ragg) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int r = row[e], J = agg[e];
+        const unsigned long long p = row_cell[r];
+        const int dx = agg_cell[3 * J] - (int)(p & kCellMask), dy = agg_cell[3 * J + 1] - (int)((p >> kCellBits) & kCellMask),
+                  dz = agg_cell[3 * J + 2] - (int)(p >> (2 * kCellBits));
+        const int sl = (dx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
+        const int at = rptr[r] + __popc(slots[r] & ((1u << sl) - 1));
+        rpos[e] = at;
+        ragg[at] = J;
+    }
+}
+
+bool ensure_modes(ofea_ctx *c, Coarse &C) {
+    if (!c->K_linear || c->matrix_only || C.md_state < 0) return false;
+    cudaStream_t s = c->stream;
+    try {
+        if (C.md_state == 0) {
+            DevBuf<unsigned> slots;
+            slots.ensure(c->nfree);
+            k_row_slots<<<grid_for(c, c->nfree, kBlock), kBlock, 0, s>>>(
+                c->nfree, c->rowptr.p, c->cols.p, C.row_cell.p, c->node_of_free.p, c->inc_ptr.p, c->inc.p, c->ne8, c->topo8.p,
+                c->topo4.p, c->free_map.p, slots.p);
+            const int most = std::max(C.na, c->nfree), tmp_len = most / 1024 + 4;
+            c->scratch_i.ensure((size_t)most + 1 + tmp_len);
+            C.md_ptr.ensure((size_t)C.na + 1);
+            const int g = std::min(C.na, c->num_sms * 16);
+            k_mode_entries<<<g, kBlock, 0, s>>>(C.na, C.agg_ptr.p, C.agg_nodes.p, C.nbr.p, slots.p, c->scratch_i.p, nullptr,
+                                                nullptr, nullptr);
+            OFEA_CHECK_LAUNCH();
+            C.md_n = (int)exclusive_scan(c->scratch_i.p, C.md_ptr.p, C.na, s, c->scratch_i.p + most + 1, tmp_len);
+            C.md_row.ensure(std::max(C.md_n, 1));
+            C.md_agg.ensure(std::max(C.md_n, 1));
+            C.md_val.ensure(18 * (size_t)std::max(C.md_n, 1));
+            k_mode_entries<<<g, kBlock, 0, s>>>(C.na, C.agg_ptr.p, C.agg_nodes.p, C.nbr.p, slots.p, nullptr, C.md_ptr.p,
+                                                C.md_row.p, C.md_agg.p);
+            C.md_rptr.ensure((size_t)c->nfree + 1);
+            C.md_rpos.ensure(std::max(C.md_n, 1));
+            C.md_ragg.ensure(std::max(C.md_n, 1));
+            C.md_rval.ensure(18 * (size_t)std::max(C.md_n, 1));
+            k_row_counts<<<grid_for(c, c->nfree, kBlock), kBlock, 0, s>>>(c->nfree, slots.p, c->scratch_i.p);
+            OFEA_CHECK_LAUNCH();
+            exclusive_scan(c->scratch_i.p, C.md_rptr.p, c->nfree, s, c->scratch_i.p + most + 1, tmp_len);
+            k_row_entries<<<grid_for(c, C.md_n, kBlock), kBlock, 0, s>>>(C.md_n, C.md_row.p, C.md_agg.p, C.row_cell.p,
+                                                                        C.agg_cell.p, slots.p, C.md_rptr.p, C.md_rpos.p,
+                                                                        C.md_ragg.p);
+            OFEA_CHECK_LAUNCH();
+            OFEA_CUDA(cudaStreamSynchronize(s));  // before slots is released
+            C.md_state = 1;
+            C.md_gen = -1;
+        }
+    } catch (const Failure &f) {
+        if (f.code != OFEA_ERR_OOM) throw;
+        C.md_state = -1;
+        return false;
+    }
+    if (C.md_gen != c->K_gen) {
+        k_mode_values<<<grid_for(c, C.md_n, kBlock), kBlock, 0, s>>>(C.md_n, C.md_row.p, C.md_agg.p, c->rowptr.p, c->cols.p,
+                                                                    reinterpret_cast<const float4 *>(C.row_off.p), kblocks(c),
+                                                                    C.md_rpos.p, C.md_val.p, C.md_rval.p);
+        OFEA_CHECK_LAUNCH();
+        setup_mark(c, "modes");
+        C.md_gen = c->K_gen;
+    }
+    return true;
+}
+
 // ---------------------------------------------------------- V-cycle kernels --
 
 // t = b - K32 x (x complete), per row.
@@ -1450,6 +1656,38 @@ __global__ void __launch_bounds__(NT) k_restrict(int na, const int *__restrict__
     }
 }
 
+// cvec_J = Z_J^T b - (K Z_J)^T x: k_restrict's sums over the aggregate's rows
+// of b, then over its entries.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_restrict_modes(int na, const int *__restrict__ agg_ptr, const float4 *__restrict__ off,
+                                                       const int *__restrict__ md_ptr, const int *__restrict__ md_row,
+                                                       const float *__restrict__ md_val, long md_n,
+                                                       const float *__restrict__ b, const float *__restrict__ x,
+                                                       float *__restrict__ cvec, const int *__restrict__ stop) {
+    constexpr int NW = NT / 32;
+    __shared__ float sh[6][NW];
+    if (vc_stopped(stop)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int I = blockIdx.x; I < na; I += gridDim.x) {
+        float a[6] = {0, 0, 0, 0, 0, 0};
+        modes_sum(agg_ptr[I] + threadIdx.x, agg_ptr[I + 1], NT, off, b, a);
+        entries_sum(md_ptr[I] + threadIdx.x, md_ptr[I + 1], NT, md_row, md_val, md_n, x, a);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            a[k] = warp_sum(a[k]);
+            if (lane == 0) sh[k][w] = a[k];
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            float v = 0.f;
+#pragma unroll
+            for (int q = 0; q < NW; ++q) v += sh[threadIdx.x][q];
+            cvec[6 * I + threadIdx.x] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // e = Einv32 c: one warp per row.
 __global__ void __launch_bounds__(kBlock) k_coarse_gemv(int m, const float *__restrict__ Ainv,
                                                         const float *__restrict__ cvec,
@@ -1489,6 +1727,18 @@ void restrict_level(ofea_ctx *c, const Coarse &C, const float *t, float *cvec) {
         k_restrict<128><<<g, 128, 0, c->stream>>>(C.na, C.agg_ptr.p, off, t, cvec, c->vc_stop);
     else
         k_restrict<256><<<g, 256, 0, c->stream>>>(C.na, C.agg_ptr.p, off, t, cvec, c->vc_stop);
+    OFEA_CHECK_LAUNCH();
+}
+
+void restrict_modes(ofea_ctx *c, const Coarse &C, const float *b, const float *x, float *cvec) {
+    const int g = std::min(C.na, c->num_sms * 16);
+    const float4 *off = reinterpret_cast<const float4 *>(C.agg_off.p);
+    if (C.max_agg <= 512)
+        k_restrict_modes<128><<<g, 128, 0, c->stream>>>(C.na, C.agg_ptr.p, off, C.md_ptr.p, C.md_row.p, C.md_val.p, C.md_n, b, x,
+                                                        cvec, c->vc_stop);
+    else
+        k_restrict_modes<256><<<g, 256, 0, c->stream>>>(C.na, C.agg_ptr.p, off, C.md_ptr.p, C.md_row.p, C.md_val.p, C.md_n, b, x,
+                                                        cvec, c->vc_stop);
     OFEA_CHECK_LAUNCH();
 }
 

@@ -16,6 +16,80 @@ __device__ __forceinline__ bool vc_stopped(const int *stop) {
     return s_stop != 0;
 }
 
+// Z_I^T v over the rows [idx, end) of an aggregate in steps, added to a: off
+// gives each row's offset from the centroid and the row.
+__device__ __forceinline__ void modes_sum(int idx, int end, int step, const float4 *__restrict__ off, const float *v,
+                                          float (&a)[6]) {
+    for (; idx < end; idx += step) {
+        const float4 o = __ldg(off + idx);
+        const int r = __float_as_int(o.w);
+        const float dx = o.x, dy = o.y, dz = o.z;
+        const float tx = v[3L * r], ty = v[3L * r + 1], tz = v[3L * r + 2];
+        a[0] += tx;
+        a[1] += ty;
+        a[2] += tz;
+        a[3] += -dz * ty + dy * tz;  // (e_x x d) . t
+        a[4] += dz * tx - dx * tz;   // (e_y x d) . t
+        a[5] += -dy * tx + dx * ty;  // (e_z x d) . t
+    }
+}
+// K Z as the row kernels read it: entries in row order.
+struct RowModes {
+    const float4 *off;  // a row's offset from its aggregate's centroid, the aggregate
+    const int *rptr, *agg;
+    const float *val;
+    long n;
+    // (Z e)_r for e of six values per aggregate
+    __device__ __forceinline__ void modes(int r, const float *e, float (&z)[3]) const {
+        const float4 o = __ldg(off + r);
+        const float *q = e + 6 * __float_as_int(o.w);
+        z[0] = q[0] + o.z * q[4] - o.y * q[5];
+        z[1] = q[1] - o.z * q[3] + o.x * q[5];
+        z[2] = q[2] + o.y * q[3] - o.x * q[4];
+    }
+    // entry t's part of K Z e
+    __device__ __forceinline__ void entry(int t, const float *e, float (&kz)[3]) const {
+        const float *v = e + 6 * __ldg(agg + t);
+        float W[18];
+#pragma unroll
+        for (int q = 0; q < 18; ++q) W[q] = __ldg(val + q * n + t);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            kz[c] = W[6 * c] * v[0];
+#pragma unroll
+            for (int l = 1; l < 6; ++l) kz[c] = fmaf(W[6 * c + l], v[l], kz[c]);
+        }
+    }
+    // (K Z e)_r
+    __device__ __forceinline__ void row(int r, const float *e, float (&kz)[3]) const {
+        kz[0] = kz[1] = kz[2] = 0.f;
+        for (int t = __ldg(rptr + r); t < __ldg(rptr + r + 1); ++t) {
+            float k[3];
+            entry(t, e, k);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) kz[c] += k[c];
+        }
+    }
+};
+inline RowModes row_modes(const Coarse &C) {
+    return {reinterpret_cast<const float4 *>(C.row_off.p), C.md_rptr.p, C.md_ragg.p, C.md_rval.p, C.md_n};
+}
+// One entry of K Z: a -= W^T x.
+__device__ __forceinline__ void entry_sub(long e, long n, const float *__restrict__ val, float x, float y, float z, float (&a)[6]) {
+    float W[18];
+#pragma unroll
+    for (int q = 0; q < 18; ++q) W[q] = __ldg(val + q * n + e);
+#pragma unroll
+    for (int l = 0; l < 6; ++l) a[l] -= fmaf(W[l], x, fmaf(W[6 + l], y, W[12 + l] * z));
+}
+__device__ __forceinline__ void entries_sum(int e, int end, int step, const int *__restrict__ row, const float *__restrict__ val,
+                                            long n, const float *x, float (&a)[6]) {
+    for (; e < end; e += step) {
+        const long r = 3L * __ldg(row + e);
+        entry_sub(e, n, val, x[r], x[r + 1], x[r + 2], a);
+    }
+}
+
 void build_aggregation(ofea_ctx *c, int target_nodes);
 void build_aggregation_fine(ofea_ctx *c);
 // Aggregation (once per mesh), E = Z^T K Z, its inverse and lambda_max(D^-1 K)
@@ -44,6 +118,12 @@ void coarse_dense_inverse(ofea_ctx *c);
 void coarse_correct(ofea_ctx *c, const float *t, float *x);
 // t = b - K32 x
 void vc_resid(ofea_ctx *c, const float *b, const float *x, float *t);
+// K Z of a level, current for K: the restriction c = Z^T b - (K Z)^T x
+// (restrict_modes) and the post-smoothing's K Z e take the place of a product
+// with K.  False where the residual is formed instead (K not the linear
+// stiffness of a mesh, or no memory for it).
+bool ensure_modes(ofea_ctx *c, Coarse &C);
+void restrict_modes(ofea_ctx *c, const Coarse &C, const float *b, const float *x, float *cvec);
 // Level-generic pieces (also used by the learned level):
 // cvec = Z^T t, x += Z g, and the Galerkin blocks of Z^T K Z into C.part
 // ([aggregate][chunk][27 neighbour slots][6 x 6], chunks summed by the caller).

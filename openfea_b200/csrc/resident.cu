@@ -26,7 +26,8 @@
 //
 // Per iteration, launch-per-phase kernels before, this after (B200): PCG64
 // 27.9 -> 7.6 us at 1.5k DOF, 28.7 -> 9.3 at 46k, 58.0 -> 18.4 at 139k; MIXED
-// 62 -> 19.5, 66 -> 24.9, 111 -> 54 and 132 -> 98 us (288k).  What is left at
+// 67 -> 17.8 (14.5k), 66 -> 21.6, 111 -> 46.5 and 132 -> 85 us (288k); without
+// K Z 22.1, 24.9, 54 and 98.  What is left at
 // the small end is the barriers: 2,600 to 2,900 cycles each, 2,000 more to
 // drain a phase's stores, and 800 for the first load after.  Sums of a phase are
 // taken under the next product where nothing needs them earlier, a CTA's own
@@ -59,6 +60,9 @@ struct RArgs {
     const float *Dinv32, *Einv;
     const int *agg_ptr;
     const float4 *agg_off, *row_off;
+    const int *md_ptr, *md_row;  // K Z by aggregate (null: the residual is restricted)
+    const float *md_val;
+    RowModes md;                 // K Z by row
     double *u, *r, *q, *p0, *p1, *z;
     float *zA, *zB, *b32, *x32, *t32, *cvec;
     float wsm;
@@ -170,6 +174,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     __shared__ double s_w[2][kResWarps], s_sum[4];
     __shared__ float s_e[MIXED ? kResMaxM : 1];
     __shared__ unsigned s_touch[MIXED ? kResMaxM / 6 / 32 : 1];
+    __shared__ uint16_t s_list[MIXED ? kResMaxM / 6 : 1];
+    __shared__ int s_ntouch;
     __shared__ int s_fail, s_k, s_done;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int G = gridDim.x;
@@ -186,10 +192,25 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     __syncthreads();
     if (s_done) return;
     int k = s_k;
-    if (MIXED) {  // the aggregates of this CTA's rows
+    if (MIXED) {  // the aggregates of this CTA's rows and of their entries
         for (int r = row0 + tid; r < row1; r += kResThreads) {
             const int I = __float_as_int(__ldg(&a.row_off[r].w));
             atomicOr(&s_touch[I >> 5], 1u << (I & 31));
+            if (a.md_ptr)
+                for (int t = __ldg(a.md.rptr + r); t < __ldg(a.md.rptr + r + 1); ++t) {
+                    const int J = __ldg(a.md.agg + t);
+                    atomicOr(&s_touch[J >> 5], 1u << (J & 31));
+                }
+        }
+        __syncthreads();
+        if (w == 0) {  // as a list, ascending
+            int at = 0;
+            for (int i = 0; i < (a.na + 31) / 32; ++i) {
+                const unsigned m = s_touch[i];
+                if (m >> lane & 1u) s_list[at + __popc(m & ((1u << lane) - 1))] = (uint16_t)(32 * i + lane);
+                at += __popc(m);
+            }
+            if (lane == 0) s_ntouch = at;
         }
     }
     // this warp's slices of the first round
@@ -318,6 +339,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
     // 0, 1: stopped, 2: a wait ran out.
     auto vcycle = [&](int kk, bool check) -> int {
         if (check && w == kResWarps - 1) sum(0, a.P.rr);
+        // t = b - K x; with K Z, beside the restriction (the post-smoothing's
+        // residual), else before it
         if (spmm16(a.x32, [&](int row) { return f3(a.b32, row); }, [&] { return check && s_sum[0] <= a.tol2; },
                    [&](int row, float (&y)[3], const F3 &b) {
 #pragma unroll
@@ -326,23 +349,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
             stop(OFEA_OK, kk + 1);
             return 1;
         }
-        if (!sync()) return 2;
-        {  // c = Z^T t, one CTA per aggregate
+        if (a.md_ptr) __syncthreads();  // s_red is read
+        else if (!sync()) return 2;
+        {  // c = Z^T t, or Z^T b - (K Z)^T x, one CTA per aggregate
             float *sh = reinterpret_cast<float *>(s_red);  // [6][warps]
             for (int I = blockIdx.x; I < a.na; I += G) {
                 float acc[6] = {0, 0, 0, 0, 0, 0};
-                for (int idx = __ldg(a.agg_ptr + I) + tid; idx < __ldg(a.agg_ptr + I + 1); idx += kResThreads) {
-                    const float4 o = __ldg(a.agg_off + idx);
-                    const int r = __float_as_int(o.w);
-                    const float dx = o.x, dy = o.y, dz = o.z;
-                    const float tx = a.t32[3L * r], ty = a.t32[3L * r + 1], tz = a.t32[3L * r + 2];
-                    acc[0] += tx;
-                    acc[1] += ty;
-                    acc[2] += tz;
-                    acc[3] += -dz * ty + dy * tz;
-                    acc[4] += dz * tx - dx * tz;
-                    acc[5] += -dy * tx + dx * ty;
-                }
+                modes_sum(__ldg(a.agg_ptr + I) + tid, __ldg(a.agg_ptr + I + 1), kResThreads, a.agg_off,
+                          a.md_ptr ? a.b32 : a.t32, acc);
+                if (a.md_ptr)
+                    entries_sum(__ldg(a.md_ptr + I) + tid, __ldg(a.md_ptr + I + 1), kResThreads, a.md_row, a.md_val, a.md.n,
+                                a.x32, acc);
 #pragma unroll
                 for (int q = 0; q < 6; ++q) {
                     acc[q] = warp_sum(acc[q]);
@@ -358,24 +375,72 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
         }
         if (!sync()) return 2;
         // e = E^-1 c for the aggregates of this CTA's rows, x += Z e
-        for (int wd = 0, seen = 0; wd < (a.na + 31) / 32; ++wd) {
-            unsigned bits = s_touch[wd];
-            while (bits) {
-                const int I = wd * 32 + __ffs(bits) - 1;
-                bits &= bits - 1;
-#pragma unroll 1
-                for (int q = 0; q < 6; ++q, ++seen) {
-                    if (seen % kResWarps != w) continue;
-                    const float *row = a.Einv + (long)(6 * I + q) * a.m;
-                    float s = 0.f;
-#pragma unroll 4
-                    for (int j = lane; j < a.m; j += 32) s = fmaf(__ldg(row + j), a.cvec[j], s);
-                    s = warp_sum(s);
-                    if (lane == 0) s_e[6 * I + q] = s;
-                }
+        for (int i0 = w; i0 < 6 * s_ntouch; i0 += 4 * kResWarps) {  // four rows of E^-1 in flight per warp
+            int at[4];
+            const float *row[4];
+            float sm[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = min(i0 + u * kResWarps, 6 * s_ntouch - 1), t = i / 6;
+                at[u] = 6 * s_list[t] + (i - 6 * t);
+                row[u] = a.Einv + (long)at[u] * a.m;
+                sm[u] = 0.f;
+            }
+#pragma unroll 2
+            for (int j = lane; j < a.m; j += 32) {
+                const float cj = a.cvec[j];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) sm[u] = fmaf(__ldg(row[u] + j), cj, sm[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                sm[u] = warp_sum(sm[u]);
+                if (lane == 0) s_e[at[u]] = sm[u];
             }
         }
         __syncthreads();
+        float *znew = ((kk + 1) & 1) ? a.zB : a.zA;
+        const float *zold = ((kk + 1) & 1) ? a.zA : a.zB;
+        double prz = 0.0, przo = 0.0;
+        if (a.md_ptr) {  // z = x0 + Z e + w Dinv32 (t - K Z e): own rows only
+            // the own entries' parts first, a thread per entry
+            float *part = reinterpret_cast<float *>(s_red);
+            const int e0 = __ldg(a.md.rptr + row0), ne = __ldg(a.md.rptr + row1) - e0;
+            const bool staged = 3 * ne <= 2 * (int)(sizeof(s_red) / sizeof(double));
+            if (staged)
+                for (int t = tid; t < ne; t += kResThreads) {
+                    float k[3];
+                    a.md.entry(e0 + t, s_e, k);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) part[3 * t + c] = k[c];
+                }
+            __syncthreads();
+            for (int r = row0 + tid; r < row1; r += kResThreads) {
+                float ze[3], kz[3] = {0.f, 0.f, 0.f}, d[3], o[3];
+                a.md.modes(r, s_e, ze);
+                if (staged) {
+                    for (int t = __ldg(a.md.rptr + r) - e0; t < __ldg(a.md.rptr + r + 1) - e0; ++t)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) kz[c] += part[3 * t + c];
+                } else {
+                    a.md.row(r, s_e, kz);
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) d[i] = a.t32[3L * r + i] - kz[i];
+                block3_apply(a.Dinv32 + 9L * r, d, o);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const long dd = 3L * r + i;
+                    const float zn = fmaf(a.wsm, o[i], a.x32[dd] + ze[i]);
+                    const double rv = a.r[dd];
+                    prz += rv * (double)zn;
+                    przo += rv * (double)zold[dd];
+                    znew[dd] = zn;
+                }
+            }
+            put(prz, ((kk + 1) & 1) ? a.P.rz1 : a.P.rz0, przo, a.P.rzo);
+            return sync() ? 0 : 2;
+        }
         for (int r = row0 + tid; r < row1; r += kResThreads) {
             const float4 o = __ldg(a.row_off + r);
             const float *e = s_e + 6 * __float_as_int(o.w);
@@ -385,9 +450,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
             a.x32[3L * r + 2] += e[2] + dy * e[3] - dx * e[4];
         }
         if (!sync()) return 2;
-        float *znew = ((kk + 1) & 1) ? a.zB : a.zA;
-        const float *zold = ((kk + 1) & 1) ? a.zA : a.zB;
-        double prz = 0.0, przo = 0.0;
         struct Own {
             F3 b, x, z;
             double r[3];
@@ -555,7 +617,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const RArgs a) {
 // are read through L1.  The coarse level: every CTA restricts its own rows, the
 // partial c of all CTAs are summed by each, and e = E^-1 c and x += Z e are
 // formed by every CTA for its whole copy of x, so the coarse correction costs
-// one barrier.  Barriers per iteration: PCG64 2, MIXED 4.
+// one barrier, or none with K Z (c's parts travel with ||r||^2).  Barriers per
+// iteration: PCG64 2, MIXED 3 (4 without K Z).
 //
 // The sums of a phase go to an inbox of their own; an inbox, and a whole
 // vector, is written again only after a barrier that follows its last reading.
@@ -775,19 +838,16 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
         cluster_sync();  // no CTA leaves while another may write into it
     };
     // z = M(b), from the pre-smoothed x in every CTA; sums r.z, r.z_old
-    auto vcycle = [&]() {
+    // own rows' part of c = Z^T t, or of Z^T b - (K Z)^T x, a warp per aggregate
+    auto restrict_own = [&]() {
         if constexpr (MIXED) {
-            spmm(std::true_type{}, (const float *)xr, [&](int i, float (&y)[3]) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) sh.t[3 * i + c] = sh.b[3 * i + c] - y[c];
-            });
-            // own rows' part of c = Z^T t, a warp per aggregate
+            const float *v = a.md_ptr ? sh.b : sh.t;
             for (int I = w; I < a.na; I += kClWarps) {
                 float acc[6] = {0, 0, 0, 0, 0, 0};
                 for (int i = lane; i < row1 - row0; i += 32) {
                     const float4 o = __ldg(a.row_off + row0 + i);
                     if (__float_as_int(o.w) != I) continue;
-                    const float tx = sh.t[3 * i], ty = sh.t[3 * i + 1], tz = sh.t[3 * i + 2];
+                    const float tx = v[3 * i], ty = v[3 * i + 1], tz = v[3 * i + 2];
                     acc[0] += tx;
                     acc[1] += ty;
                     acc[2] += tz;
@@ -795,6 +855,11 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
                     acc[4] += o.z * tx - o.x * tz;
                     acc[5] += -o.y * tx + o.x * ty;
                 }
+                if (a.md_ptr)
+                    for (int e = __ldg(a.md_ptr + I) + lane; e < __ldg(a.md_ptr + I + 1); e += 32) {
+                        const int r = __ldg(a.md_row + e);
+                        if (r >= row0 && r < row1) entry_sub(e, a.md.n, a.md_val, xr[3 * r], xr[3 * r + 1], xr[3 * r + 2], acc);
+                    }
 #pragma unroll
                 for (int q = 0; q < 6; ++q) acc[q] = warp_sum(acc[q]);
                 if (lane < C)
@@ -802,7 +867,19 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
                     for (int q = 0; q < 6; ++q) peer_st(peer(&sh.cin[rank][6 * I + q], lane), acc[q]);
             }
             peer_done();
-            cluster_sync();
+        }
+    };
+    // with K Z, c's parts are already here (restrict_own before the barrier)
+    auto vcycle = [&]() {
+        if constexpr (MIXED) {
+            if (!a.md_ptr) {
+                spmm(std::true_type{}, (const float *)xr, [&](int i, float (&y)[3]) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) sh.t[3 * i + c] = sh.b[3 * i + c] - y[c];
+                });
+                restrict_own();
+                cluster_sync();
+            }
             for (int i = tid; i < a.m; i += kClThreads) {
                 float s = 0.f;
                 for (int j = 0; j < C; ++j) s += sh.cin[j][i];
@@ -817,24 +894,34 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
                 if (lane == 0) sh.e[i] = s;
             }
             __syncthreads();
-            for (int r = tid; r < a.nfree; r += kClThreads) {
-                const float4 o = __ldg(a.row_off + r);
-                const float *e = sh.e + 6 * __float_as_int(o.w);
-                xr[3 * r] += e[0] + o.z * e[4] - o.y * e[5];
-                xr[3 * r + 1] += e[1] - o.z * e[3] + o.x * e[5];
-                xr[3 * r + 2] += e[2] + o.y * e[3] - o.x * e[4];
+            if (!a.md_ptr) {
+                for (int r = tid; r < a.nfree; r += kClThreads) {
+                    const float4 o = __ldg(a.row_off + r);
+                    const float *e = sh.e + 6 * __float_as_int(o.w);
+                    xr[3 * r] += e[0] + o.z * e[4] - o.y * e[5];
+                    xr[3 * r + 1] += e[1] - o.z * e[3] + o.x * e[5];
+                    xr[3 * r + 2] += e[2] + o.y * e[3] - o.x * e[4];
+                }
+                __syncthreads();
             }
-            __syncthreads();
             double prz = 0.0, przo = 0.0;
             spmm(std::true_type{}, (const float *)xr, [&](int i, float (&y)[3]) {
                 float d[3], o[3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) d[c] = sh.b[3 * i + c] - y[c];
+                float ze[3] = {0.f, 0.f, 0.f};
+                if (a.md_ptr) {
+                    float kz[3];
+                    a.md.modes(row0 + i, sh.e, ze);
+                    a.md.row(row0 + i, sh.e, kz);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) d[c] -= kz[c];
+                }
                 block3_apply(a.Dinv32 + 9L * (row0 + i), d, o);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const int g = 3 * (row0 + i) + c;
-                    const float zn = fmaf(a.wsm, o[c], xr[g]);
+                    const float zn = fmaf(a.wsm, o[c], xr[g] + ze[c]);
                     const double rv = sh.r[3 * i + c];
                     prz += rv * (double)zn;
                     przo += rv * (double)zr[g];
@@ -848,7 +935,13 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
             rzo = inbox(2, 1);
         }
     };
-    if (MIXED && a.first) vcycle();
+    if (MIXED && a.first) {
+        if (a.md_ptr) {
+            restrict_own();
+            cluster_sync();
+        }
+        vcycle();
+    }
     for (int it = 0; it < a.iters; ++it) {
         if (!MIXED && rr <= a.tol2) {
             leave(OFEA_OK, 1);
@@ -904,8 +997,12 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const RArgs a) 
                 }
             }
         }
-        if constexpr (MIXED) spread(xr);
-        else spread(zr);
+        if constexpr (MIXED) {
+            spread(xr);
+            if (a.md_ptr) restrict_own();
+        } else {
+            spread(zr);
+        }
         send(1, a.spc, prr, prz);
         cluster_sync();
         rr = inbox(1, 0);
@@ -982,9 +1079,9 @@ int cluster_limit(int device) {
 bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
     const int nslice = (c->nfree + kSlice - 1) / kSlice;
     // MIXED: up to 3,500 slices (336k DOF), beyond which the launch-per-phase
-    // kernels' wider grids win (288k DOF: 98 us per iteration here, 132
-    // there; 467k DOF: 191 here, 164 there, the coarse solve of 930 unknowns
-    // repeated by every CTA); PCG64 with the stored K is the faster one at
+    // kernels' wider grids win (288k DOF: 85 us per iteration here, 132
+    // there before; 467k DOF: 191 here, 164 there, both without K Z, the coarse
+    // solve of 930 unknowns repeated by every CTA); PCG64 with the stored K is the faster one at
     // every size measured (706k DOF 105 against 122 us).
     if (nslice < 1) return false;
     const int W = (int)std::max<long long>(1, c->sell_len / nslice);
@@ -1022,7 +1119,7 @@ bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
     return true;
 }
 
-void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, const Parts &P, Flags *fl, double *d_u,
+void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, bool modes, const Parts &P, Flags *fl, double *d_u,
                          float wsm, double tol2, int iters, int first) {
     SolverWork &w = c->w;
     const Coarse &C = c->coarse;
@@ -1060,6 +1157,12 @@ void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, const P
         a.x32 = w.x32.p;
         a.t32 = w.t32.p;
         a.cvec = C.cvec.p;
+        if (modes) {
+            a.md_ptr = C.md_ptr.p;
+            a.md_row = C.md_row.p;
+            a.md_val = C.md_val.p;
+            a.md = row_modes(C);
+        }
     }
     a.wsm = wsm;
     a.tol2 = tol2;

@@ -46,6 +46,9 @@ namespace ofea {
 // measured on the B200 at 79 % of HBM peak for the FP64 outer SpMV against
 // 69 % at the 48 registers the compiler picks on its own.
 constexpr int kSpmvCtas = 2048 / kBlock;
+// The post-smoothing with its K Z part: 64 registers; the grid is two full waves
+// then (6 CTAs per SM: 83 us at 1.56M DOF, 5: 88, 4: 79; without the part 62).
+constexpr int kPostModesCtas = 4;
 
 // ---------------------------------------------------------- plain SpMV --
 
@@ -340,11 +343,15 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_init(
 // Post-smoothing and the end of the preconditioner:
 // z_{k+1} = x + w Dinv32 (b32 - K32 x); partials r.z_{k+1} and r.z_k (FP64).
 // k = itB (itB = -1 for the initial application).
-__global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_post(
+// MODES: x is x0 still, and the correction Z e and K Z e are added here:
+// z_{k+1} = x0 + Z e + w Dinv32 (b32 - K32 x0 - K Z e).
+template <bool MODES>
+__global__ void __launch_bounds__(kBlock, MODES ? kPostModesCtas : kSpmvCtas) k_fcg_post(
     int nfree, const int *__restrict__ sl_ptr, const int *__restrict__ scols,
     const int *__restrict__ sl_g, const __nv_bfloat16 *__restrict__ svg, const float *__restrict__ Dinv32, float w,
     const float *__restrict__ b32, const float *__restrict__ x32, const double *__restrict__ r,
-    float *__restrict__ zA, float *__restrict__ zB, Parts P, Flags *fl) {
+    float *__restrict__ zA, float *__restrict__ zB, Parts P, Flags *fl, const RowModes md,
+    const float *__restrict__ evec) {
     __shared__ double sh[kWarpsPerBlock];
     if (cta_done(fl)) return;
     const int k = fl->itB;
@@ -353,13 +360,15 @@ __global__ void __launch_bounds__(kBlock, kSpmvCtas) k_fcg_post(
     double *Pnext = ((k + 1) & 1) ? P.rz1 : P.rz0;
     double prz = 0, przo = 0;
     for_each_sell_row(nfree, sl_ptr, [&](int rw, long S, int t, int W) {
-        float y[3], d[3], o[3];
+        float y[3], d[3], o[3], ze[3] = {0.f, 0.f, 0.f}, kz[3] = {0.f, 0.f, 0.f};
+        if constexpr (MODES) md.row(rw, evec, kz);
         sell_row_g4(S, sl_g[rw / kSlice], t, W, scols, svg, [&](int kk) { return x32[kk]; }, y[0], y[1], y[2]);
-        for (int i = 0; i < 3; ++i) d[i] = b32[3L * rw + i] - y[i];
+        for (int i = 0; i < 3; ++i) d[i] = MODES ? (b32[3L * rw + i] - y[i]) - kz[i] : b32[3L * rw + i] - y[i];
         block3_apply(Dinv32 + 9L * rw, d, o);
+        if constexpr (MODES) md.modes(rw, evec, ze);
         for (int i = 0; i < 3; ++i) {
             const long dd = 3L * rw + i;
-            const float zn = fmaf(w, o[i], x32[dd]);
+            const float zn = fmaf(w, o[i], MODES ? x32[dd] + ze[i] : x32[dd]);
             const double rv = r[dd];
             prz += rv * (double)zn;
             przo += rv * (double)zold[dd];
@@ -543,7 +552,7 @@ void drive(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, int per_chunk, 
 // one launch takes up to kResidentChunk iterations; with a time budget or a
 // poll interval of the caller's the launches are as long as those.  The iteration limit is rounded up to whole poll intervals.
 constexpr int kResidentChunk = 4096;
-void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const ResidentPlan &plan, bool mixed,
+void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const ResidentPlan &plan, bool mixed, bool modes,
                     int per_chunk, double *d_u, float wsm, double tol2, Flags &hf, long long &launches,
                     bool &timed_out, double t_start) {
     cudaStream_t s = c->stream;
@@ -552,7 +561,7 @@ void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const 
     const long limit = ((long)o.max_iter + per_chunk - 1) / per_chunk * per_chunk;
     for (long done = 0;;) {
         const int iters = (int)std::min<long>(polled ? per_chunk : kResidentChunk, limit - done);
-        resident_iterations(c, plan, mixed, ws.P, ws.fl, d_u, wsm, tol2, iters, mixed && done == 0);
+        resident_iterations(c, plan, mixed, modes, ws.P, ws.fl, d_u, wsm, tol2, iters, mixed && done == 0);
         ++launches;
         done += iters;
         OFEA_CUDA(cudaMemcpyAsync(h, ws.fl, sizeof(Flags), cudaMemcpyDeviceToHost, s));
@@ -624,6 +633,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     const bool learned = o.method == OFEA_SOLVER_LEARNED;
     const bool mixed = o.method == OFEA_SOLVER_MIXED || learned;
     float setup_ms = 0.f;
+    bool modes = false;  // the restriction takes K Z instead of the residual
     if (mixed) {
         const bool had = c->coarse.K_ok;
         cudaEvent_t es;
@@ -636,6 +646,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         } else {
             setup_coarse(c, c->coarse_nodes);
         }
+        modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
         OFEA_CUDA(cudaEventSynchronize(es));
         OFEA_CUDA(cudaEventElapsedTime(&setup_ms, e0, es));
@@ -705,7 +716,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         ofea_solve_opts oo = o;
         oo.max_iter = o.max_iter - total_iters;
         if (resident) {
-            drive_resident(c, oo, ws, plan, mixed, per_chunk, d_u, wsm, tol2, hf, launches, timed_out, t_start);
+            drive_resident(c, oo, ws, plan, mixed, modes, per_chunk, d_u, wsm, tol2, hf, launches, timed_out, t_start);
         } else if (mixed) {
             // the V-cycle kernels of this attempt return at once once the
             // solve has stopped (the flag is cleared at every attempt)
@@ -714,15 +725,26 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
             // initial preconditioner application z_0 = M(r_0)
             k_set_itB<<<1, 1, 0, s>>>(ws.fl, -1);
             auto precondition = [&] {
-                vc_resid(c, w.b32.p, w.x32.p, w.t32.p);
-                if (learned) learned_coarse_correct(c, w.t32.p, w.x32.p);
-                else coarse_correct(c, w.t32.p, w.x32.p);
-                k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm, w.b32.p,
-                                                w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl);
+                if (modes) {
+                    Coarse &C = learned ? c->coarse2 : c->coarse;
+                    restrict_modes(c, C, w.b32.p, w.x32.p, C.cvec.p);
+                    if (learned) learned_coarse_solve(c);
+                    else coarse_gemv(c, C.cvec.p, C.evec.p);
+                    k_fcg_post<true><<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p,
+                                                          wsm, w.b32.p, w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl,
+                                                          row_modes(C), learned ? C.cvec.p : C.evec.p);
+                } else {
+                    vc_resid(c, w.b32.p, w.x32.p, w.t32.p);
+                    if (learned) learned_coarse_correct(c, w.t32.p, w.x32.p);
+                    else coarse_correct(c, w.t32.p, w.x32.p);
+                    k_fcg_post<false><<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p,
+                                                           wsm, w.b32.p, w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl,
+                                                           RowModes{}, nullptr);
+                }
                 OFEA_CHECK_LAUNCH();
             };
             precondition();
-            launches += learned ? 12 : 6;
+            launches += (learned ? 12 : 6) - (modes ? 2 : 0);
             auto chunk = [&](int iters) {
                 for (int it = 0; it < iters; ++it) {
                     auto A = [&](auto K) {
@@ -740,7 +762,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
                 }
                 OFEA_CHECK_LAUNCH();
             };
-            drive(c, oo, ws, per_chunk, chunk, hf, launches, (learned ? 13 : 7) + (matfree ? 1 : 0), timed_out, t_start, {});
+            drive(c, oo, ws, per_chunk, chunk, hf, launches, (learned ? 13 : 7) + (matfree ? 1 : 0) - (modes ? 2 : 0), timed_out, t_start, {});
         } else {
             auto chunk = [&](int iters) {
                 for (int it = 0; it < iters; ++it) {
@@ -844,8 +866,9 @@ void profile_kernels(ofea_ctx *c, int method, int reps, double *ms, double *byte
             k_fcg_A<<<G, kBlock, 0, s>>>(nf, sell_rows(c), w.z32a.p, w.z32b.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, tol2);
         OFEA_CUDA(cudaEventRecord(e1, s));
         for (int i = 0; i < reps; ++i)
-            k_fcg_post<<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm, w.b32.p,
-                                            w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl);
+            k_fcg_post<false><<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p, c->Dinv32.p, wsm,
+                                                   w.b32.p, w.x32.p, w.r.p, w.z32a.p, w.z32b.p, ws.P, ws.fl, RowModes{},
+                                                   nullptr);
         OFEA_CUDA(cudaEventRecord(e2, s));
         // FP64 K + columns + slice pointers, z (FP32), p_old and q_old read, p_new and q written
         bytes[0] = 8 * nnzv + 4 * nblk + 4.0 * ((nf + 31) / 32 + 1) + 4.0 * n + 8.0 * n * 4;

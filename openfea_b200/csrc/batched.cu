@@ -13,7 +13,10 @@
 // descriptors points at them, one of records at their slices.
 //
 // Algorithm per (variant, load case): the MIXED method of solve.cu, FP64
-// flexible CG with the FP32 two-level V(1,1) preconditioner of precond.cu, or
+// flexible CG with the FP32 two-level V(1,1) preconditioner of precond.cu (with
+// K Z where every variant has it: one product instead of two, 8 to 46 % less
+// time at 1 to 32 variants of 7k and 27k nodes and 3 to 16 load cases; the
+// phases of a trace stay, the residual's is then a barrier alone), or
 // PCG64 (FP64 CG, block Jacobi).  The kernel runs every variant in lock step
 // through phases separated by grid barriers.  In the matrix phases a CTA owns
 // one slice (32 block rows) of some variant at a time: bulk copies bring the
@@ -75,6 +78,9 @@ struct BVar {
     const int *agg_ptr;
     const float4 *agg_off, *row_off;  // offsets from the centroids (precond.cu)
     const float *Einv32;
+    const int *md_ptr, *md_row;  // K Z by aggregate and by row (precond.cu)
+    const float *md_val;
+    RowModes md;
     float wsm, pad2;
 };
 
@@ -103,6 +109,9 @@ struct BArgs {
     const BVar *var;
     const BSlice *slice;
     unsigned *vmask;  // [V]: bit j set while load case j runs
+    int modes, parts; // the V-cycle takes K Z (every variant has it); parts per aggregate of its restriction
+    int ncoarse;      // values of cvec per load case
+    float *cpart;     // cvec's parts
     int cap;          // columns the staged products' buffer holds
     const int *slice_var, *agg_var, *crow_var;
     const double *f;
@@ -667,8 +676,9 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
     // phase before); partials r.z_new (pa), r.z_old (pb).  Inlined at both
     // call sites: a call would put every captured local on the stack.
     auto precondition = [&](float *znew, const float *zold) __attribute__((always_inline)) -> bool {
-        // t = b - K32 x
-        matrix_phase<float, float, true, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, a.x32, false,
+        // t = b - K32 x; not with K Z
+        if (!a.modes)
+            matrix_phase<float, float, true, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, a.x32, false,
                                                  [&](const BSlice &Rn) { pf_vec(Rn, a.b32, 4); },
                                                  [&](const BSlice &B, int, unsigned mask, float (&y)[3][RL]) {
             const int row = B.row0 + r;
@@ -682,111 +692,157 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
                 }
         });
         if (!sync()) return false;
-        // c = Z^T t: CTA per aggregate, NP lanes per node (one load case
-        // each), G = threads / NP nodes side by side and 4 nodes per thread in
-        // flight; per-warp sums, then a fixed-order sum over the warps.
+        // c = Z^T t, or Z^T b - (K Z)^T x in parts: CTA per aggregate (part), JW lanes of RL load cases per node, G nodes
+        // side by side and kU per thread in flight; per-warp sums, then a
+        // fixed-order sum over the warps.  RL load cases per lane share the 18
+        // values of a K Z entry: one per lane reads them NP times per warp.
+        // Parts because aggregates are few (about a thousand nodes each): whole
+        // ones leave CTAs idle (5 variants of 7k nodes: 21 us of a 75 us
+        // iteration, in parts 7 of 61).
         {
-            constexpr int JW = NP, kU = 4;
-            const int G = blockDim.x / JW, sub = threadIdx.x / JW, jj = threadIdx.x % JW;
+            constexpr int JW = NP / RL, kU = 4 / RL > 1 ? 4 / RL : 2;
+            const int G = blockDim.x / JW, sub = threadIdx.x / JW, jj = (threadIdx.x % JW) * RL;
             const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-            float *red = reinterpret_cast<float *>(st.v);  // [warp][6][JW]: 6 * 32 * 32 floats at most
-            for (int ga = blockIdx.x; ga < a.naggs; ga += gridDim.x) {
-                const int v = a.agg_var[ga];
-                const BVar B = a.var[v];
+            float *red = reinterpret_cast<float *>(st.v);  // [warp][6][NP]: 6 * 32 * 32 floats at most
+            const float *tv = a.modes ? a.b32 : a.t32;
+            const int np = a.modes ? a.parts : 1;
+            for (int it = blockIdx.x; it < a.naggs * np; it += gridDim.x) {
+                const int ga = it / np, part = it - ga * np, v = a.agg_var[ga];
+                auto cut = [&](const int *p, int I, int q) { return p[I] + (int)((long)(p[I + 1] - p[I]) * q / np); };
+                const BVar &B = a.var[v];
                 const int I = ga - B.agg0;
-                const bool live = jj < NR && a.live[v * NR + jj] != 0;
-                float acc[6] = {0, 0, 0, 0, 0, 0};
+                bool live = false;
+#pragma unroll
+                for (int q = 0; q < RL; ++q) live |= jj + q < NR && a.live[v * NR + jj + q] != 0;
+                float acc[6][RL] = {};
                 if (live) {
-                    auto add = [&](const float4 &o, float tx, float ty, float tz) {
-                        const float dx = o.x, dy = o.y, dz = o.z;
-                        acc[0] += tx;
-                        acc[1] += ty;
-                        acc[2] += tz;
-                        acc[3] += -dz * ty + dy * tz;
-                        acc[4] += dz * tx - dx * tz;
-                        acc[5] += -dy * tx + dx * ty;
+                    auto at = [&](const float *p, int node, float (&x)[3][RL]) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) ldv<float, RL>(p + vidx<NP>(B, node, c, jj), x[c]);
                     };
-                    const int e = B.agg_ptr[I + 1];
-                    int idx = B.agg_ptr[I] + sub;
+                    auto add = [&](const float4 &o, const float (&t)[3][RL]) {
+#pragma unroll
+                        for (int q = 0; q < RL; ++q) {
+                            acc[0][q] += t[0][q];
+                            acc[1][q] += t[1][q];
+                            acc[2][q] += t[2][q];
+                            acc[3][q] += -o.z * t[1][q] + o.y * t[2][q];
+                            acc[4][q] += o.z * t[0][q] - o.x * t[2][q];
+                            acc[5][q] += -o.y * t[0][q] + o.x * t[1][q];
+                        }
+                    };
+                    const int e = cut(B.agg_ptr, I, part + 1);
+                    int idx = cut(B.agg_ptr, I, part) + sub;
                     for (; idx + (kU - 1) * G < e; idx += kU * G) {
                         float4 o[kU];
-                        float t[kU][3];
+                        float t[kU][3][RL];
 #pragma unroll
                         for (int u = 0; u < kU; ++u) o[u] = __ldg(B.agg_off + idx + u * G);
 #pragma unroll
-                        for (int u = 0; u < kU; ++u)
+                        for (int u = 0; u < kU; ++u) at(tv, __float_as_int(o[u].w), t[u]);
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) t[u][c] = a.t32[vidx<NP>(B, __float_as_int(o[u].w), c, jj)];
-#pragma unroll
-                        for (int u = 0; u < kU; ++u) add(o[u], t[u][0], t[u][1], t[u][2]);
+                        for (int u = 0; u < kU; ++u) add(o[u], t[u]);
                     }
                     for (; idx < e; idx += G) {
                         const float4 o = __ldg(B.agg_off + idx);
-                        const int rr = __float_as_int(o.w);
-                        add(o, a.t32[vidx<NP>(B, rr, 0, jj)], a.t32[vidx<NP>(B, rr, 1, jj)], a.t32[vidx<NP>(B, rr, 2, jj)]);
+                        float t[3][RL];
+                        at(tv, __float_as_int(o.w), t);
+                        add(o, t);
+                    }
+                    if (a.modes) {  // less (K Z)^T x0, the next entry's row in flight
+                        const int end = cut(B.md_ptr, I, part + 1);
+                        int t = cut(B.md_ptr, I, part) + sub;
+                        int rr = t < end ? __ldg(B.md_row + t) : 0;
+                        while (t < end) {
+                            float x[3][RL], W[18];
+                            mode_entry(t, B.md.n, B.md_val, W);
+                            at(a.x32, rr, x);
+                            t += G;
+                            if (t < end) rr = __ldg(B.md_row + t);
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                                for (int l = 0; l < 6; ++l) fma_cases<RL>(acc[l], -W[6 * c + l], x[c]);
+                        }
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
+                for (int k = 0; k < 6; ++k)
 #pragma unroll
-                    for (int off = JW; off < 32; off <<= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-                }
+                    for (int q = 0; q < RL; ++q)
+#pragma unroll
+                        for (int off = JW; off < 32; off <<= 1) acc[k][q] += __shfl_xor_sync(0xffffffffu, acc[k][q], off);
                 if (lane < JW)
 #pragma unroll
-                    for (int k = 0; k < 6; ++k) red[(w * 6 + k) * JW + lane] = acc[k];
+                    for (int k = 0; k < 6; ++k) stv<float, RL>(red + (w * 6 + k) * NP + jj, acc[k]);
                 __syncthreads();
-                if ((int)threadIdx.x < 6 * JW) {
-                    const int k = threadIdx.x / JW, j = threadIdx.x % JW;
+                for (int s = threadIdx.x; s < 6 * NP; s += blockDim.x) {
+                    const int k = s / NP, j = s % NP;
                     float sum = 0.f;
-                    for (int ww = 0; ww < nw; ++ww) sum += red[(ww * 6 + k) * JW + j];
-                    if (j < NR && a.live[v * NR + j] != 0) a.cvec[(B.c0 + 6L * I + k) * NP + j] = sum;
+                    for (int ww = 0; ww < nw; ++ww) sum += red[(ww * 6 + k) * NP + j];
+                    const long o = B.c0 + 6L * I + k;
+                    if (j < NR && a.live[v * NR + j] != 0) (a.modes ? a.cpart[(o * np + part) * NP + j] : a.cvec[o * NP + j]) = sum;
                 }
                 __syncthreads();
             }
         }
         if (!sync()) return false;
-        // e = E^-1 c: warp per coarse row, NP lanes per load case group
-        {
-            constexpr int JW = NP, RPW = 32 / NP;
-            const int warps = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x & 31;
-            const int sub = lane / JW, jj = lane % JW;
-            for (int gr = blockIdx.x * warps + w; gr < a.ncrows; gr += gridDim.x * warps) {
-                const int v = a.crow_var[gr];
-                const BVar B = a.var[v];
-                const bool live = jj < NR && a.live[v * NR + jj] != 0;
-                const int i = gr - B.crow0, m = B.m;
-                const float *row = B.Einv32 + (long)i * m;
-                float acc = 0.f;
-                if (live)
-                    for (int k = sub; k < m; k += RPW) acc = fmaf(__ldg(row + k), a.cvec[(B.c0 + k) * NP + jj], acc);
+        // Two phases: e = E^-1 c and x += Z e, or with K Z the sum of c's parts
+        // and e = E^-1 c (z's Z e is added where z is formed).
+#pragma unroll 1
+        for (int ph = 0; ph < 2; ++ph) {
+            if (a.modes == ph) {
+                // e = E^-1 c: warp per coarse row, NP lanes per load case group
+                constexpr int JW = NP, RPW = 32 / NP;
+                const int warps = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x & 31;
+                const int sub = lane / JW, jj = lane % JW;
+                for (int gr = blockIdx.x * warps + w; gr < a.ncrows; gr += gridDim.x * warps) {
+                    const int v = a.crow_var[gr];
+                    const BVar B = a.var[v];
+                    const bool live = jj < NR && a.live[v * NR + jj] != 0;
+                    const int i = gr - B.crow0, m = B.m;
+                    const float *row = B.Einv32 + (long)i * m;
+                    float acc = 0.f;
+                    if (live)
+                        for (int k = sub; k < m; k += RPW) acc = fmaf(__ldg(row + k), a.cvec[(B.c0 + k) * NP + jj], acc);
 #pragma unroll
-                for (int off = JW; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-                if (sub == 0 && live) a.evec[(B.c0 + i) * NP + jj] = acc;
+                    for (int off = JW; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+                    if (sub == 0 && live) a.evec[(B.c0 + i) * NP + jj] = acc;
+                }
+            } else if (a.modes) {
+                for (long o = (long)blockIdx.x * blockDim.x + threadIdx.x; o < (long)a.ncoarse * NP;
+                     o += (long)gridDim.x * blockDim.x) {
+                    const float *p = a.cpart + (o / NP) * a.parts * NP + o % NP;
+                    float sum = 0.f;
+#pragma unroll 4
+                    for (int q = 0; q < a.parts; ++q) sum += p[(long)q * NP];
+                    a.cvec[o] = sum;
+                }
+            } else {
+                // x += Z e
+                for_slices_pf(
+                    [&](const BVar &Bn, int lsn) {
+                        pf_rows(Bn, lsn, a.x32, 4);
+                    },
+                    [&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
+                    if (!any || row >= B.nfree) return;
+                    const float4 o = __ldg(B.row_off + row);
+                    const int I = __float_as_int(o.w);
+                    const float dx = o.x, dy = o.y, dz = o.z;
+                    float e[6][RL], x[3][RL];
+                    for (int k = 0; k < 6; ++k) ldv<float, RL>(a.evec + (B.c0 + 6L * I + k) * NP + j0, e[k]);
+                    for (int c = 0; c < 3; ++c) ldv<float, RL>(a.x32 + X(B, row, c), x[c]);
+#pragma unroll
+                    for (int q = 0; q < RL; ++q) {
+                        x[0][q] += e[0][q] + dz * e[4][q] - dy * e[5][q];
+                        x[1][q] += e[1][q] - dz * e[3][q] + dx * e[5][q];
+                        x[2][q] += e[2][q] + dy * e[3][q] - dx * e[4][q];
+                    }
+                    for (int c = 0; c < 3; ++c) stv<float, RL>(a.x32 + X(B, row, c), x[c]);
+                });
             }
+            if (!sync()) return false;
         }
-        if (!sync()) return false;
-        // x += Z e
-        for_slices_pf(
-            [&](const BVar &Bn, int lsn) {
-                pf_rows(Bn, lsn, a.x32, 4);
-            },
-            [&](const BVar &B, int v, int gsl, int ls, int row, const bool (&live)[RL], bool any) {
-            if (!any || row >= B.nfree) return;
-            const float4 o = __ldg(B.row_off + row);
-            const int I = __float_as_int(o.w);
-            const float dx = o.x, dy = o.y, dz = o.z;
-            float e[6][RL], x[3][RL];
-            for (int k = 0; k < 6; ++k) ldv<float, RL>(a.evec + (B.c0 + 6L * I + k) * NP + j0, e[k]);
-            for (int c = 0; c < 3; ++c) ldv<float, RL>(a.x32 + X(B, row, c), x[c]);
-#pragma unroll
-            for (int q = 0; q < RL; ++q) {
-                x[0][q] += e[0][q] + dz * e[4][q] - dy * e[5][q];
-                x[1][q] += e[1][q] - dz * e[3][q] + dx * e[5][q];
-                x[2][q] += e[2][q] + dy * e[3][q] - dx * e[4][q];
-            }
-            for (int c = 0; c < 3; ++c) stv<float, RL>(a.x32 + X(B, row, c), x[c]);
-        });
-        if (!sync()) return false;
         // post-smoothing: z_new = x + w Dinv32 (b - K32 x); partials r.z_new, r.z_old
         matrix_phase<float, float, true, NP, RL>(a, st, pipe, dyn, a.cap, &s_fail, a.x32, false,
                                                  [&](const BSlice &Rn) {
@@ -800,6 +856,21 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
 #pragma unroll
             for (int q = 0; q < RL; ++q) any |= live[q] = (mask >> (j0 + q)) & 1u;
             double pn[RL] = {}, po[RL] = {};
+            if (a.modes && any && row < B.nfree) {  // y: K x0 + K Z e
+                const BVar &V = a.var[B.v];
+                for (int t = __ldg(V.md.rptr + row); t < __ldg(V.md.rptr + row + 1); ++t) {
+                    const float *ev = a.evec + (V.c0 + 6L * __ldg(V.md.agg + t)) * NP + j0;
+                    float W[18];
+                    mode_entry(t, V.md.n, V.md.val, W);
+#pragma unroll
+                    for (int l = 0; l < 6; ++l) {
+                        float e[RL];
+                        ldv<float, RL>(ev + l * NP, e);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) fma_cases<RL>(y[c], W[6 * c + l], e);
+                    }
+                }
+            }
             if (any && row < B.nfree) {
                 float res[3][RL], xv[3][RL], zn[3][RL], zo[3][RL];
                 double rv[3][RL];
@@ -811,6 +882,20 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
                     if (zold) ldv<float, RL>(zold + XR(B, row, c), zo[c]);
 #pragma unroll
                     for (int q = 0; q < RL; ++q) res[c][q] = bv[q] - y[c][q];
+                }
+                if (a.modes) {  // x0 + Z e
+                    const BVar &V = a.var[B.v];
+                    const float4 o = __ldg(V.row_off + row);
+                    const float *ev = a.evec + (V.c0 + 6L * __float_as_int(o.w)) * NP + j0;
+                    float e[6][RL];
+#pragma unroll
+                    for (int l = 0; l < 6; ++l) ldv<float, RL>(ev + l * NP, e[l]);
+#pragma unroll
+                    for (int q = 0; q < RL; ++q) {
+                        xv[0][q] += e[0][q] + o.z * e[4][q] - o.y * e[5][q];
+                        xv[1][q] += e[1][q] - o.z * e[3][q] + o.x * e[5][q];
+                        xv[2][q] += e[2][q] + o.y * e[3][q] - o.x * e[4][q];
+                    }
                 }
 #pragma unroll
                 for (int q = 0; q < RL; ++q) {
@@ -1261,13 +1346,14 @@ struct ofea_batch {
     std::vector<long> dof0, c0;
     long ndof = 0, ncoarse = 0;
     int nslices = 0, naggs = 0, ncrows = 0, su_max = 0;
-    bool mixed_ready = false, have_rhs = false;
+    bool mixed_ready = false, have_rhs = false, modes = false;
+    int parts = 1;
     ofea::DevBuf<ofea::BVar> var;
     ofea::DevBuf<ofea::BSlice> slice;
     ofea::DevBuf<unsigned> vmask;
     ofea::DevBuf<int> slice_var, agg_var, crow_var;
     ofea::DevBuf<double> f, u, r, p0, p1, q, z64, pa, pb, ff, tol2, rz, alpha, beta, rel, stage;
-    ofea::DevBuf<float> b32, x32, t32, zA, zB, cvec, evec;
+    ofea::DevBuf<float> b32, x32, t32, zA, zB, cvec, evec, cpart;
     ofea::DevBuf<int> live, iters, status, live_cnt;
     ofea::DevBuf<ofea::GridBar> gs;
     ofea::DevBuf<unsigned long long> trace;  // per-phase timestamps when tracing (trace_cap > 0)
@@ -1345,6 +1431,12 @@ void build_desc(ofea_batch *b, bool mixed) {
             B.agg_off = reinterpret_cast<const float4 *>(C.agg_off.p);
             B.row_off = reinterpret_cast<const float4 *>(C.row_off.p);
             B.Einv32 = C.Einv32.p;
+            if (b->modes) {
+                B.md_ptr = C.md_ptr.p;
+                B.md_row = C.md_row.p;
+                B.md_val = C.md_val.p;
+                B.md = row_modes(C);
+            }
             B.wsm = smoother_weight(c, kBatchSmootherDamping);
             for (int a = 0; a < C.na; ++a) av.push_back(v);
             for (int i = 0; i < C.m; ++i) cv.push_back(v);
@@ -1382,14 +1474,21 @@ void prepare(ofea_batch *b, bool mixed) {
             coarse_dense_inverse(c);
             OFEA_CUDA(cudaStreamSynchronize(c->stream));
         }
+        const size_t n = (size_t)b->ndof * b->NP;
+        for (auto *buf : {&b->b32, &b->x32, &b->t32, &b->zA, &b->zB}) buf->ensure(n);
+        b->modes = true;  // after the vectors: where memory ends, K Z gives way
+        for (ofea_ctx *c : b->ctx) {
+            b->modes = b->modes && ensure_modes(c, c->coarse);
+            OFEA_CUDA(cudaStreamSynchronize(c->stream));
+        }
         build_desc(b, true);
-        const size_t n = (size_t)b->ndof * b->NP, nc = std::max<size_t>(1, (size_t)b->ncoarse * b->NP);
-        b->b32.ensure(n);
-        b->x32.ensure(n);
-        b->t32.ensure(n);
-        b->zA.ensure(n);
-        b->zB.ensure(n);
+        const size_t nc = std::max<size_t>(1, (size_t)b->ncoarse * b->NP);
         b->cvec.ensure(nc);
+        if (b->modes) {  // about eight parts per SM
+            b->parts = std::min(16, 8 * b->num_sms / std::max(1, b->naggs) + 1);
+            b->cpart.ensure(nc * b->parts);
+            OFEA_CUDA(cudaMemsetAsync(b->cpart.p, 0, sizeof(float) * nc * b->parts, b->stream));
+        }
         b->evec.ensure(nc);
         for (auto *buf : {&b->b32, &b->x32, &b->t32, &b->zA, &b->zB})
             OFEA_CUDA(cudaMemsetAsync(buf->p, 0, sizeof(float) * n, b->stream));
@@ -1417,6 +1516,10 @@ BArgs make_args(ofea_batch *b, bool mixed, const TuneCfg &t, int max_iter, doubl
     a.var = b->var.p;
     a.slice = b->slice.p;
     a.vmask = b->vmask.p;
+    a.modes = mixed && b->modes;
+    a.parts = b->parts;
+    a.ncoarse = b->ncoarse;
+    a.cpart = b->cpart.p;
     a.cap = stage_cap(b->su_max, b->NP, t.rl, mixed);
     a.slice_var = b->slice_var.p;
     a.agg_var = b->agg_var.p;

@@ -33,6 +33,11 @@ __device__ __forceinline__ void modes_sum(int idx, int end, int step, const floa
         a[5] += -dy * tx + dx * ty;  // (e_z x d) . t
     }
 }
+// Entry e of K Z, W[6 c + l], in 18 planes.
+__device__ __forceinline__ void mode_entry(long e, long n, const float *__restrict__ val, float (&W)[18]) {
+#pragma unroll
+    for (int q = 0; q < 18; ++q) W[q] = __ldg(val + q * n + e);
+}
 // K Z as the row kernels read it: entries in row order.
 struct RowModes {
     const float4 *off;  // a row's offset from its aggregate's centroid, the aggregate
@@ -51,8 +56,7 @@ struct RowModes {
     __device__ __forceinline__ void entry(int t, const float *e, float (&kz)[3]) const {
         const float *v = e + 6 * __ldg(agg + t);
         float W[18];
-#pragma unroll
-        for (int q = 0; q < 18; ++q) W[q] = __ldg(val + q * n + t);
+        mode_entry(t, n, val, W);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             kz[c] = W[6 * c] * v[0];
@@ -77,8 +81,7 @@ inline RowModes row_modes(const Coarse &C) {
 // One entry of K Z: a -= W^T x.
 __device__ __forceinline__ void entry_sub(long e, long n, const float *__restrict__ val, float x, float y, float z, float (&a)[6]) {
     float W[18];
-#pragma unroll
-    for (int q = 0; q < 18; ++q) W[q] = __ldg(val + q * n + e);
+    mode_entry(e, n, val, W);
 #pragma unroll
     for (int l = 0; l < 6; ++l) a[l] -= fmaf(W[l], x, fmaf(W[6 + l], y, W[12 + l] * z));
 }

@@ -1593,10 +1593,11 @@ void residuals(ofea_batch *b, const TuneCfg &t) {
     BArgs a = make_args(b, false, t, 0, 0.0);
     cudaStream_t s = b->stream;
     const void *fn = residual_kernel(b->NP, t.rl);
-    const int G = std::min(kMaxGrid, b->num_sms * 4);
+    const int G = std::min(kMaxGrid, b->num_sms * 4), smem = red_bytes(b->NP, t.rl);
+    // with the slot stage above 48 KB at 32 cases, one per lane
+    OFEA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     void *args[] = {(void *)&a};
-    OFEA_CUDA(cudaLaunchKernel(fn, dim3(G), dim3(threads_for(b->NP, t.rl)), args,
-                               (size_t)red_bytes(b->NP, t.rl), s));
+    OFEA_CUDA(cudaLaunchKernel(fn, dim3(G), dim3(threads_for(b->NP, t.rl)), args, (size_t)smem, s));
     k_batch_rel<<<std::max(1, std::min(kMaxGrid, (b->V * b->NR + 7) / 8)), 256, 0, s>>>(a, b->rel.p);
     OFEA_CHECK_LAUNCH();
 }

@@ -4,6 +4,7 @@ against the per-variant solver, the oracle's assembly + a direct solve, its
 own determinism, and the failure path of its grid barrier."""
 import json
 import os
+import re
 
 import numpy as np
 import pytest
@@ -200,3 +201,59 @@ def test_staged_and_direct_columns(gpu_ctx_factory, method, nrhs):
         floor = np.diff(rp).max() * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u.T), axis=0)
         norms = np.linalg.norm(F, axis=1)
         assert np.all(np.linalg.norm(F.T - K @ u.T, axis=0) <= 1e-9 * norms + floor)
+
+
+@pytest.mark.parametrize("tangent", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 6, 20])
+def test_vcycle_with_and_without_sparse_modes(gpu_ctx_factory, tangent, nrhs):
+    # K Z exists for linear assemblies only: one variant with a tangent (at
+    # zero displacement, the same K) sends the whole batch to the products.
+    # Aggregates cut into more parts than some have K Z entries for.
+    meshes = [mg.structured_hex(n, 6, 5, 0.05 * n, 0.3, 0.25, 210e9, 0.3) for n in (1, 9, 30)]
+    ctxs, loads = [], []
+    for i, m in enumerate(meshes):
+        c = gpu_ctx_factory()
+        c.upload_mesh(m)
+        c.assemble_pattern()
+        if tangent and i == 1:
+            c.assemble_nl(np.zeros(c.n))
+        else:
+            c.assemble_linear()
+        ctxs.append(c)
+        loads.append(np.random.default_rng(i).normal(size=(nrhs, c.n)))
+    U, _ = ob.Batch(ctxs, nrhs).solve(loads, method="GPU_MIXED", rtol=1e-9)
+    for c, F, u in zip(ctxs, loads, U):
+        rp, col, val = c.get_csr()
+        K = sp.csr_matrix((val, col, rp), shape=(c.n, c.n))
+        floor = np.diff(rp).max() * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u.T), axis=0)
+        norms = np.linalg.norm(F, axis=1)
+        assert np.all(np.linalg.norm(F.T - K @ u.T, axis=0) <= 1e-9 * norms + floor)
+
+
+@pytest.mark.parametrize("nrhs", [3, 8, 16, 20, 32])
+@pytest.mark.parametrize("rl", [1, 2, 4])
+def test_every_tile_configuration(gpu_ctx_factory, tmp_path, monkeypatch, rl, nrhs):
+    # whichever configuration the tuner finds fastest has to run: each by a
+    # stored choice, every load-case stride and both methods
+    path = tmp_path / "tune.json"
+    monkeypatch.setenv("OFEA_TUNE_FILE", str(path))
+    c = gpu_ctx_factory()
+    c.upload_mesh(mg.structured_hex(5, 4, 3, 0.025, 0.02, 0.015, 210e9, 0.3))
+    c.assemble_pattern()
+    c.assemble_linear()
+    rp, col, val = c.get_csr()
+    K = sp.csr_matrix((val, col, rp), shape=(c.n, c.n))
+    F = np.random.default_rng(nrhs).normal(size=(nrhs, c.n))
+    for method in ("GPU_MIXED", "GPU_PCG"):
+        b = ob.Batch([c], nrhs)
+        b.tuning(method)
+        b.close()
+    stored = re.sub(r'"rl": \d+', '"rl": %d' % rl, path.read_text())
+    path.write_text(re.sub(r'"ctas_per_sm": \d+', '"ctas_per_sm": 1', stored))  # one entry per line
+    for method in ("GPU_MIXED", "GPU_PCG"):
+        b = ob.Batch([c], nrhs)
+        assert b.tuning(method)["rhs_per_lane"] == rl
+        (u,), _ = b.solve([F], method=method, rtol=1e-9)
+        floor = np.diff(rp).max() * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u.T), axis=0)
+        assert np.all(np.linalg.norm(F.T - K @ u.T, axis=0) <= 1e-9 * np.linalg.norm(F, axis=1) + floor)
+        b.close()

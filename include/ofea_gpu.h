@@ -334,6 +334,11 @@ OFEA_API int ofea_solve_batched(ofea_ctx *const *ctxs, int n_variants, const dou
  * wait gives up after limit_ms and *released is set to 0 (1 would mean the
  * barrier opened).  The context stays usable. */
 OFEA_API int ofea_check_barrier_timeout(ofea_ctx *ctx, int limit_ms, int *released);
+/* The same for its copies into shared memory: the batch's solver and residual
+ * kernels are launched with copies that never count as complete; every wait
+ * gives up after limit_ms without reading them and *released is set to 0.
+ * The batch and its contexts stay usable. */
+OFEA_API int ofea_check_copy_timeout(ofea_batch *batch, int method, int limit_ms, int *released);
 
 /* ---- stress recovery ------------------------------------------------------ */
 /* Replaces simulation_post::get_cauchy_stress_3d (src/post_process.cpp:79-167):

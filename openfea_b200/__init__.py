@@ -142,6 +142,7 @@ def lib():
         "ofea_batch_phase_times": (_I, [_P, _P, _I, ctypes.POINTER(_I)]),
         "ofea_solve_batched": (_I, [_P, _I, _P, _P, _I, _P, _P]),
         "ofea_check_barrier_timeout": (_I, [_P, _I, ctypes.POINTER(_I)]),
+        "ofea_check_copy_timeout": (_I, [_P, _I, _I, ctypes.POINTER(_I)]),
         "ofea_learned_train": (_I, [_P, _P, _P, _P]),
         "ofea_learned_get_weights": (_I, [_P, _P, ctypes.POINTER(_LL)]),
         "ofea_learned_set_weights": (_I, [_P, _P, _LL]),
@@ -235,6 +236,14 @@ class Batch:
         _check(lib().ofea_batch_tuning(self.h, SOLVERS[method], ctypes.byref(r), ctypes.byref(t), ctypes.byref(c),
                                        ctypes.byref(ms)), "ofea_batch_tuning")
         return {"rhs_per_lane": r.value, "threads": t.value, "ctas_per_sm": c.value, "ms_per_iteration": ms.value}
+
+    def check_copy_timeout(self, method="GPU_MIXED", limit_ms=20):
+        """The solver's kernels given copies that never complete: returns 0
+        when every wait ran out as designed, 1 if a kernel went on."""
+        r = _I(-1)
+        _check(lib().ofea_check_copy_timeout(self.h, SOLVERS[method], int(limit_ms), ctypes.byref(r)),
+               "ofea_check_copy_timeout")
+        return r.value
 
     def set_trace(self, max_phases):
         """Record the device clock after each grid barrier of later solves

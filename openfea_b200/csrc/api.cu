@@ -993,6 +993,15 @@ int ofea_check_barrier_timeout(ofea_ctx *c, int limit_ms, int *released) {
     });
 }
 
+int ofea_check_copy_timeout(ofea_batch *b, int method, int limit_ms, int *released) {
+    return guarded([&] {
+        need(b != nullptr && released != nullptr, OFEA_ERR_INVALID_ARG, "NULL argument");
+        need(method == OFEA_SOLVER_PCG64 || method == OFEA_SOLVER_MIXED, OFEA_ERR_UNKNOWN_SOLVER, "method");
+        need(limit_ms >= 1 && limit_ms <= 10000, OFEA_ERR_INVALID_ARG, "limit_ms must be 1..10000");
+        copy_probe(b, method, limit_ms, released);
+    });
+}
+
 int ofea_stress(ofea_ctx *c, const double *u, int mode, double *elem, double *node) {
     return guarded([&] {
         need(c != nullptr && u != nullptr, OFEA_ERR_INVALID_ARG, "NULL argument");

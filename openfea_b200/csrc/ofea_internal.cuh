@@ -331,6 +331,7 @@ void batch_tuning(ofea_batch *b, int method, int *rl, int *threads, int *ctas_pe
 void batch_set_trace(ofea_batch *b, int max_phases);
 void batch_phase_times(ofea_batch *b, double *ms, int cap, int *count);
 void barrier_probe(ofea_ctx *c, int limit_ms, int *released);
+void copy_probe(ofea_batch *b, int method, int limit_ms, int *released);
 void learned_begin_dataset(ofea_ctx *c, int max_samples);
 void learned_add_sample(ofea_ctx *c, const double *d_r);
 void learned_train(ofea_ctx *c, int steps, int batch, float lr, unsigned seed, double *loss0, double *loss1);

@@ -129,6 +129,21 @@ def test_grid_barrier_wait_runs_out_and_context_stays_usable(gpu_ctx_factory):
     b.close()
 
 
+@pytest.mark.parametrize("method", ["GPU_MIXED", "GPU_PCG"])
+@pytest.mark.parametrize("nrhs", [2, 17])
+def test_copy_wait_runs_out_and_batch_stays_usable(gpu_ctx_factory, method, nrhs):
+    # copies into shared memory that never complete: the kernels end with the
+    # error, nothing of the copies is used, and the batch solves afterwards
+    vs = variants(gpu_ctx_factory, count=3, nrhs=nrhs)
+    b = ob.Batch([v[0] for v in vs], nrhs)
+    before, _ = b.solve([v[3] for v in vs], method=method, rtol=1e-9)
+    assert b.check_copy_timeout(method, limit_ms=20) == 0
+    after, st = b.solve([v[3] for v in vs], method=method, rtol=1e-9)
+    assert all(s["status"] == 0 for s in st)
+    assert all(np.array_equal(x, y) for x, y in zip(before, after))
+    b.close()
+
+
 def test_batched_mixes_element_types(gpu_ctx_factory, oracle):
     """A batch holding a C3D4 tet block (per-element E) beside C3D8 variants:
     each variant is solved against its own K (checked with the oracle's)."""

@@ -612,8 +612,8 @@ int ofea_precond_reset(ofea_ctx *c) {
     return guarded([&] {
         need(c != nullptr, OFEA_ERR_INVALID_ARG, "ctx is NULL");
         geometry_join(c);
-        c->coarse.K_ok = false;
-        c->coarse2.K_ok = false;
+        c->coarse.K_ok = c->coarse2.K_ok = false;
+        c->coarse.md_gen = c->coarse2.md_gen = -1;
     });
 }
 

@@ -67,3 +67,32 @@ def test_preconditioner_with_and_without_its_mode_table(gpu_ctx_factory, kind, s
         rel, floor = host_residual(ctx, f, u)
         assert rel <= 1e-10 + floor
     assert abs(sa["iterations"] - sb["iterations"]) <= max(3, 0.1 * sb["iterations"])
+
+
+@pytest.mark.parametrize("method", ["GPU_MIXED", "GPU_LEARNED"])
+def test_a_reset_rebuilds_the_mode_table(gpu_ctx_factory, method):
+    # precond_reset: the next solve pays for the whole set-up, as after an assembly
+    m = mg.structured_hex(40, 12, 11, 0.2, 0.06, 0.055, 210e9, 0.3)
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    if method == "GPU_LEARNED":
+        ctx.learned_train(sample_iters=64, sample_every=4, steps=10, batch=8)
+    f = np.random.default_rng(3).normal(size=ctx.n)
+    ctx.set_setup_trace(True)
+
+    def phases():
+        u, _ = ctx.solve(f, method=method, rtol=1e-9)
+        return u, [p for p in ctx.setup_phase_times()]
+
+    u0, first = phases()
+    assert "modes" in first
+    u1, again = phases()
+    assert "modes" not in again
+    ctx.precond_reset()
+    u2, reset = phases()
+    ctx.assemble_linear()
+    u3, assembled = phases()
+    assert "modes" in assembled and reset == assembled
+    assert all(np.array_equal(u0, u) for u in (u1, u2, u3))

@@ -98,6 +98,11 @@ OFEA_API int ofea_ctx_destroy(ofea_ctx *ctx);
  * returns both to the driver / the C allocator (e.g. before handing the GPU
  * to another allocator). */
 OFEA_API int ofea_trim_device_memory(void);
+/* Checks what the library does where device memory ends: until the next call
+ * the calling thread's buffers may take `bytes` more (negative: no limit), and
+ * an allocation beyond that fails as one the device has no memory for.
+ * *allocated = what the thread's buffers have taken since the last call. */
+OFEA_API int ofea_limit_allocations(long long bytes, long long *allocated);
 /* Run this context's work on an existing cudaStream_t (NULL: library-owned stream). */
 OFEA_API int ofea_ctx_set_stream(ofea_ctx *ctx, void *cuda_stream);
 

@@ -129,6 +129,7 @@ def lib():
         "ofea_set_assembly_path": (_I, [_P, _I]),
         "ofea_get_assembly_path": (_I, [_P, ctypes.POINTER(ctypes.c_int)]),
         "ofea_trim_device_memory": (_I, []),
+        "ofea_limit_allocations": (_I, [_LL, ctypes.POINTER(_LL)]),
         "ofea_learn_opts_default": (None, [_P]),
         "ofea_batch_create": (_I, [ctypes.POINTER(_P), _P, _I, _I]),
         "ofea_batch_destroy": (_I, [_P]),
@@ -179,6 +180,14 @@ def _i32(a):
 def trim_device_memory():
     """Return the library's cached device memory to the driver."""
     _check(lib().ofea_trim_device_memory(), "ofea_trim_device_memory")
+
+
+def limit_allocations(nbytes=-1):
+    """Let this thread's device buffers take nbytes more (negative: no limit);
+    returns what they have taken since the last call."""
+    t = _LL(0)
+    _check(lib().ofea_limit_allocations(int(nbytes), ctypes.byref(t)), "ofea_limit_allocations")
+    return t.value
 
 
 class Batch:

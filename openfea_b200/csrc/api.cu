@@ -608,6 +608,13 @@ int ofea_trim_device_memory(void) {
     });
 }
 
+int ofea_limit_allocations(long long bytes, long long *allocated) {
+    return guarded([&] {
+        const long long taken = dev_limit(bytes);
+        if (allocated) *allocated = taken;
+    });
+}
+
 int ofea_precond_reset(ofea_ctx *c) {
     return guarded([&] {
         need(c != nullptr, OFEA_ERR_INVALID_ARG, "ctx is NULL");

@@ -59,10 +59,24 @@ size_t round_size(size_t bytes) {
     return (bytes + step - 1) / step * step;
 }
 
+// The calling thread's allocations since dev_limit, and what it may take
+// (negative: no limit).
+thread_local long long t_taken = 0, t_limit = -1;
+
 }  // namespace
+
+long long dev_limit(long long bytes) {
+    const long long taken = t_taken;
+    t_taken = 0;
+    t_limit = bytes;
+    return taken;
+}
 
 void *dev_alloc(size_t bytes, size_t *got, int *device) {
     const size_t want = round_size(bytes == 0 ? 1 : bytes);
+    if (t_limit >= 0 && t_taken + (long long)want > t_limit)
+        fail(OFEA_ERR_OOM, "allocation of " + std::to_string(want) + " bytes is beyond the set limit");
+    t_taken += (long long)want;
     int dev = 0;
     OFEA_CUDA(cudaGetDevice(&dev));
     *device = dev;

@@ -65,6 +65,7 @@ void set_last_error(const std::string &msg);
 void *dev_alloc(size_t bytes, size_t *got, int *device);
 void dev_free(void *p, size_t bytes, int device);
 void dev_trim();
+long long dev_limit(long long bytes);  // ofea_limit_allocations
 
 template <class T>
 struct DevBuf {

@@ -667,8 +667,12 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     // an unsmoothed density field gave weights 3 % apart), so a model trained
     // before is still the one that training gives.
     const bool sampling = (bool)on_chunk;
-    const bool matfree = !sampling && nf >= kMatfreeRows && matfree_ready(c);
-    const bool resident = !sampling && !learned && !(matfree && !mixed) && resident_plan(c, mixed, plan);
+    // plain PCG prefers the elements to the resident kernel, MIXED the other way
+    // round: the elements' tables are built for the solves that use them
+    auto from_elements = [&] { return !sampling && nf >= kMatfreeRows && matfree_ready(c); };
+    bool matfree = !mixed && from_elements();
+    const bool resident = !sampling && !learned && !matfree && resident_plan(c, mixed, plan);
+    if (mixed && !resident) matfree = from_elements();
     if (resident && mixed) coarse_dense_inverse(c);
     const int G = resident ? plan.G : solver_grid(c);
     Workspace ws = setup(c, G);

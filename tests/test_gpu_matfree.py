@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
+import openfea_b200 as ob
 from openfea_b200 import meshgen as mg
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +77,23 @@ def test_the_current_k_is_solved(gpu_ctx_factory):
         u, _ = ctx.solve(f, method="GPU_PCG", rtol=1e-9)
         rel, floor = residual(ctx, f, u)
         assert rel <= 1e-9 + floor, step
+
+
+def test_element_tables_are_built_for_the_solves_that_use_them(gpu_ctx_factory):
+    # MIXED on the resident kernel reads the stored K; plain PCG of the same
+    # model then builds the tables (24 FP64 forces per element among them)
+    m = model((62, 35, 32), "lines")
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    f = np.random.default_rng(7).normal(size=ctx.n)
+    ctx.solve(f, method="GPU_MIXED", rtol=1e-6)
+    try:
+        ob.limit_allocations()
+        ctx.solve(f, method="GPU_PCG", rtol=1e-6)
+        assert ob.limit_allocations() >= 192 * m.ne
+        ctx.solve(f, method="GPU_PCG", rtol=1e-6)
+        assert ob.limit_allocations() < 192 * m.ne
+    finally:
+        ob.limit_allocations()

@@ -1495,20 +1495,34 @@ void prepare(ofea_batch *b, bool mixed) {
         }
         const size_t n = (size_t)b->ndof * b->NP;
         for (auto *buf : {&b->b32, &b->x32, &b->t32, &b->zA, &b->zB}) buf->ensure(n);
-        b->modes = true;  // after the vectors: where memory ends, K Z gives way
+        size_t naggs = 0, ncrows = 0;
+        for (ofea_ctx *c : b->ctx) {
+            naggs += c->coarse.na;
+            ncrows += c->coarse.m;
+        }
+        const size_t nc = std::max<size_t>(1, ncrows * b->NP);
+        b->agg_var.ensure(naggs);
+        b->crow_var.ensure(ncrows);
+        b->cvec.ensure(nc);
+        b->evec.ensure(nc);
+        // K Z after all that the solve cannot do without: where memory ends, it
+        // gives way
+        b->modes = true;
         for (ofea_ctx *c : b->ctx) {
             b->modes = b->modes && ensure_modes(c, c->coarse);
             OFEA_CUDA(cudaStreamSynchronize(c->stream));
         }
-        build_desc(b, true);
-        const size_t nc = std::max<size_t>(1, (size_t)b->ncoarse * b->NP);
-        b->cvec.ensure(nc);
         if (b->modes) {  // about eight parts per SM
-            b->parts = std::min(16, 8 * b->num_sms / std::max(1, b->naggs) + 1);
-            b->cpart.ensure(nc * b->parts);
-            OFEA_CUDA(cudaMemsetAsync(b->cpart.p, 0, sizeof(float) * nc * b->parts, b->stream));
+            b->parts = std::min(16, 8 * b->num_sms / (int)std::max<size_t>(1, naggs) + 1);
+            try {
+                b->cpart.ensure(nc * b->parts);
+                OFEA_CUDA(cudaMemsetAsync(b->cpart.p, 0, sizeof(float) * nc * b->parts, b->stream));
+            } catch (const Failure &f) {
+                if (f.code != OFEA_ERR_OOM) throw;
+                b->modes = false;
+            }
         }
-        b->evec.ensure(nc);
+        build_desc(b, true);
         for (auto *buf : {&b->b32, &b->x32, &b->t32, &b->zA, &b->zB})
             OFEA_CUDA(cudaMemsetAsync(buf->p, 0, sizeof(float) * n, b->stream));
         OFEA_CUDA(cudaMemsetAsync(b->cvec.p, 0, sizeof(float) * nc, b->stream));

@@ -302,7 +302,7 @@ static bool build_tables(ofea_ctx *c) {
 }
 
 // mf_state: 0 not built, 1 built, -1 not for this mesh or no memory for it
-// (the stored K is used).
+// (the stored K is used, until the next pattern; nothing of the tables is kept).
 bool matfree_ready(ofea_ctx *c) {
     if (c->matrix_only || c->ne4 != 0 || c->ne8 == 0 || !c->K_linear) return false;
     if (c->mf_state == 0) {
@@ -311,6 +311,12 @@ bool matfree_ready(ofea_ctx *c) {
         } catch (const Failure &e) {
             if (e.code != OFEA_ERR_OOM) throw;
             c->mf_state = -1;
+        }
+        if (c->mf_state < 0) {
+            c->mf_link.release();
+            c->mf_rows.release();
+            c->mf_list.release();
+            c->mf_fe.release();
         }
     }
     return c->mf_state == 1;

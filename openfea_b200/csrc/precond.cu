@@ -1544,8 +1544,15 @@ __global__ void k_row_entries(int n, const int *__restrict__ row, const int *__r
     }
 }
 
+static void release_modes(Coarse &C) {
+    for (DevBuf<int> *b : {&C.md_ptr, &C.md_row, &C.md_agg, &C.md_rptr, &C.md_rpos, &C.md_ragg}) b->release();
+    C.md_val.release();
+    C.md_rval.release();
+}
+
 bool ensure_modes(ofea_ctx *c, Coarse &C) {
     if (!c->K_linear || c->matrix_only || C.md_state < 0) return false;
+    const bool fresh = C.md_rval.p == nullptr;  // tables of an earlier pattern stay: a batch may hold them
     cudaStream_t s = c->stream;
     try {
         if (C.md_state == 0) {
@@ -1584,7 +1591,8 @@ bool ensure_modes(ofea_ctx *c, Coarse &C) {
         }
     } catch (const Failure &f) {
         if (f.code != OFEA_ERR_OOM) throw;
-        C.md_state = -1;
+        C.md_state = -1;  // until the next pattern
+        if (fresh) release_modes(C);
         return false;
     }
     if (C.md_gen != c->K_gen) {

@@ -1184,7 +1184,6 @@ void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, bool mo
         OFEA_CUDA(cudaLaunchKernelExC(&cfg, mixed ? (const void *)k_cluster_solve<true> : (const void *)k_cluster_solve<false>, args));
         return;
     }
-    w.bar.ensure(2);
     a.bar = reinterpret_cast<GridBar *>(w.bar.p);
     a.limit_ns = 5000000000ull;  // 5 s: far above any phase
     OFEA_CUDA(cudaMemsetAsync(w.bar.p, 0, sizeof(GridBar), c->stream));

@@ -425,11 +425,14 @@ struct Workspace {
     double *scal;  // device scalars [4]
 };
 
+int solver_grid(const ofea_ctx *c) { return std::min(kMaxGrid, c->num_sms * (2048 / kBlock)); }
+
 Workspace setup(ofea_ctx *c, int G) {
     SolverWork &w = c->w;
     const size_t nd = 6 * (size_t)kMaxGrid + 8;
     w.partials.ensure(nd);
     w.flags.ensure(sizeof(Flags) / sizeof(int));
+    w.bar.ensure(2);
     double *b = w.partials.p;
     Workspace ws;
     ws.P.pq = b;
@@ -575,8 +578,6 @@ void drive_resident(ofea_ctx *c, const ofea_solve_opts &o, Workspace &ws, const 
     hf = *h;
 }
 
-int solver_grid(const ofea_ctx *c) { return std::min(kMaxGrid, c->num_sms * (2048 / kBlock)); }
-
 // Clears the context's V-cycle stop flag when the solve's iterations end
 // (normally or by an exception).
 struct StopFlagScope {
@@ -634,6 +635,20 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     const bool mixed = o.method == OFEA_SOLVER_MIXED || learned;
     float setup_ms = 0.f;
     bool modes = false;  // the restriction takes K Z instead of the residual
+    // every buffer the solve cannot do without, before the tables that are
+    // optional (K Z, the elements'): where memory ends, those give way
+    Workspace ws = setup(c, solver_grid(c));
+    ResidentPlan plan;
+    // A solve that hands its residuals to a callback (the learned stage's
+    // training samples) keeps the launch-per-phase kernels on the stored K and
+    // their order of sums: training amplifies rounding (samples 1e-13 apart on
+    // an unsmoothed density field gave weights 3 % apart), so a model trained
+    // before is still the one that training gives.
+    const bool sampling = (bool)on_chunk;
+    // plain PCG prefers the elements to the resident kernel, MIXED the other way
+    // round: the elements' tables are built for the solves that use them
+    auto from_elements = [&] { return !sampling && nf >= kMatfreeRows && matfree_ready(c); };
+    bool matfree = false, resident = false;
     if (mixed) {
         const bool had = c->coarse.K_ok;
         cudaEvent_t es;
@@ -646,36 +661,26 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         } else {
             setup_coarse(c, c->coarse_nodes);
         }
+        w.b32.ensure(n);
+        w.x32.ensure(n);
+        w.t32.ensure(n);
+        w.z32a.ensure(n);
+        w.z32b.ensure(n);
+        resident = !sampling && !learned && resident_plan(c, true, plan);
+        if (resident) coarse_dense_inverse(c);
         modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
         OFEA_CUDA(cudaEventSynchronize(es));
         OFEA_CUDA(cudaEventElapsedTime(&setup_ms, e0, es));
         cudaEventDestroy(es);
         if (!had) launches += 4 + 4 * ((c->coarse.m + 31) / 32) + 14;
-        w.b32.ensure(n);
-        w.x32.ensure(n);
-        w.t32.ensure(n);
-        w.z32a.ensure(n);
-        w.z32b.ensure(n);
+        if (!resident) matfree = from_elements();
     } else {
         w.z.ensure(n);
+        matfree = from_elements();
+        resident = !sampling && !matfree && resident_plan(c, false, plan);
     }
-    ResidentPlan plan;
-    // A solve that hands its residuals to a callback (the learned stage's
-    // training samples) keeps the launch-per-phase kernels on the stored K and
-    // their order of sums: training amplifies rounding (samples 1e-13 apart on
-    // an unsmoothed density field gave weights 3 % apart), so a model trained
-    // before is still the one that training gives.
-    const bool sampling = (bool)on_chunk;
-    // plain PCG prefers the elements to the resident kernel, MIXED the other way
-    // round: the elements' tables are built for the solves that use them
-    auto from_elements = [&] { return !sampling && nf >= kMatfreeRows && matfree_ready(c); };
-    bool matfree = !mixed && from_elements();
-    const bool resident = !sampling && !learned && !matfree && resident_plan(c, mixed, plan);
-    if (mixed && !resident) matfree = from_elements();
-    if (resident && mixed) coarse_dense_inverse(c);
-    const int G = resident ? plan.G : solver_grid(c);
-    Workspace ws = setup(c, G);
+    const int G = ws.P.G = resident ? plan.G : solver_grid(c);
     const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;
     for (int attempt = 0; attempt < 8; ++attempt) {
         // the whole GPU forms the residual, whatever the iterations run on; its

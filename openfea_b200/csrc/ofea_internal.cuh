@@ -165,12 +165,13 @@ struct Coarse {
     // K Z of the level (precond.cu): entries (row, aggregate) grouped by
     // aggregate, aggregate J's at md_ptr[J], 18 planes of md_n values; and the
     // same in row order, row r's at md_rptr[r] (entry e at md_rpos[e]).
-    // md_state 0: not built, 1: built for the pattern, -1: no memory for it;
-    // md_gen: the assembly whose values md_val holds.
+    // md_state 0: not built for the geometry, 1: built, -1: no memory for it,
+    // both for the pattern md_pattern; md_gen: the assembly whose values md_val
+    // holds.
     DevBuf<int> md_ptr, md_row, md_agg, md_rptr, md_rpos, md_ragg;
     DevBuf<float> md_val, md_rval;
     int md_state = 0, md_n = 0;
-    long md_gen = -1;
+    long md_gen = -1, md_pattern = -1;
     std::vector<int> agg_cell_h, cell_agg_h;  // host copies (nesting of the learned level)
     std::vector<double> centroid_h;
 };
@@ -252,6 +253,7 @@ struct ofea_ctx {
     // pattern; mf_fe: the element forces
     bool K_linear = false;
     long K_gen = 0;  // counts the assemblies
+    long pattern_gen = 0;  // counts the patterns
     ofea::DevBuf<int> mf_list, mf_rows;
     ofea::DevBuf<unsigned char> mf_link;
     ofea::DevBuf<double> mf_fe;

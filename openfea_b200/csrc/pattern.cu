@@ -335,9 +335,12 @@ void build_pattern(ofea_ctx *c) {
     c->sell_layout_ok = false;
     c->se_state = 0;
     c->mf_state = 0;
-    c->coarse.md_state = c->coarse2.md_state = 0;
     c->K_linear = false;
-    c->coarse.K_ok = false;  // the coarse geometry depends on the mesh alone: it stays
+    // The coarse geometry depends on the mesh alone: it stays, and its job may
+    // be running.  Of the coarse levels, only what the job does not write is set
+    // here; their tables are for a pattern by its number.
+    ++c->pattern_gen;
+    c->coarse.K_ok = false;
     c->coarse2.K_ok = false;
     c->learned.links_ok = false;
 }

@@ -1551,6 +1551,10 @@ static void release_modes(Coarse &C) {
 }
 
 bool ensure_modes(ofea_ctx *c, Coarse &C) {
+    if (C.md_pattern != c->pattern_gen) {
+        C.md_state = 0;
+        C.md_pattern = c->pattern_gen;
+    }
     if (!c->K_linear || c->matrix_only || C.md_state < 0) return false;
     const bool fresh = C.md_rval.p == nullptr;  // tables of an earlier pattern stay: a batch may hold them
     cudaStream_t s = c->stream;

@@ -303,8 +303,11 @@ static bool build_tables(ofea_ctx *c) {
 
 // mf_state: 0 not built, 1 built, -1 not for this mesh or no memory for it
 // (the stored K is used, until the next pattern; nothing of the tables is kept).
+bool matfree_possible(const ofea_ctx *c) {
+    return !c->matrix_only && c->ne4 == 0 && c->ne8 != 0 && c->K_linear && c->mf_state >= 0;
+}
 bool matfree_ready(ofea_ctx *c) {
-    if (c->matrix_only || c->ne4 != 0 || c->ne8 == 0 || !c->K_linear) return false;
+    if (!matfree_possible(c)) return false;
     if (c->mf_state == 0) {
         try {
             c->mf_state = build_tables(c) ? 1 : -1;

@@ -6,8 +6,9 @@
 namespace ofea {
 
 // Whether K is the linear stiffness of a mesh of C3D8 elements alone, so that
-// its products can be formed from the elements; builds the mesh's tables on
-// first use.
+// its products can be formed from the elements.
+bool matfree_possible(const ofea_ctx *c);
+// The same, and the mesh's tables are there: builds them on first use.
 bool matfree_ready(ofea_ctx *c);
 
 // Element forces of the free-DOF vector x, FP64: xA or xB by the parity of

@@ -1076,13 +1076,23 @@ int cluster_limit(int device) {
 
 }  // namespace
 
-bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
+// Where the lines lie, solve with its set-up on a new K here / launch per phase
+// (ms, at 1e-8; C3D8, smoothed moduli).  MIXED up to 3,500 slices (336k DOF):
+// with the elements' outer product there, 328k DOF (702 coarse unknowns) 6.2 /
+// 6.7, 402k (864) 7.2 / 7.1, 467k (1152) 9.9 / 8.3; without (a tangent) 6.6 /
+// 9.0, 7.3 / 9.5, 10.3 / 10.0.  The coarse level is bounded because its dense
+// inverse has to be formed, and every CTA multiplies the rows of it that its
+// own rows need: 218k DOF with 936 unknowns 4.7 / 5.1, 1344 5.2 / 5.0, 2850
+// 11.4 / 5.8; the same as a tangent, 1536 5.3 / 6.6, 2850 10.7 / 7.1; 106k DOF
+// with 1440 4.0 / 4.9, 1728 4.8 / 4.8; C3D4, 142k DOF, 1200 3.9 / 5.0, 1980
+// 6.3 / 5.1.  PCG64 with the stored K is the faster one at every size measured
+// (us per iteration: 807k DOF tangent 114 / 131, 1.56M 221 / 234, C3D4 of 3.0M
+// 266 / 280).
+constexpr int kResMixedSlices = 3500;
+constexpr int kResElementsM = 1250;  // coarse unknowns, where the other side has the elements' product
+
+bool resident_plan(const ofea_ctx *c, bool mixed, bool elements, ResidentPlan &p) {
     const int nslice = (c->nfree + kSlice - 1) / kSlice;
-    // MIXED: up to 3,500 slices (336k DOF), beyond which the launch-per-phase
-    // kernels' wider grids win (288k DOF: 85 us per iteration here, 132
-    // there before; 467k DOF: 191 here, 164 there, both without K Z, the coarse
-    // solve of 930 unknowns repeated by every CTA); PCG64 with the stored K is the faster one at
-    // every size measured (706k DOF 105 against 122 us).
     if (nslice < 1) return false;
     const int W = (int)std::max<long long>(1, c->sell_len / nslice);
     // warps per slice: the fewest serial steps over all rounds, a round's own
@@ -1112,7 +1122,7 @@ bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p) {
         p.S64 = p.S16 = pick((W + 1) / 2, kClWarps);
         return true;
     }
-    if (mixed && (nslice > 3500 || c->coarse.m > kResMaxM)) return false;
+    if (mixed && (nslice > kResMixedSlices || c->coarse.m > (elements ? kResElementsM : kResMaxM))) return false;
     p.spc = (nslice + c->num_sms - 1) / c->num_sms;
     p.G = (nslice + p.spc - 1) / p.spc;
     p.S64 = p.S16 = pick((W + 1) / 2, kResWarps);  // two slots in flight per step

@@ -15,11 +15,12 @@ struct ResidentPlan {
 };
 
 constexpr int kResThreads = 1024;
-constexpr int kResMaxM = 3072;  // coarse unknowns the preconditioned form holds in shared memory
+constexpr int kResMaxM = 1536;  // coarse unknowns the preconditioned form holds in shared memory
 
 // Whether the resident solver takes this matrix (and its plan).  With mixed,
-// the coarse level must be set up.
-bool resident_plan(const ofea_ctx *c, bool mixed, ResidentPlan &p);
+// the coarse level must be set up; elements: a launch per phase would form the
+// outer products from the elements.
+bool resident_plan(const ofea_ctx *c, bool mixed, bool elements, ResidentPlan &p);
 
 // Enqueues `iters` iterations from fl->itA on (fewer when the solve stops) on
 // the context's stream.  MIXED with first != 0 starts with the preconditioner

@@ -647,7 +647,8 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     const bool sampling = (bool)on_chunk;
     // plain PCG prefers the elements to the resident kernel, MIXED the other way
     // round: the elements' tables are built for the solves that use them
-    auto from_elements = [&] { return !sampling && nf >= kMatfreeRows && matfree_ready(c); };
+    const bool elements = !sampling && nf >= kMatfreeRows && matfree_possible(c);
+    auto from_elements = [&] { return elements && matfree_ready(c); };
     bool matfree = false, resident = false;
     if (mixed) {
         const bool had = c->coarse.K_ok;
@@ -666,7 +667,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         w.t32.ensure(n);
         w.z32a.ensure(n);
         w.z32b.ensure(n);
-        resident = !sampling && !learned && resident_plan(c, true, plan);
+        resident = !sampling && !learned && resident_plan(c, true, elements, plan);
         if (resident) coarse_dense_inverse(c);
         modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
@@ -678,7 +679,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     } else {
         w.z.ensure(n);
         matfree = from_elements();
-        resident = !sampling && !matfree && resident_plan(c, false, plan);
+        resident = !sampling && !matfree && resident_plan(c, false, elements, plan);
     }
     const int G = ws.P.G = resident ? plan.G : solver_grid(c);
     const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;

@@ -96,3 +96,26 @@ def test_a_reset_rebuilds_the_mode_table(gpu_ctx_factory, method):
     u3, assembled = phases()
     assert "modes" in assembled and reset == assembled
     assert all(np.array_equal(u0, u) for u in (u1, u2, u3))
+
+
+@pytest.mark.parametrize("shape,nodes,tangent", [((50, 16, 16), 60, False), ((80, 20, 20), 160, False), ((80, 20, 20), 100, False),
+                                                 ((100, 27, 25), 350, False), ((100, 27, 25), 350, True), ((100, 27, 25), 250, True)])
+def test_coarse_levels_on_both_sides_of_the_resident_limit(gpu_ctx_factory, shape, nodes, tangent):
+    # 1,248 to 1,728 coarse unknowns: the resident kernel takes 1,536 at most,
+    # 1,250 where the products could be formed from the elements
+    ctx = gpu_ctx_factory()
+    m = mg.structured_hex(*shape, *(0.005 * s for s in shape), 210e9, 0.3)
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.set_coarse_nodes(nodes)
+    if tangent:
+        ctx.assemble_nl(np.zeros(ctx.n))
+    else:
+        ctx.assemble_linear()
+    f = np.random.default_rng(7).normal(size=ctx.n)
+    u, _ = ctx.solve(f, method="GPU_MIXED", rtol=1e-9)
+    rel, floor = host_residual(ctx, f, u)
+    assert rel <= 1e-9 + floor
+    assert 1200 < ctx.coarse_apply()[0] < 1800
+    u2, _ = ctx.solve(f, method="GPU_MIXED", rtol=1e-9)
+    assert np.array_equal(u, u2)

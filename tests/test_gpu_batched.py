@@ -192,6 +192,40 @@ def test_batched_phase_trace(gpu_ctx_factory, tmp_path, monkeypatch, method, ini
     b.close()
 
 
+def test_stored_tuning_is_for_its_kernels_and_matrices(gpu_ctx_factory, tmp_path, monkeypatch):
+    # an entry of the file decides for the kernels, the preconditioner form and
+    # the slices it was measured with, and for no others
+    path = tmp_path / "tune.json"
+    monkeypatch.setenv("OFEA_TUNE_FILE", str(path))
+
+    def tuned(mesh, tangent=False):
+        c = gpu_ctx_factory()
+        c.upload_mesh(mesh)
+        c.assemble_pattern()
+        if tangent:
+            c.assemble_nl(np.zeros(c.n))
+        else:
+            c.assemble_linear()
+        b = ob.Batch([c], 4)
+        t = b.tuning("GPU_MIXED")
+        b.close()
+        return t, {e["key"] for e in json.load(open(path))["entries"]}
+
+    hexa = mg.structured_hex(9, 8, 5, 0.045, 0.04, 0.025, 210e9, 0.3)
+    _, first = tuned(hexa)
+    assert len(first) == 1
+    (key,) = first
+    _, again = tuned(hexa)
+    assert again == first
+    _, both = tuned(hexa, tangent=True)
+    assert len(both) == 2 and first < both
+    # what a build before this one wrote: device, method, load cases, rows, variants
+    path.write_text('{"entries": [\n{"key": "%s", "rl": 1, "ctas_per_sm": 1, "ms_per_iter": 123.0}\n]}'
+                    % "|".join(key.split("|")[:5]))
+    t, keys = tuned(hexa)
+    assert t["ms_per_iteration"] != 123.0 and key in keys
+
+
 @pytest.mark.parametrize("method", ["GPU_MIXED", "GPU_PCG"])
 @pytest.mark.parametrize("nrhs", [2, 5, 9, 17, 32])
 def test_staged_and_direct_columns(gpu_ctx_factory, method, nrhs):

@@ -393,14 +393,24 @@ OFEA_API int ofea_ca_reanalysis(ofea_ctx *base, ofea_ctx *modified, const double
 
 /* ---- measurement ------------------------------------------------------- */
 /* No counterpart in the reference (it only prints clock() spans): times the
- * solver's two per-iteration kernels (A: p update + SpMV + p.q, B: vector
- * updates + block-Jacobi + dots) of `method` in isolation, `reps` launches
- * each between CUDA events on the context's stream, on the current K and
- * solver vectors (call after a solve).  ms[0], ms[1] = average milliseconds
- * per launch of A and B; bytes[0], bytes[1] = algorithmic bytes per launch
- * (every array the kernel must touch, counted once). */
+ * solver's two kernels that stream the stored K (PCG64: A: p update + SpMV +
+ * p.q, B: vector updates + block-Jacobi + dots; MIXED: A, and the
+ * post-smoothing without K Z) in isolation, `reps` launches each between CUDA
+ * events on the context's stream, on the current K and solver vectors (call
+ * after a solve), whether or not a solve of this K runs these forms.  ms[0],
+ * ms[1] = average milliseconds per launch; bytes[0], bytes[1] = algorithmic
+ * bytes per launch (every array the kernel must touch, counted once). */
 OFEA_API int ofea_profile_solver_kernels(ofea_ctx *ctx, int method, int reps, double *ms,
                                          double *bytes);
+/* The same for the kernels that one iteration of a `method` solve launches on
+ * the current K, in order, as the solve chooses them (call after a solve with
+ * that method): *count of them (0 where one resident kernel runs the
+ * iterations), names separated by ',' (NUL terminated, cut at names_len),
+ * average ms per launch (back to back: operands that fit the L2 stay there),
+ * algorithmic bytes (0: not counted) and FP64
+ * operations (element forces only); up to cap are written. */
+OFEA_API int ofea_profile_iteration(ofea_ctx *ctx, int method, int reps, double *ms, double *bytes, double *flops,
+                                    int cap, int *count, char *names, int names_len);
 /* Set-up trace (no counterpart in the reference): with on != 0 every later
  * MIXED or LEARNED solve records CUDA events on the context's stream at the
  * phase boundaries of its preconditioner set-up (the coarse levels' Galerkin

@@ -120,6 +120,7 @@ def lib():
         "ofea_write_vtk_stress": (_I, [ctypes.c_char_p, _I, _P, _I, _P, _P, _P, _D, _P]),
         "ofea_stress": (_I, [_P, _P, _I, _P, _P]),
         "ofea_profile_solver_kernels": (_I, [_P, _I, _I, _P, _P]),
+        "ofea_profile_iteration": (_I, [_P, _I, _I, _P, _P, _P, _I, ctypes.POINTER(_I), ctypes.c_char_p, _I]),
         "ofea_set_setup_trace": (_I, [_P, _I]),
         "ofea_setup_phase_times": (_I, [_P, _P, _I, ctypes.POINTER(_I), ctypes.c_char_p, _I]),
         "ofea_precond_reset": (_I, [_P]),
@@ -465,14 +466,27 @@ class Context:
         _check(lib().ofea_precond_reset(self.h), "ofea_precond_reset")
 
     def profile_kernels(self, method="GPU_MIXED", reps=20):
-        """Average ms and algorithmic bytes per launch of the solver's A and B
-        kernels (CUDA events on the context stream)."""
+        """Average ms and algorithmic bytes per launch of the solver's two
+        kernels that stream the stored K (CUDA events on the context stream)."""
         ms = np.zeros(2)
         by = np.zeros(2)
         m = SOLVERS[method] if isinstance(method, str) else int(method)
         _check(lib().ofea_profile_solver_kernels(self.h, m, reps, _ptr(ms), _ptr(by)),
                "ofea_profile_solver_kernels")
         return ms, by
+
+    def profile_iteration(self, method="GPU_MIXED", reps=20):
+        """The kernels one iteration launches on this K, in order: dicts of
+        name, ms, bytes, flops (call after a solve with the method; empty
+        where one resident kernel runs the iterations)."""
+        cap = 16
+        ms, by, fl = np.zeros(cap), np.zeros(cap), np.zeros(cap)
+        n, buf = _I(0), ctypes.create_string_buffer(1024)
+        m = SOLVERS[method] if isinstance(method, str) else int(method)
+        _check(lib().ofea_profile_iteration(self.h, m, reps, _ptr(ms), _ptr(by), _ptr(fl), cap, ctypes.byref(n), buf,
+                                            len(buf)), "ofea_profile_iteration")
+        names = buf.value.decode().split(",") if n.value else []
+        return [dict(name=k, ms=float(ms[i]), bytes=float(by[i]), flops=float(fl[i])) for i, k in enumerate(names)]
 
     def set_setup_trace(self, on=True):
         """Record the preconditioner set-up's phase boundaries (CUDA events)

@@ -1074,6 +1074,35 @@ int ofea_profile_solver_kernels(ofea_ctx *c, int method, int reps, double *ms, d
     });
 }
 
+int ofea_profile_iteration(ofea_ctx *c, int method, int reps, double *ms, double *bytes, double *flops, int cap, int *count,
+                           char *names, int names_len) {
+    return guarded([&] {
+        need(c != nullptr && ms && bytes && flops && count && reps > 0 && cap >= 0 && names_len >= 0, OFEA_ERR_INVALID_ARG,
+             "bad argument");
+        need(c->K_ok, OFEA_ERR_STATE, "K not assembled");
+        need(method == OFEA_SOLVER_PCG64 || method == OFEA_SOLVER_MIXED || method == OFEA_SOLVER_LEARNED,
+             OFEA_ERR_UNKNOWN_SOLVER, "method");
+        use_device(c);
+        c->w.t.ensure(std::max(c->n, 1));
+        const std::vector<KernelTime> k = profile_iteration(c, method, reps);
+        *count = (int)k.size();
+        std::string joined;
+        for (int i = 0; i < *count; ++i) {
+            if (i < cap) {
+                ms[i] = k[i].ms;
+                bytes[i] = k[i].bytes;
+                flops[i] = k[i].flops;
+            }
+            joined += (i ? "," : "") + k[i].name;
+        }
+        if (names && names_len > 0) {
+            const size_t l = std::min(joined.size(), (size_t)names_len - 1);
+            std::copy(joined.begin(), joined.begin() + l, names);
+            names[l] = '\0';
+        }
+    });
+}
+
 int ofea_set_setup_trace(ofea_ctx *c, int on) {
     return guarded([&] {
         need(c != nullptr, OFEA_ERR_INVALID_ARG, "ctx is NULL");

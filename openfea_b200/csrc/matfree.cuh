@@ -5,6 +5,8 @@
 
 namespace ofea {
 
+constexpr double kHexForceOps = 1250;  // FP64 operations of one element's forces
+
 // Whether K is the linear stiffness of a mesh of C3D8 elements alone, so that
 // its products can be formed from the elements.
 bool matfree_possible(const ofea_ctx *c);

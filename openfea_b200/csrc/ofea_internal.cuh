@@ -311,6 +311,11 @@ void spmv64(ofea_ctx *c, const double *d_x, double *d_y);
 void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_opts &o,
                   ofea_solve_stats &st, const std::function<void(const double *)> &on_chunk = {});
 void profile_kernels(ofea_ctx *c, int method, int reps, double *ms, double *bytes);
+struct KernelTime {
+    std::string name;
+    double ms, bytes, flops;
+};
+std::vector<KernelTime> profile_iteration(ofea_ctx *c, int method, int reps);
 // set-up trace: setup_mark records an event named `phase` (the phase that
 // ends there) when tracing is on; setup_marks_clear drops the last set-up's
 void setup_mark(ofea_ctx *c, const char *phase);

@@ -897,4 +897,123 @@ void profile_kernels(ofea_ctx *c, int method, int reps, double *ms, double *byte
     cudaEventDestroy(e2);
 }
 
+// The kernels that one iteration of a solve launches on the context's K, in
+// order (none where the resident kernel runs them all), each timed by itself.
+// bytes: what it has to read and write, each array once (0: not counted);
+// flops: FP64 operations of the element forces.
+std::vector<KernelTime> profile_iteration(ofea_ctx *c, int method, int reps) {
+    cudaStream_t s = c->stream;
+    const int n = c->n, nf = c->nfree;
+    SolverWork &w = c->w;
+    const bool learned = method == OFEA_SOLVER_LEARNED, mixed = method == OFEA_SOLVER_MIXED || learned;
+    Coarse &C = learned ? c->coarse2 : c->coarse;
+    if (mixed ? !c->coarse.K_ok || !C.K_ok || !w.z32a.p || w.z32a.n < (size_t)n : !w.z.p || w.z.n < (size_t)n)
+        fail(OFEA_ERR_STATE, "run a solve with this method first");
+    const int G = solver_grid(c);
+    Workspace ws = setup(c, G);
+    ResidentPlan plan;
+    const bool elements = nf >= kMatfreeRows && matfree_possible(c);
+    bool matfree = !mixed && elements && matfree_ready(c);
+    if (!learned && !matfree && resident_plan(c, mixed, elements, plan)) return {};
+    const bool modes = mixed && ensure_modes(c, C);
+    if (mixed) matfree = elements && matfree_ready(c);
+    const double nnzv = 9.0 * c->sell_len * kSlice, nblk = (double)c->sell_len * kSlice;  // incl. padding
+    const double zb = mixed ? 4.0 : 8.0, vec = 8.0 * n, slices = 4.0 * ((nf + 31) / 32 + 1);
+    const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;
+    double *u = w.t.p;
+
+    struct Step {
+        const char *name;
+        double bytes, flops;
+        std::function<void()> launch;
+    };
+    std::vector<Step> steps;
+    double listed = 0;  // element forces a row reads
+    if (matfree) {
+        std::vector<int> list((size_t)c->mf_width * nf);
+        std::vector<unsigned char> link(c->ne8);
+        OFEA_CUDA(cudaMemcpyAsync(list.data(), c->mf_list.p, sizeof(int) * list.size(), cudaMemcpyDeviceToHost, s));
+        OFEA_CUDA(cudaMemcpyAsync(link.data(), c->mf_link.p, link.size(), cudaMemcpyDeviceToHost, s));
+        OFEA_CUDA(cudaStreamSynchronize(s));
+        for (int p : list) listed += p >= 0;
+        double written = 4.0 * c->ne8;
+        for (unsigned char l : link) written += l ? 0 : 4;
+        // nodes and rows of the elements, moduli, links, coordinates, z; forces
+        steps.push_back({"k_hex_forces", 73.0 * c->ne8 + 24.0 * c->nd + zb * n + 24.0 * written, kHexForceOps * c->ne8, [=, &w] {
+                             if (mixed) matfree_forces(c, w.z32a.p, w.z32b.p, ws.fl);
+                             else matfree_forces(c, w.z.p, ws.fl);
+                         }});
+    }
+    auto A = [=, &w](auto K) {
+        if (mixed) k_fcg_A<<<G, kBlock, 0, s>>>(nf, K, w.z32a.p, w.z32b.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, -1.0);
+        else k_pcg64_A<<<G, kBlock, 0, s>>>(nf, K, w.z.p, w.p0.p, w.p1.p, w.q.p, ws.P, ws.fl, -1.0);
+    };
+    // K (or the list and the forces), z, p and q read, p and q written
+    const double kb = matfree ? 4.0 * c->mf_width * nf + 24.0 * listed : 8 * nnzv + 4 * nblk + slices;
+    steps.push_back({mixed ? "k_fcg_A" : "k_pcg64_A", kb + zb * n + 4 * vec, 0.0, [=] {
+                         if (matfree) A(matfree_rows(c));
+                         else A(sell_rows(c));
+                     }});
+    if (!mixed) {
+        steps.push_back({"k_pcg64_B", 72.0 * nf + 7 * vec, 0.0, [=, &w] {
+                             k_pcg64_B<<<G, kBlock, 0, s>>>(nf, c->Dinv.p, w.p0.p, w.p1.p, w.q.p, u, w.r.p, w.z.p, ws.P, ws.fl);
+                         }});
+    } else {
+        steps.push_back({"k_fcg_B", 36.0 * nf + 6 * vec + 8.0 * n, 0.0, [=, &w] {
+                             k_fcg_B<<<G, kBlock, 0, s>>>(nf, c->Dinv32.p, wsm, w.p0.p, w.p1.p, w.q.p, u, w.r.p, w.b32.p, w.x32.p,
+                                                          ws.P, ws.fl);
+                         }});
+        const double k16 = 2 * nnzv + 4 * nblk + 2 * slices, entries = modes ? 76.0 * C.md_n : 0.0;
+        const float *evec = learned ? C.cvec.p : C.evec.p;
+        if (modes) {
+            steps.push_back({"k_restrict_modes", 16.0 * nf + 8.0 * n + entries, 0.0,
+                             [=, &w, &C] { restrict_modes(c, C, w.b32.p, w.x32.p, C.cvec.p); }});
+        } else {
+            steps.push_back({"k_vc_resid", k16 + 12.0 * n, 0.0, [=, &w] { vc_resid(c, w.b32.p, w.x32.p, w.t32.p); }});
+            steps.push_back({"k_restrict", 16.0 * nf + 4.0 * n, 0.0, [=, &w, &C] { restrict_level(c, C, w.t32.p, C.cvec.p); }});
+        }
+        steps.push_back({learned ? "learned coarse solve" : "coarse solve", 0.0, 0.0, [=, &C] {
+                             if (learned) learned_coarse_solve(c);
+                             else coarse_gemv(c, C.cvec.p, C.evec.p);
+                         }});
+        if (!modes)
+            steps.push_back({"k_prolong", 16.0 * nf + 8.0 * n, 0.0, [=, &w, &C] { prolong_level(c, C, evec, w.x32.p); }});
+        // BF16 K, b, x, Dinv32, r and z_old read, z written; with K Z its entries by row and the rows' offsets
+        steps.push_back({"k_fcg_post", k16 + 8.0 * n + 36.0 * nf + vec + 8.0 * n + (modes ? entries + 20.0 * nf : 0.0), 0.0, [=, &w, &C] {
+                             if (modes)
+                                 k_fcg_post<true><<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p,
+                                                                       c->Dinv32.p, wsm, w.b32.p, w.x32.p, w.r.p, w.z32a.p,
+                                                                       w.z32b.p, ws.P, ws.fl, row_modes(C), evec);
+                             else
+                                 k_fcg_post<false><<<G, kBlock, 0, s>>>(nf, c->sl_ptr.p, c->scols.p, c->sl_g.p, c->sv16g.p,
+                                                                        c->Dinv32.p, wsm, w.b32.p, w.x32.p, w.r.p, w.z32a.p,
+                                                                        w.z32b.p, ws.P, ws.fl, RowModes{}, nullptr);
+                         }});
+    }
+    Flags f0{};
+    f0.itA = f0.itB = 1;
+    const std::vector<double> ones(6 * kMaxGrid, 1.0);
+    cudaEvent_t e[2];
+    for (auto &x : e) OFEA_CUDA(cudaEventCreate(&x));
+    std::vector<KernelTime> out;
+    for (const Step &k : steps) {
+        Flags f{};
+        OFEA_CUDA(cudaMemcpyAsync(ws.fl, &f0, sizeof(Flags), cudaMemcpyHostToDevice, s));
+        OFEA_CUDA(cudaMemcpyAsync(ws.P.pq, ones.data(), sizeof(double) * ones.size(), cudaMemcpyHostToDevice, s));
+        k.launch();
+        OFEA_CUDA(cudaEventRecord(e[0], s));
+        for (int i = 0; i < reps; ++i) k.launch();
+        OFEA_CUDA(cudaEventRecord(e[1], s));
+        OFEA_CHECK_LAUNCH();
+        OFEA_CUDA(cudaMemcpyAsync(&f, ws.fl, sizeof(Flags), cudaMemcpyDeviceToHost, s));
+        OFEA_CUDA(cudaStreamSynchronize(s));
+        if (f.done) fail(OFEA_ERR_STATE, std::string(k.name) + " stopped while it was timed");
+        float t = 0;
+        OFEA_CUDA(cudaEventElapsedTime(&t, e[0], e[1]));
+        out.push_back({k.name, t / reps, k.bytes, k.flops});
+    }
+    for (auto &x : e) cudaEventDestroy(x);
+    return out;
+}
+
 }  // namespace ofea

@@ -97,3 +97,35 @@ def test_element_tables_are_built_for_the_solves_that_use_them(gpu_ctx_factory):
         assert ob.limit_allocations() < 192 * m.ne
     finally:
         ob.limit_allocations()
+
+
+def test_profiled_kernels_are_those_the_solve_launches(gpu_ctx_factory):
+    # elements, K Z or the stored K by what the solve of this K takes; nothing
+    # where the resident kernel runs the iterations
+    def names(ctx, method):
+        f = np.random.default_rng(7).normal(size=ctx.n)
+        ctx.solve(f, method=method, rtol=1e-6)
+        ks = ctx.profile_iteration(method, reps=3)
+        assert all(k["ms"] > 0 for k in ks)
+        u, _ = ctx.solve(f, method=method, rtol=1e-9)  # the vectors it timed on are scratch
+        rel, floor = residual(ctx, f, u)
+        assert rel <= 1e-9 + floor
+        return [k["name"] for k in ks]
+
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(model((95, 36, 33), "lines"))
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    assert names(ctx, "GPU_PCG") == ["k_hex_forces", "k_pcg64_A", "k_pcg64_B"]
+    assert names(ctx, "GPU_MIXED") == ["k_hex_forces", "k_fcg_A", "k_fcg_B", "k_restrict_modes", "coarse solve", "k_fcg_post"]
+    ctx.assemble_nl(np.zeros(ctx.n))
+    assert names(ctx, "GPU_PCG") == []
+    assert names(ctx, "GPU_MIXED") == ["k_fcg_A", "k_fcg_B", "k_vc_resid", "k_restrict", "coarse solve", "k_prolong",
+                                       "k_fcg_post"]
+    small = gpu_ctx_factory()
+    small.upload_mesh(model((12, 8, 6), "lines"))
+    small.assemble_pattern()
+    small.assemble_linear()
+    assert names(small, "GPU_MIXED") == []
+    small.learned_train(sample_iters=64, sample_every=4, steps=10, batch=8)
+    assert names(small, "GPU_LEARNED") == ["k_fcg_A", "k_fcg_B", "k_restrict_modes", "learned coarse solve", "k_fcg_post"]

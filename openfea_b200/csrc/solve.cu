@@ -427,12 +427,16 @@ struct Workspace {
 
 int solver_grid(const ofea_ctx *c) { return std::min(kMaxGrid, c->num_sms * (2048 / kBlock)); }
 
-Workspace setup(ofea_ctx *c, int G) {
-    SolverWork &w = c->w;
-    const size_t nd = 6 * (size_t)kMaxGrid + 8;
-    w.partials.ensure(nd);
+constexpr size_t kPartials = 6 * (size_t)kMaxGrid + 8;
+void reserve(SolverWork &w) {
+    w.partials.ensure(kPartials);
     w.flags.ensure(sizeof(Flags) / sizeof(int));
     w.bar.ensure(2);
+}
+
+Workspace setup(ofea_ctx *c, int G) {
+    SolverWork &w = c->w;
+    reserve(w);
     double *b = w.partials.p;
     Workspace ws;
     ws.P.pq = b;
@@ -444,7 +448,7 @@ Workspace setup(ofea_ctx *c, int G) {
     ws.scal = b + 6 * kMaxGrid;
     ws.P.G = G;
     ws.fl = reinterpret_cast<Flags *>(w.flags.p);
-    OFEA_CUDA(cudaMemsetAsync(w.partials.p, 0, nd * sizeof(double), c->stream));
+    OFEA_CUDA(cudaMemsetAsync(w.partials.p, 0, kPartials * sizeof(double), c->stream));
     OFEA_CUDA(cudaMemsetAsync(w.flags.p, 0, sizeof(Flags), c->stream));
     w.hflags.ensure(2 * sizeof(Flags) / sizeof(int));  // two slots: drive() reads one chunk's flags while the next runs
     w.hscal.ensure(4);
@@ -637,7 +641,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     bool modes = false;  // the restriction takes K Z instead of the residual
     // every buffer the solve cannot do without, before the tables that are
     // optional (K Z, the elements'): where memory ends, those give way
-    Workspace ws = setup(c, solver_grid(c));
+    reserve(w);
     ResidentPlan plan;
     // A solve that hands its residuals to a callback (the learned stage's
     // training samples) keeps the launch-per-phase kernels on the stored K and
@@ -668,20 +672,22 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         w.z32a.ensure(n);
         w.z32b.ensure(n);
         resident = !sampling && !learned && resident_plan(c, true, elements, plan);
-        if (resident) coarse_dense_inverse(c);
+        if (resident) c->coarse.Einv32.ensure((size_t)c->coarse.m * c->coarse.m);
         modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
         OFEA_CUDA(cudaEventSynchronize(es));
         OFEA_CUDA(cudaEventElapsedTime(&setup_ms, e0, es));
         cudaEventDestroy(es);
         if (!had) launches += 4 + 4 * ((c->coarse.m + 31) / 32) + 14;
-        if (!resident) matfree = from_elements();
+        if (resident) coarse_dense_inverse(c);  // after the wait: the GPU forms it while the solve is enqueued
+        else matfree = from_elements();
     } else {
         w.z.ensure(n);
         matfree = from_elements();
         resident = !sampling && !matfree && resident_plan(c, false, elements, plan);
     }
-    const int G = ws.P.G = resident ? plan.G : solver_grid(c);
+    const int G = resident ? plan.G : solver_grid(c);
+    Workspace ws = setup(c, G);
     const float wsm = mixed ? smoother_weight(c, kSmootherDamping) : 0.f;
     for (int attempt = 0; attempt < 8; ++attempt) {
         // the whole GPU forms the residual, whatever the iterations run on; its

@@ -339,7 +339,12 @@ OFEA_API int ofea_solve_batched(ofea_ctx *const *ctxs, int n_variants, const dou
  * wait gives up after limit_ms and *released is set to 0 (1 would mean the
  * barrier opened).  The context stays usable. */
 OFEA_API int ofea_check_barrier_timeout(ofea_ctx *ctx, int limit_ms, int *released);
-/* The same for its copies into shared memory: the batch's solver and residual
+/* The same for the grid barrier of the single-matrix resident solver: a solve
+ * whose barrier waits for one CTA more than exists ends with OFEA_ERR_TIMEOUT
+ * after limit_ms and *released is set to 0 (1: the solve ended otherwise, as
+ * for a model that does not run on the grid). */
+OFEA_API int ofea_check_resident_timeout(ofea_ctx *ctx, int method, int limit_ms, int *released);
+/* The same for the batched solver's copies into shared memory: the batch's solver and residual
  * kernels are launched with copies that never count as complete; every wait
  * gives up after limit_ms without reading them and *released is set to 0.
  * The batch and its contexts stay usable. */

@@ -144,6 +144,7 @@ def lib():
         "ofea_batch_phase_times": (_I, [_P, _P, _I, ctypes.POINTER(_I)]),
         "ofea_solve_batched": (_I, [_P, _I, _P, _P, _I, _P, _P]),
         "ofea_check_barrier_timeout": (_I, [_P, _I, ctypes.POINTER(_I)]),
+        "ofea_check_resident_timeout": (_I, [_P, _I, _I, ctypes.POINTER(_I)]),
         "ofea_check_copy_timeout": (_I, [_P, _I, _I, ctypes.POINTER(_I)]),
         "ofea_learned_train": (_I, [_P, _P, _P, _P]),
         "ofea_learned_get_weights": (_I, [_P, _P, ctypes.POINTER(_LL)]),
@@ -303,6 +304,15 @@ def check_barrier_timeout(ctx, limit_ms=20):
     1 if it opened (it must not), 0 when every wait ran out as designed."""
     r = _I(-1)
     _check(lib().ofea_check_barrier_timeout(ctx.h, int(limit_ms), ctypes.byref(r)), "ofea_check_barrier_timeout")
+    return r.value
+
+
+def check_resident_timeout(ctx, method="GPU_MIXED", limit_ms=20):
+    """The same for the resident solver's grid barrier: 0 when the solve ended
+    with the time-out status, 1 if it ended otherwise."""
+    r = _I(-1)
+    _check(lib().ofea_check_resident_timeout(ctx.h, SOLVERS[method], int(limit_ms), ctypes.byref(r)),
+           "ofea_check_resident_timeout")
     return r.value
 
 

@@ -1000,6 +1000,39 @@ int ofea_check_barrier_timeout(ofea_ctx *c, int limit_ms, int *released) {
     });
 }
 
+int ofea_check_resident_timeout(ofea_ctx *c, int method, int limit_ms, int *released) {
+    return guarded([&] {
+        need(c != nullptr && released != nullptr, OFEA_ERR_INVALID_ARG, "NULL argument");
+        need(method == OFEA_SOLVER_PCG64 || method == OFEA_SOLVER_MIXED, OFEA_ERR_UNKNOWN_SOLVER, "method");
+        need(limit_ms >= 1 && limit_ms <= 10000, OFEA_ERR_INVALID_ARG, "limit_ms must be 1..10000");
+        ofea_solve_opts o;
+        ofea_solve_opts_default(&o);
+        o.method = method;
+        check_solve_ready(c, o);
+        use_device(c);
+        const std::vector<double> f(std::max(c->n, 1), 1.0);
+        c->w.f.upload(f.data(), f.size(), c->stream);
+        c->w.u.ensure(f.size());
+        OFEA_CUDA(cudaMemsetAsync(c->w.u.p, 0, sizeof(double) * f.size(), c->stream));
+        OFEA_CUDA(cudaStreamSynchronize(c->stream));
+        const unsigned long long limit = c->wait_limit_ns;
+        c->wait_limit_ns = (unsigned long long)limit_ms * 1000000ull;
+        c->wait_missing = true;
+        *released = 1;
+        int code = OFEA_OK;
+        ofea_solve_stats st{};
+        try {
+            solve_device(c, c->w.f.p, c->w.u.p, o, st);
+        } catch (const Failure &e) {
+            code = e.code;
+            if (code == OFEA_ERR_TIMEOUT) *released = 0;
+        }
+        c->wait_limit_ns = limit;
+        c->wait_missing = false;
+        need(code == OFEA_OK || code == OFEA_ERR_TIMEOUT, code, "the solve failed otherwise");
+    });
+}
+
 int ofea_check_copy_timeout(ofea_batch *b, int method, int limit_ms, int *released) {
     return guarded([&] {
         need(b != nullptr && released != nullptr, OFEA_ERR_INVALID_ARG, "NULL argument");

@@ -134,7 +134,7 @@ struct SolverWork {
     DevBuf<float> b32, x32, t32, z32a, z32b;    // FP32 preconditioner vectors
     DevBuf<double> partials;   // reduction partials (several arrays of kMaxGrid)
     DevBuf<int> flags;         // [0]=done [1]=iters [2]=status
-    DevBuf<unsigned> bar;      // the resident solver's barrier slots and error flag
+    DevBuf<unsigned> bar;      // the resident solver's barrier: count and error flag
     HostBuf<int> hflags;
     HostBuf<double> hscal;
 };
@@ -258,6 +258,10 @@ struct ofea_ctx {
     ofea::DevBuf<unsigned char> mf_link;
     ofea::DevBuf<double> mf_fe;
     int mf_state = 0, mf_width = 0;
+    // the resident solver's barrier: its time limit (far above any phase), and
+    // whether it counts one arrival too few (ofea_check_resident_timeout)
+    unsigned long long wait_limit_ns = 5000000000ull;
+    bool wait_missing = false;
     bool fused_off = false;  // ofea_set_assembly_path(ctx, 1): always the two-pass assembly
     // solver layout of K (sell.cuh): BSELL-32, FP64 and BF16 values
     ofea::DevBuf<int> sl_ptr, scols;

@@ -12,7 +12,8 @@
 // loads in flight at once) and are summed through shared memory in a fixed
 // order, and the coarse level's solve and prolongation are one phase: each
 // CTA forms the few aggregates' corrections its own rows need from the dense
-// inverse.  Phases per iteration: PCG64 A | B; MIXED A | B | residual |
+// inverse.  Phases per iteration: PCG64 A | B; MIXED with K Z A | B | product
+// K x0 and restriction | coarse solve and z, without it A | B | residual |
 // restriction | coarse solve + prolongation | post-smoothing.  The arithmetic
 // is that of the launch-per-phase kernels of solve.cu and precond.cu; only
 // the order of the sums differs.  Every sum has a fixed order: results are
@@ -36,8 +37,11 @@
 // DOF), the next step's columns or the own rows in registers across the
 // product (spills: 25 against 18).
 //
-// Every wait is bounded (%globaltimer): on expiry the kernel sets the error
-// status and every CTA returns.
+// Every wait of this kernel is bounded (%globaltimer): on expiry it sets the
+// error status and every CTA returns.  The cluster form below waits at the
+// hardware's cluster barrier only: no spin on memory; its CTAs are
+// resident together and all pass the same barriers, their exits decided by
+// values that every CTA sums alike.
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -1195,8 +1199,9 @@ void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, bool mo
         return;
     }
     a.bar = reinterpret_cast<GridBar *>(w.bar.p);
-    a.limit_ns = 5000000000ull;  // 5 s: far above any phase
+    a.limit_ns = c->wait_limit_ns;
     OFEA_CUDA(cudaMemsetAsync(w.bar.p, 0, sizeof(GridBar), c->stream));
+    if (c->wait_missing) OFEA_CUDA(cudaMemsetAsync(&a.bar->count, 0xff, sizeof(a.bar->count), c->stream));  // -1
     void *args[] = {(void *)&a};
     const void *fn = mixed ? (const void *)k_resident<true> : (const void *)k_resident<false>;
     OFEA_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.G), dim3(kResThreads), args, 0, c->stream));

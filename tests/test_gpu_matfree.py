@@ -129,3 +129,26 @@ def test_profiled_kernels_are_those_the_solve_launches(gpu_ctx_factory):
     assert names(small, "GPU_MIXED") == []
     small.learned_train(sample_iters=64, sample_every=4, steps=10, batch=8)
     assert names(small, "GPU_LEARNED") == ["k_fcg_A", "k_fcg_B", "k_restrict_modes", "learned coarse solve", "k_fcg_post"]
+
+
+def test_learned_solve_from_the_elements_and_from_the_stored_k(gpu_ctx_factory):
+    # the learned stage on the same weights: outer products from the elements
+    # (and K Z), and from K loaded as a matrix
+    m = model((62, 35, 32), "lines")
+    a, b = gpu_ctx_factory(), gpu_ctx_factory()
+    fm = a.upload_mesh(m)
+    a.assemble_pattern()
+    a.assemble_linear()
+    a.learned_train(sample_iters=64, sample_every=4, steps=10, batch=8)
+    rp, col, val = a.get_csr()
+    b.upload_csc(m.xyz, fm, rp, col, val)
+    b.set_learned_weights(a.learned_weights())
+    f = np.random.default_rng(7).normal(size=a.n)
+    ua, sa = a.solve(f, method="GPU_LEARNED", rtol=1e-9)
+    ub, sb = b.solve(f, method="GPU_LEARNED", rtol=1e-9)
+    for u in (ua, ub):
+        rel, floor = residual(a, f, u)
+        assert rel <= 1e-9 + floor
+    assert [k["name"] for k in a.profile_iteration("GPU_LEARNED", reps=2)][0] == "k_hex_forces"
+    assert [k["name"] for k in b.profile_iteration("GPU_LEARNED", reps=2)][0] == "k_fcg_A"
+    assert abs(sa["iterations"] - sb["iterations"]) <= max(3, 0.1 * sb["iterations"])

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
+import openfea_b200 as ob
 from openfea_b200 import meshgen as mg
 
 pytestmark = pytest.mark.gpu
@@ -119,3 +120,36 @@ def test_coarse_levels_on_both_sides_of_the_resident_limit(gpu_ctx_factory, shap
     assert 1200 < ctx.coarse_apply()[0] < 1800
     u2, _ = ctx.solve(f, method="GPU_MIXED", rtol=1e-9)
     assert np.array_equal(u, u2)
+
+
+@pytest.mark.parametrize("method", ["GPU_PCG", "GPU_MIXED"])
+def test_barrier_wait_runs_out_and_context_stays_usable(gpu_ctx_factory, method):
+    m = mg.structured_hex(41, 9, 8, 0.2, 0.045, 0.04, 210e9, 0.3)
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    f = np.random.default_rng(7).normal(size=ctx.n)
+    u, _ = ctx.solve(f, method=method, rtol=1e-9)
+    assert ob.check_resident_timeout(ctx, method, limit_ms=20) == 0
+    again, _ = ctx.solve(f, method=method, rtol=1e-9)
+    assert np.array_equal(u, again)
+
+
+def test_time_budget_ends_a_resident_solve(gpu_ctx_factory):
+    # a budget that is over at the first poll: one launch of a few iterations,
+    # the residual of what it reached, and the same solve without one afterwards
+    m = mg.structured_hex(41, 9, 8, 0.2, 0.045, 0.04, 210e9, 0.3)
+    ctx = gpu_ctx_factory()
+    ctx.upload_mesh(m)
+    ctx.assemble_pattern()
+    ctx.assemble_linear()
+    f = np.random.default_rng(7).normal(size=ctx.n)
+    for method in ("GPU_PCG", "GPU_MIXED"):
+        u, full = ctx.solve(f, method=method, rtol=1e-10)
+        part, st = ctx.solve(f, method=method, rtol=1e-10, time_budget_s=1e-9, raise_on_error=False)
+        assert st["status"] != 0 and 0 < st["iterations"] < full["iterations"]
+        rel, floor = host_residual(ctx, f, part)
+        assert 1e-10 < rel and abs(rel - st["rel_residual"]) <= 1e-6 * rel + floor
+        again, _ = ctx.solve(f, method=method, rtol=1e-10)
+        assert np.array_equal(u, again)

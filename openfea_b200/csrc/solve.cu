@@ -639,9 +639,6 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
     const bool mixed = o.method == OFEA_SOLVER_MIXED || learned;
     float setup_ms = 0.f;
     bool modes = false;  // the restriction takes K Z instead of the residual
-    // every buffer the solve cannot do without, before the tables that are
-    // optional (K Z, the elements'): where memory ends, those give way
-    reserve(w);
     ResidentPlan plan;
     // A solve that hands its residuals to a callback (the learned stage's
     // training samples) keeps the launch-per-phase kernels on the stored K and
@@ -673,6 +670,9 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         w.z32b.ensure(n);
         resident = !sampling && !learned && resident_plan(c, true, elements, plan);
         if (resident) c->coarse.Einv32.ensure((size_t)c->coarse.m * c->coarse.m);
+        // every buffer the solve cannot do without is there, before the tables
+        // that are optional (K Z, the elements'): where memory ends, those give way
+        reserve(w);
         modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
         OFEA_CUDA(cudaEventSynchronize(es));
@@ -683,6 +683,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         else matfree = from_elements();
     } else {
         w.z.ensure(n);
+        reserve(w);
         matfree = from_elements();
         resident = !sampling && !matfree && resident_plan(c, false, elements, plan);
     }

@@ -1406,7 +1406,8 @@ void setup_coarse(ofea_ctx *c, int target_nodes) {
 // K once) a cycle takes one product with the smoother's BF16 K, K x0, instead
 // of two: M = 2 S - S K S + (Z - S K Z) E^-1 (Z - S K Z)^T stays symmetric
 // whatever K x0 is rounded to, and no pass writes x0 + Z e: at 1.56M DOF
-// restriction 17 us and post-smoothing 79 against 61 + 7 + 5 + 62 us.  (Taking K Z in the
+// restriction 17 us and post-smoothing 79 against 61 + 7 + 5 + 62 us (each alone
+// and back to back: 10 and 87, the post-smoothing without K Z 72).  (Taking K Z in the
 // restriction alone leaves the two halves apart by that rounding: 129
 // iterations instead of 113 at 1.5k DOF.)
 //

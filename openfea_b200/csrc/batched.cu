@@ -1486,6 +1486,15 @@ void build_desc(ofea_batch *b, bool mixed) {
     OFEA_CUDA(cudaStreamSynchronize(s));
 }
 
+// K Z in a batch up to so many entries per row (about 1,000 nodes per
+// aggregate give 0.3 to 1): a product serves all load cases with one read of a
+// matrix value, K Z's sums gather six coarse values per entry and load case.
+// MIXED solve with K Z / without, ms, 1 variant: 16 load cases, 17.6k nodes C3D8,
+// 0.7 entries per row 4.84 / 5.94, 1.3 4.41 / 4.50, 1.8 4.53 / 4.26, 2.6 5.68 /
+// 5.14; 32, 4.8k nodes C3D4, 0.4 5.16 / 6.67, 1.4 3.29 / 3.20, 2.2 3.05 / 2.56;
+// 16, 46k nodes C3D8, 0.8 12.2 / 13.7, 1.4 10.7 / 11.3, 2.0 11.8 / 11.6.
+constexpr double kBatchModes = 1.5;
+
 void prepare(ofea_batch *b, bool mixed) {
     if (mixed && !b->mixed_ready) {
         for (ofea_ctx *c : b->ctx) {
@@ -1507,9 +1516,18 @@ void prepare(ofea_batch *b, bool mixed) {
         b->evec.ensure(nc);
         // K Z after all that the solve cannot do without: where memory ends, it
         // gives way
+        long entries = 0, rows = 0;
         b->modes = true;
         for (ofea_ctx *c : b->ctx) {
-            b->modes = b->modes && ensure_modes(c, c->coarse);
+            const long e = b->modes ? count_modes(c, c->coarse) : -1;
+            b->modes = e >= 0;
+            entries += e;
+            rows += c->nfree;
+        }
+        b->modes = b->modes && entries <= kBatchModes * rows;
+        for (ofea_ctx *c : b->ctx) {
+            if (b->modes) b->modes = ensure_modes(c, c->coarse);
+            else c->coarse.md_slots.release();
             OFEA_CUDA(cudaStreamSynchronize(c->stream));
         }
         if (b->modes) {  // about eight parts per SM
@@ -1640,7 +1658,8 @@ constexpr int kTuneVersion = 2;  // raised when the kernels' best shapes may hav
 std::string tune_key(ofea_batch *b, bool mixed) {
     // problem class: device, method, load cases, rows rounded to 2 significant
     // digits, variants; what else decides the best shape: the kernels' version,
-    // K Z, the most columns of a slice (whether they fit the stage; rounded too).
+    // K Z, the most columns of a slice (whether they fit the stage) and the coarse
+    // unknowns (both rounded too).
     // With the choices of the kernels before these, 4 variants x 32 load cases
     // took 1,285 us per iteration instead of 551, 1 x 16 54.5 instead of 47.0.
     auto round2 = [](long x) {
@@ -1651,7 +1670,8 @@ std::string tune_key(ofea_batch *b, bool mixed) {
     std::ostringstream k;
     k << device_name(b->device) << "|" << (mixed ? "mixed" : "pcg64") << "|nrhs=" << b->NR
       << "|rows~" << round2((long)b->nslices * kSlice) << "|variants=" << b->V << "|kernels=" << kTuneVersion
-      << "|kz=" << (mixed && b->modes ? 1 : 0) << "|columns~" << round2(b->su_max);
+      << "|kz=" << (mixed && b->modes ? 1 : 0) << "|columns~" << round2(b->su_max) << "|coarse~"
+      << round2(mixed ? b->ncrows : 0);
     return k.str();
 }
 

@@ -165,11 +165,13 @@ struct Coarse {
     // K Z of the level (precond.cu): entries (row, aggregate) grouped by
     // aggregate, aggregate J's at md_ptr[J], 18 planes of md_n values; and the
     // same in row order, row r's at md_rptr[r] (entry e at md_rpos[e]).
-    // md_state 0: not built for the geometry, 1: built, -1: no memory for it,
-    // both for the pattern md_pattern; md_gen: the assembly whose values md_val
+    // md_state 0: nothing for the geometry, 2: counted (md_n, md_ptr, and the
+    // rows' slots until they are given back), 1: built, -1: no memory for it,
+    // all for the pattern md_pattern; md_gen: the assembly whose values md_val
     // holds.
     DevBuf<int> md_ptr, md_row, md_agg, md_rptr, md_rpos, md_ragg;
     DevBuf<float> md_val, md_rval;
+    DevBuf<unsigned> md_slots;
     int md_state = 0, md_n = 0;
     long md_gen = -1, md_pattern = -1;
     std::vector<int> agg_cell_h, cell_agg_h;  // host copies (nesting of the learned level)

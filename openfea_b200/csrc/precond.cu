@@ -1545,6 +1545,55 @@ __global__ void k_row_entries(int n, const int *__restrict__ row, const int *__r
     }
 }
 
+// How many entries a level has, or -1 where K Z is not used.
+long count_modes(ofea_ctx *c, Coarse &C) {
+    if (C.md_pattern != c->pattern_gen) {
+        C.md_state = 0;
+        C.md_pattern = c->pattern_gen;
+    }
+    if (!c->K_linear || c->matrix_only || C.md_state < 0) return -1;
+    if (C.md_state != 0) return C.md_n;
+    cudaStream_t s = c->stream;
+    try {
+        C.md_slots.ensure(c->nfree);
+        k_row_slots<<<grid_for(c, c->nfree, kBlock), kBlock, 0, s>>>(
+            c->nfree, c->rowptr.p, c->cols.p, C.row_cell.p, c->node_of_free.p, c->inc_ptr.p, c->inc.p, c->ne8, c->topo8.p,
+            c->topo4.p, c->free_map.p, C.md_slots.p);
+        const int most = std::max(C.na, c->nfree), tmp_len = most / 1024 + 4;
+        c->scratch_i.ensure((size_t)most + 1 + tmp_len);
+        C.md_ptr.ensure((size_t)C.na + 1);
+        k_mode_entries<<<std::min(C.na, c->num_sms * 16), kBlock, 0, s>>>(C.na, C.agg_ptr.p, C.agg_nodes.p, C.nbr.p, C.md_slots.p,
+                                                                         c->scratch_i.p, nullptr, nullptr, nullptr);
+        OFEA_CHECK_LAUNCH();
+        C.md_n = (int)exclusive_scan(c->scratch_i.p, C.md_ptr.p, C.na, s, c->scratch_i.p + most + 1, tmp_len);
+        C.md_state = 2;
+        C.md_gen = -1;
+    } catch (const Failure &f) {
+        C.md_slots.release();
+        if (f.code != OFEA_ERR_OOM) throw;
+        C.md_state = -1;  // until the next pattern
+    }
+    return C.md_state < 0 ? -1 : C.md_n;
+}
+
+// K Z in a single solve, by the entries per row: a row costs 152 bytes of K Z
+// per entry and cycle against about 600 (C3D8) or 330 (C3D4) of a second
+// product.  Where K Z stays in L2 it is the faster one to about 8 entries per
+// row (LEARNED, solve with K Z / without, ms: 15k DOF 6.3 per row 2.22 / 2.44,
+// 9.8 2.25 / 2.19; 139k DOF 5.6 4.49 / 4.81, 10.6 6.3 / 5.9), in large models to
+// about 3 (624k DOF 3.0 7.47 / 7.64, 3.8 7.74 / 7.48, 6.0 11.2 / 10.1).  About
+// 1,000 nodes per aggregate give 0.3 to 1, those of the nested level 1.8 to 3.
+bool solver_modes(ofea_ctx *c, Coarse &C) {
+    const double most = c->nfree < 70000 ? 8.0 : 3.2;
+    const long n = count_modes(c, C);
+    if (n < 0) return false;
+    if (n > most * c->nfree) {
+        C.md_slots.release();
+        return false;
+    }
+    return ensure_modes(c, C);
+}
+
 static void release_modes(Coarse &C) {
     for (DevBuf<int> *b : {&C.md_ptr, &C.md_row, &C.md_agg, &C.md_rptr, &C.md_rpos, &C.md_ragg}) b->release();
     C.md_val.release();
@@ -1552,28 +1601,18 @@ static void release_modes(Coarse &C) {
 }
 
 bool ensure_modes(ofea_ctx *c, Coarse &C) {
-    if (C.md_pattern != c->pattern_gen) {
-        C.md_state = 0;
-        C.md_pattern = c->pattern_gen;
-    }
-    if (!c->K_linear || c->matrix_only || C.md_state < 0) return false;
+    if (count_modes(c, C) < 0) return false;
     const bool fresh = C.md_rval.p == nullptr;  // tables of an earlier pattern stay: a batch may hold them
     cudaStream_t s = c->stream;
     try {
-        if (C.md_state == 0) {
-            DevBuf<unsigned> slots;
-            slots.ensure(c->nfree);
-            k_row_slots<<<grid_for(c, c->nfree, kBlock), kBlock, 0, s>>>(
-                c->nfree, c->rowptr.p, c->cols.p, C.row_cell.p, c->node_of_free.p, c->inc_ptr.p, c->inc.p, c->ne8, c->topo8.p,
-                c->topo4.p, c->free_map.p, slots.p);
+        if (C.md_state == 2) {
+            if (!C.md_slots.p) {  // given back when the count was too high for the caller before
+                C.md_state = 0;
+                if (count_modes(c, C) < 0) return false;
+            }
+            const DevBuf<unsigned> &slots = C.md_slots;
             const int most = std::max(C.na, c->nfree), tmp_len = most / 1024 + 4;
-            c->scratch_i.ensure((size_t)most + 1 + tmp_len);
-            C.md_ptr.ensure((size_t)C.na + 1);
             const int g = std::min(C.na, c->num_sms * 16);
-            k_mode_entries<<<g, kBlock, 0, s>>>(C.na, C.agg_ptr.p, C.agg_nodes.p, C.nbr.p, slots.p, c->scratch_i.p, nullptr,
-                                                nullptr, nullptr);
-            OFEA_CHECK_LAUNCH();
-            C.md_n = (int)exclusive_scan(c->scratch_i.p, C.md_ptr.p, C.na, s, c->scratch_i.p + most + 1, tmp_len);
             C.md_row.ensure(std::max(C.md_n, 1));
             C.md_agg.ensure(std::max(C.md_n, 1));
             C.md_val.ensure(18 * (size_t)std::max(C.md_n, 1));
@@ -1590,11 +1629,11 @@ bool ensure_modes(ofea_ctx *c, Coarse &C) {
                                                                         C.agg_cell.p, slots.p, C.md_rptr.p, C.md_rpos.p,
                                                                         C.md_ragg.p);
             OFEA_CHECK_LAUNCH();
-            OFEA_CUDA(cudaStreamSynchronize(s));  // before slots is released
+            C.md_slots.release();
             C.md_state = 1;
-            C.md_gen = -1;
         }
     } catch (const Failure &f) {
+        C.md_slots.release();
         if (f.code != OFEA_ERR_OOM) throw;
         C.md_state = -1;  // until the next pattern
         if (fresh) release_modes(C);

@@ -124,8 +124,12 @@ void vc_resid(ofea_ctx *c, const float *b, const float *x, float *t);
 // K Z of a level, current for K: the restriction c = Z^T b - (K Z)^T x
 // (restrict_modes) and the post-smoothing's K Z e take the place of a product
 // with K.  False where the residual is formed instead (K not the linear
-// stiffness of a mesh, or no memory for it).
+// stiffness of a mesh, or no memory for it).  solver_modes: the same for a single
+// solve, only where it is the faster of the two; count_modes: the level's
+// entries (-1: none), before anything else of it is built.
 bool ensure_modes(ofea_ctx *c, Coarse &C);
+bool solver_modes(ofea_ctx *c, Coarse &C);
+long count_modes(ofea_ctx *c, Coarse &C);
 void restrict_modes(ofea_ctx *c, const Coarse &C, const float *b, const float *x, float *cvec);
 // Level-generic pieces (also used by the learned level):
 // cvec = Z^T t, x += Z g, and the Galerkin blocks of Z^T K Z into C.part

@@ -25,7 +25,7 @@ bool resident_plan(const ofea_ctx *c, bool mixed, bool elements, ResidentPlan &p
 // Enqueues `iters` iterations from fl->itA on (fewer when the solve stops) on
 // the context's stream.  MIXED with first != 0 starts with the preconditioner
 // applied to b32 / x32 (z_0); with modes its restriction takes K Z
-// (ensure_modes).  Partials of the kernels before it: G each.
+// (solver_modes).  Partials of the kernels before it: G each.
 void resident_iterations(ofea_ctx *c, const ResidentPlan &p, bool mixed, bool modes, const Parts &P, Flags *fl, double *d_u,
                          float wsm, double tol2, int iters, int first);
 

@@ -673,7 +673,7 @@ void solve_device(ofea_ctx *c, const double *d_f, double *d_u, const ofea_solve_
         // every buffer the solve cannot do without is there, before the tables
         // that are optional (K Z, the elements'): where memory ends, those give way
         reserve(w);
-        modes = ensure_modes(c, learned ? c->coarse2 : c->coarse);
+        modes = solver_modes(c, learned ? c->coarse2 : c->coarse);
         OFEA_CUDA(cudaEventRecord(es, s));
         OFEA_CUDA(cudaEventSynchronize(es));
         OFEA_CUDA(cudaEventElapsedTime(&setup_ms, e0, es));
@@ -922,7 +922,7 @@ std::vector<KernelTime> profile_iteration(ofea_ctx *c, int method, int reps) {
     const bool elements = nf >= kMatfreeRows && matfree_possible(c);
     bool matfree = !mixed && elements && matfree_ready(c);
     if (!learned && !matfree && resident_plan(c, mixed, elements, plan)) return {};
-    const bool modes = mixed && ensure_modes(c, C);
+    const bool modes = mixed && solver_modes(c, C);
     if (mixed) matfree = elements && matfree_ready(c);
     const double nnzv = 9.0 * c->sell_len * kSlice, nblk = (double)c->sell_len * kSlice;  // incl. padding
     const double zb = mixed ? 4.0 : 8.0, vec = 8.0 * n, slices = 4.0 * ((nf + 31) / 32 + 1);

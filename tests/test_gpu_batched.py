@@ -279,6 +279,38 @@ def test_vcycle_with_and_without_sparse_modes(gpu_ctx_factory, tangent, nrhs):
         assert np.all(np.linalg.norm(F.T - K @ u.T, axis=0) <= 1e-9 * norms + floor)
 
 
+@pytest.mark.parametrize("shape,nodes,kz_batch,kz_single", [((30, 12, 12), 1000, 1, True), ((30, 12, 12), 250, 1, True),
+                                                            ((30, 12, 12), 30, 0, True), ((130, 25, 22), 30, 0, False)])
+def test_sparse_modes_by_entries_per_row(gpu_ctx_factory, tmp_path, monkeypatch, shape, nodes, kz_batch, kz_single):
+    # 0.4 to 4 entries of K Z per row: the batch takes it to 1.5, a single solve
+    # to 8 (3.2 from 70,000 rows); a count that the batch did without is taken
+    # again by the single solve
+    path = tmp_path / "tune.json"
+    monkeypatch.setenv("OFEA_TUNE_FILE", str(path))
+    c = gpu_ctx_factory()
+    c.upload_mesh(mg.structured_hex(*shape, *(0.005 * s for s in shape), 210e9, 0.3))
+    c.assemble_pattern()
+    c.set_coarse_nodes(nodes)
+    c.assemble_linear()
+    F = np.random.default_rng(5).normal(size=(3, c.n))
+    b = ob.Batch([c], 3)
+    (ub,), _ = b.solve([F], method="GPU_MIXED", rtol=1e-9)
+    (key,) = {e["key"] for e in json.load(open(path))["entries"]}
+    assert "kz=%d" % kz_batch in key
+    c.set_setup_trace(True)
+    us, _ = c.solve(F[0], method="GPU_MIXED", rtol=1e-9)
+    if kz_batch == 0:  # else its values are there already
+        assert ("modes" in c.setup_phase_times()) == kz_single
+    rp, col, val = c.get_csr()
+    K = sp.csr_matrix((val, col, rp), shape=(c.n, c.n))
+    for u, f in [(us, F[0])] + list(zip(ub, F)):
+        floor = np.diff(rp).max() * np.finfo(float).eps * np.linalg.norm(abs(K) @ abs(u))
+        assert np.linalg.norm(f - K @ u) <= 1e-9 * np.linalg.norm(f) + floor
+    (again,), _ = b.solve([F], method="GPU_MIXED", rtol=1e-9)
+    assert np.array_equal(again, ub)
+    b.close()
+
+
 @pytest.mark.parametrize("nrhs", [3, 8, 16, 20, 32])
 @pytest.mark.parametrize("rl", [1, 2, 4])
 def test_every_tile_configuration(gpu_ctx_factory, tmp_path, monkeypatch, rl, nrhs):

@@ -813,8 +813,11 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
 #pragma unroll 1
         for (int ph = 0; ph < 2; ++ph) {
             if (a.modes == ph) {
-                // e = E^-1 c: warp per coarse row, NP lanes per load case group
-                constexpr int JW = NP, RPW = 32 / NP;
+                // e = E^-1 c: warp per coarse row, NP lanes per load case group,
+                // kE entries per lane in flight (a row is one serial sum, and only 4
+                // to 16 warps share an SM: 20 load cases, 4,536 unknowns 294 us,
+                // one after another 443; 16 cases, 2,880 138 and 141)
+                constexpr int JW = NP, RPW = 32 / NP, kE = 8;
                 const int warps = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x & 31;
                 const int sub = lane / JW, jj = lane % JW;
                 for (int gr = blockIdx.x * warps + w; gr < a.ncrows; gr += gridDim.x * warps) {
@@ -824,8 +827,21 @@ __global__ void __launch_bounds__(32 * (NP / RL), batch_min_ctas(32 * (NP / RL))
                     const int i = gr - B.crow0, m = B.m;
                     const float *row = B.Einv32 + (long)i * m;
                     float acc = 0.f;
-                    if (live)
-                        for (int k = sub; k < m; k += RPW) acc = fmaf(__ldg(row + k), a.cvec[(B.c0 + k) * NP + jj], acc);
+                    if (live) {
+                        const float *cv = a.cvec + B.c0 * NP + jj;
+                        int k = sub;
+                        for (; k + (kE - 1) * RPW < m; k += kE * RPW) {
+                            float e[kE], x[kE];
+#pragma unroll
+                            for (int u = 0; u < kE; ++u) {
+                                e[u] = __ldg(row + k + u * RPW);
+                                x[u] = cv[(long)(k + u * RPW) * NP];
+                            }
+#pragma unroll
+                            for (int u = 0; u < kE; ++u) acc = fmaf(e[u], x[u], acc);
+                        }
+                        for (; k < m; k += RPW) acc = fmaf(__ldg(row + k), cv[(long)k * NP], acc);
+                    }
 #pragma unroll
                     for (int off = JW; off < 32; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
                     if (sub == 0 && live) a.evec[(B.c0 + i) * NP + jj] = acc;

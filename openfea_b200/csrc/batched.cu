@@ -14,9 +14,10 @@
 //
 // Algorithm per (variant, load case): the MIXED method of solve.cu, FP64
 // flexible CG with the FP32 two-level V(1,1) preconditioner of precond.cu (with
-// K Z where every variant has it: one product instead of two, 8 to 46 % less
-// time at 1 to 32 variants of 7k and 27k nodes and 3 to 16 load cases; the
-// phases of a trace stay, the residual's is then a barrier alone), or
+// K Z where every variant has it, with few entries per row: one product
+// instead of two, 8 to 46 % less time at 1 to 32 variants of 7k and 27k nodes
+// and 3 to 16 load cases; the phases of a trace stay, the residual's is then a
+// barrier alone), or
 // PCG64 (FP64 CG, block Jacobi).  The kernel runs every variant in lock step
 // through phases separated by grid barriers.  In the matrix phases a CTA owns
 // one slice (32 block rows) of some variant at a time: bulk copies bring the
